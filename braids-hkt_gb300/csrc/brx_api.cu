@@ -23,6 +23,7 @@
 #include "../../include/braids_gb300.h"
 #define BRX_NS brx
 #include "brx_kernels.cuh"
+#include "brx_cells64.cuh"
 #include "brx_launch.h"
 #include "brx_turbine.cuh"
 #include "brx_exner.cuh"
@@ -85,6 +86,8 @@ struct brx_solver {
     LaunchShape shape[NSHAPE];       // tunable launch shape per kernel kind (brx_launch_shape_set)
     int launches_per_substep = 0;
     MixedGeo mx{};                   // FP32 geometry of the mixed form
+    Cells64 c64{};                   // FP64 form, cells of at most four faces: tables of the cell sweep
+    bool small64 = false;            // c64 is in use
     std::vector<int2> h_cidx;        // host copy: stage-outlet flags follow brx_boundary_set
     int2 *d_cidx = nullptr;
     std::vector<int> h_faces_csr;
@@ -356,6 +359,18 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
         TRY(s->alloc(&a.cstart, nscen + 1)); TRY(s->alloc(&a.fstart, nscen + 1));
         CK(cudaMemset(a.count, 0, sizeof(int) * 3));
         a.cell_off = s->d_cell_off; a.face_off = s->d_face_off;
+        s->small64 = precision == BRX_FP64 && s->maxdeg <= 4;
+        if (s->small64) {
+            // the cell sweep's tables, formed on the device from the uploaded
+            // geometry: the default stream follows the uploads
+            Cells64 &g = s->c64;
+            TRY(s->alloc(&g.ls, nc)); TRY(s->alloc(&g.lsr, nc)); TRY(s->alloc(&g.par, nc)); TRY(s->alloc(&g.ccls, nc));
+            TRY(s->alloc(&g.cidx, nadj)); TRY(s->alloc(&g.ent, nadj)); TRY(s->alloc(&g.unit, nadj));
+            TRY(s->alloc(&g.gbed, nc)); TRY(s->alloc(&g.prim[0], nc)); TRY(s->alloc(&g.prim[1], nc));
+            k64_tables<<<std::max(1, std::min((nc + 255) / 256, s->sms * 32)), 256>>>(m, g);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(nullptr));
+        }
         if (precision == BRX_MIXED) {
             // FP32 geometry packed per cell, per CSR entry and per face; the LS
             // inverse is formed in FP64 here so the sweep only multiplies.
@@ -537,6 +552,12 @@ extern "C" int brx_boundary_set(brx_solver *s, const int *seg_mode, const int *s
     CK(cudaMemcpy(s->d_stage_policy_rw, stage_policy, sizeof(int) * nseg, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(s->d_ext_bed_rw, ext.data(), sizeof(double) * s->nslot, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(s->bnd.forcing, forcing, sizeof(double) * 2 * nseg, cudaMemcpyHostToDevice));
+    if (s->small64) {
+        // the modes changed: the entries' stage-outlet flags with them
+        k64_tables<<<std::max(1, std::min((s->nc + 255) / 256, s->sms * 32)), 256>>>(s->mesh, s->c64);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(nullptr));
+    }
     if (s->precision == BRX_MIXED) {
         // entries on a stage outlet face (flag bit1) for the mixed cell sweep
         std::fill(s->h_ccls.begin(), s->h_ccls.end(), 0);
@@ -1063,7 +1084,10 @@ static int max_block(const brx_solver *s, int kind)
     const void *fn = nullptr;
     switch (kind) {
     case K_DRAG: fn = (const void *)k_open_drag<double>; break;
-    case K_CELLS: fn = small ? (const void *)k_cells<double, 4> : (const void *)k_cells<double, MAX_CELL_FACES>; break;
+    case K_CELLS:
+        fn = s->maxdeg <= 3 ? (const void *)k64_cells<3> : small ? (const void *)k64_cells<4>
+                            : (const void *)k_cells<double, MAX_CELL_FACES>;
+        break;
     case K_FACES: fn = (const void *)k_faces<double>; break;
     case K_GATHER: fn = (const void *)k_gather; break;
     case K_LIMIT: fn = (const void *)k_limit; break;
@@ -1512,14 +1536,18 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
     if (s->precision == BRX_MIXED) return mixed_kernel(make_launch(s, st), kind, stage, rate_out);
     switch (kind) {
     case K_DRAG:
-        k_open_drag<double><<<SSHAPE(K_DRAG, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl);
+        k_open_drag<double><<<SSHAPE(K_DRAG, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl,
+                                                             s->method == BRX_METHOD_FWAVE ? s->c64.prim[0] : nullptr);
         return 1;
     case K_BOUNDARY:
         if (!s->nslot) return 0;
         k_boundary<double><<<s->nscen, 256, 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, stage);
         return 1;
     case K_CELLS:
-        if (s->maxdeg <= 4) k_cells<double, 4><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
+        if (s->maxdeg <= 3)
+            k64_cells<3><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, s->c64, stage);
+        else if (s->maxdeg <= 4)
+            k64_cells<4><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, s->c64, stage);
         else k_cells<double, MAX_CELL_FACES><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
         return 1;
     case K_FACES:
@@ -1534,7 +1562,7 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
         return 1;
     case K_UPDATE:
         k_update<double><<<SSHAPE(K_UPDATE, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage, rate_out,
-                                                        s->turb, s->has_turb);
+                                                        s->turb, s->has_turb, s->c64.prim[1]);
         return 1;
     }
     return 0;
@@ -1702,11 +1730,17 @@ static void begin_interval(brx_solver *s, double dt, double time, bool fixed)
     begin_interval_each(s, d.data(), t.data(), fixed);
 }
 
-// Mixed form: bed-derived tables from the bed as it is now (it may have
+// Bed-derived tables of both forms from the bed as it is now (it may have
 // changed since the last call).
 static void refresh_bed(brx_solver *s)
 {
     if (s->precision == BRX_MIXED) s->launches += mixed_kernel(make_launch(s, s->stream), K_BED, 0, nullptr);
+    // the HLLC method limits its bed gradient with its own rule
+    if (s->small64 && s->method == BRX_METHOD_FWAVE) {
+        if (s->maxdeg <= 3) k64_bed<3><<<s->grid_c, 128, 0, s->stream>>>(s->mesh, s->c64, s->state.z);
+        else k64_bed<4><<<s->grid_c, 128, 0, s->stream>>>(s->mesh, s->c64, s->state.z);
+        s->launches++;
+    }
 }
 
 static int ensure_ready(brx_solver *s)
@@ -1990,6 +2024,10 @@ extern "C" int brx_rate(brx_solver *s, double dt, double time, double *rate_devi
     CK(cudaMemcpyAsync(s->state.work, s->state.q[0], sizeof(double) * 3 * s->nc, cudaMemcpyDeviceToDevice, s->stream));
     refresh_bed(s);
     if (s->precision == BRX_MIXED) s->launches += launch_kernel(s, K_PRIM, 1, nullptr);
+    else if (s->small64) {
+        k64_prim<<<s->grid_c256, 256, 0, s->stream>>>(s->mesh, s->state, s->d_ctrl, s->c64);
+        s->launches++;
+    }
     enqueue_stage(s, 1, rate_device);
     // the limited water flux of each face, for the caller's water buffer
     s->launches += launch_kernel(s, K_LIMIT, 1, nullptr);
@@ -2335,7 +2373,7 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     k_faces<double><<<(nf + 127) / 128, 128, 0, st>>>(m, sd, b, ctrl, w, 1, nullptr, nullptr);
     k_gather<<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1);
     k_limit<<<(nf + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1);
-    k_update<double><<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0);
+    k_update<double><<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);
     k_noalloc_water<<<(nf + 255) / 256, 256, 0, st>>>(m, w, ctrl, water);
     CK(cudaGetLastError());
     Ctrl out{};

@@ -8,6 +8,7 @@
 // evaluate exactly the FP64 expressions of the reference.
 #pragma once
 #include "brx_common.cuh"
+#include "brx_num64.cuh"
 
 #ifndef BRX_NS
 #error "define BRX_NS before including brx_kernels.cuh"
@@ -41,9 +42,9 @@ __device__ __forceinline__ void drag_cell(const Ctrl &ct, double dt, double &h, 
     hv *= factor;
 }
 
-// work = drag(accepted, trial/2)
+// work = drag(accepted, trial/2); prim (may be null): the first stage's primitives
 template <class F>
-__global__ void k_open_drag(MeshDev m, StateDev s, Ctrl *ctrl)
+__global__ void k_open_drag(MeshDev m, StateDev s, Ctrl *ctrl, Prim64 *prim)
 {
     const int nc = m.nc;
     FOR_ACTIVE_CELLS(m.act, c) {
@@ -53,6 +54,7 @@ __global__ void k_open_drag(MeshDev m, StateDev s, Ctrl *ctrl)
         double h = q[c], hu = q[nc + c], hv = q[2 * nc + c];
         drag_cell<F>(ct, .5 * ct.trial, h, hu, hv);
         s.work[c] = h; s.work[nc + c] = hu; s.work[2 * nc + c] = hv;
+        if (prim) put_prim64(prim, c, h, hu, hv, s.z[c], ct.dry);
     }
 }
 
@@ -2103,7 +2105,7 @@ __device__ __forceinline__ void add_viscosity(const MeshDev &m, const ViscDev &v
 // of a single residual).
 template <class F>
 __global__ void __launch_bounds__(256) k_update(MeshDev m, StateDev s, Ctrl *ctrl, Work w, int stage,
-                                                double *rate_out, TurbDev t, int turb)
+                                                double *rate_out, TurbDev t, int turb, Prim64 *prim)
 {
     const int nc = m.nc;
     const double *q = stage == 1 ? s.work : s.q1;
@@ -2147,6 +2149,7 @@ __global__ void __launch_bounds__(256) k_update(MeshDev m, StateDev s, Ctrl *ctr
             if (h < 0) raise_status(ct, 1, ST_ENDPOINT);
             if (h <= dry) { hu = 0.; hv = 0.; }
             s.q1[c] = h; s.q1[nc + c] = hu; s.q1[2 * nc + c] = hv;
+            if (prim) put_prim64(prim, c, h, hu, hv, s.z[c], dry);   // the second stage's
         } else {
             double h = .5 * s.work[c] + .5 * (s.q1[c] + dt * r0);
             double hu = .5 * s.work[nc + c] + .5 * (s.q1[nc + c] + dt * r1);
