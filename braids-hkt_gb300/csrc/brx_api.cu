@@ -24,6 +24,7 @@
 #define BRX_NS brx
 #include "brx_kernels.cuh"
 #include "brx_cells64.cuh"
+#include "brx_faces64.cuh"
 #include "brx_launch.h"
 #include "brx_turbine.cuh"
 #include "brx_exner.cuh"
@@ -1088,7 +1089,7 @@ static int max_block(const brx_solver *s, int kind)
         fn = s->maxdeg <= 3 ? (const void *)k64_cells<3> : small ? (const void *)k64_cells<4>
                             : (const void *)k_cells<double, MAX_CELL_FACES>;
         break;
-    case K_FACES: fn = (const void *)k_faces<double>; break;
+    case K_FACES: fn = (const void *)k64_faces; break;
     case K_GATHER: fn = (const void *)k_gather; break;
     case K_LIMIT: fn = (const void *)k_limit; break;
     case K_UPDATE: fn = (const void *)k_update<double>; break;
@@ -1551,7 +1552,7 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
         else k_cells<double, MAX_CELL_FACES><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
         return 1;
     case K_FACES:
-        k_faces<double><<<SSHAPE(K_FACES, s->nf), 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, s->work, stage,
+        k64_faces<<<SSHAPE(K_FACES, s->nf), 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, s->work, stage,
                                                     s->has_turb ? s->turb.trace : nullptr, s->turb.hkt);
         return 1;
     case K_GATHER:
@@ -1698,6 +1699,7 @@ static void host_set_trial(Ctrl &c)
     c.truncated = c.trial < c.hint * (1 - 1e-12);
     c.status1 = c.status2 = 0;
     c.peak1 = c.peak2 = 0ull;
+    c.g16r = 1. / (16. * c.grav);
     c.gravf = float(c.grav); c.dryf = float(c.dry); c.trialf = float(c.trial);
     c.roughf = float(c.roughness_value); c.cfl1 = 0;
 }
@@ -2363,6 +2365,7 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     Ctrl init{};
     init.grav = gravity; init.dry = dry; init.cfl = cfl; init.speed_limit = 50.0;
     init.roughness_mode = 1; init.roughness_value = 1.0; init.active = 1;
+    init.g16r = 1. / (16. * gravity);
     init.dt_outer = dt; init.hint = dt; init.trial = dt; init.max_substeps = 1;
     // Every field the residual reads is rewritten here: the array keeps the
     // previous call's contents, and calls that overlap on the GPU race on it.
@@ -2370,7 +2373,7 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     const int n = nc > nf ? nc : nf;
     k_noalloc_tables<<<(n + 255) / 256, 256, 0, st>>>(m, ctrl, cell_sid, cflags, face_sid, bslot, bmode, disp_unit);
     k_cells<double, MAX_CELL_FACES><<<(nc + 127) / 128, 128, 0, st>>>(m, sd, ctrl, w, 1);
-    k_faces<double><<<(nf + 127) / 128, 128, 0, st>>>(m, sd, b, ctrl, w, 1, nullptr, nullptr);
+    k64_faces<<<(nf + 127) / 128, 128, 0, st>>>(m, sd, b, ctrl, w, 1, nullptr, nullptr);
     k_gather<<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1);
     k_limit<<<(nf + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1);
     k_update<double><<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);

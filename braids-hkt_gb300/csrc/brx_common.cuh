@@ -79,6 +79,7 @@ struct Ctrl {
     // inequality), which scales its roundoff allowance
     double bflux[2], ledger;
     double bgross[2], gross;
+    double g16r;                            // 1 / (16 grav), the two-rarefaction depth's factor
     // FP32 copies for the mixed form's sweeps, refreshed with every trial
     float gravf, dryf, trialf, roughf;
     int cfl1, pad1;                         // stage 1 exceeded the CFL limit (mixed form, set after its gather)

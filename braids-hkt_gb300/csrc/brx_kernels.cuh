@@ -1733,202 +1733,6 @@ __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl
 }
 
 // ---------------------------------------------------------------------------
-// Faces: traces, hydrostatic reconstruction, f-wave, flux assembly.
-// Traces, the common-bed stage, pressures and the bed source are FP64; the
-// Riemann solve and the advective fluxes run in F.
-// ---------------------------------------------------------------------------
-struct Side { double h, hu, hv, b, raw; };
-
-template <class F>
-__device__ __forceinline__ Side face_side(const CellRec &r, double rx_, double ry_, double dry, bool dryface,
-                                          unsigned &bad)
-{
-    const F rx = F(rx_), ry = F(ry_);
-    double val[4] = {(r.eta + double(F(r.gx[0]) * rx)) + double(F(r.gy[0]) * ry),
-                     double((F(r.u) + F(r.gx[1]) * rx) + F(r.gy[1]) * ry),
-                     double((F(r.v) + F(r.gx[2]) * rx) + F(r.gy[2]) * ry),
-                     (r.b + double(F(r.gx[3]) * rx)) + double(F(r.gy[3]) * ry)};
-    const bool constant = r.flags & 1;
-    if (constant) {
-        val[0] = r.eta; val[1] = r.u; val[2] = r.v;
-        if (r.eta - r.b <= dry) val[3] = r.b;
-    }
-    if (!isfinite(val[0]) || !isfinite(val[1]) || !isfinite(val[2]) || !isfinite(val[3])) bad = 1;
-    Side o = {0., 0., 0., 0., 0.};
-    if (dryface) return o;
-    double depth = fmax(val[0] - val[3], 0.);
-    o.raw = depth;
-    if (r.h <= dry || (constant && depth <= dry)) depth = 0.;
-    o.h = depth; o.hu = depth * val[1]; o.hv = depth * val[2]; o.b = val[3];
-    return o;
-}
-
-template <class F>
-// Four resident blocks of 128 threads (at most 128 registers): a single
-// 75k-face scenario then fits the 152 SMs in one wave of 16 warps each; with
-// the unconstrained 168 registers it took 1.3 waves at 12 warps per SM and
-// the FP64 pipe sat idle in the tail.
-#ifndef BRX_FP64_FACES_MIN_BLOCKS
-#define BRX_FP64_FACES_MIN_BLOCKS 4
-#endif
-__global__ void __launch_bounds__(128, BRX_FP64_FACES_MIN_BLOCKS) k_faces(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, Work w, int stage,
-                                               double *trace, const int *hkt)
-{
-    const int nf = m.nf, nc = m.nc;
-    FOR_ACTIVE_FACES(m.act, f) {
-        Ctrl &ct = ctrl[m.face_sid[f]];
-        if (skip_stage(ct, stage)) continue;
-        const double dry = ct.dry, grav = ct.grav;
-        const int c = m.owner[f], n = m.neighbour[f];
-        const double nx = m.normal[f], ny = m.normal[nf + f];
-        const CellRec rc = w.rec[c];
-        const double pc = .5 * grav * rc.h * rc.h;
-        const int slot = m.bslot[f];
-        if (slot >= 0) {
-            // open face: the exterior owner's flux, owner/exterior CFL speed
-            const double *q = stage == 1 ? s.work : s.q1;
-            const double fl0 = b.flux[slot], fl1 = b.flux[(size_t)b.nslot + slot], fl2 = b.flux[2 * (size_t)b.nslot + slot];
-            const double hb = b.trace[slot];
-            const double hq = q[c];
-            const double a = hq > dry ? fabs((q[nc + c] * nx + q[2 * nc + c] * ny) / hq) + sqrt(grav * hq) : 0.;
-            const double bb = hb > dry ? fabs((b.trace[(size_t)b.nslot + slot] * nx + b.trace[2 * (size_t)b.nslot + slot] * ny) / hb) +
-                                             sqrt(grav * hb) : 0.;
-            w.ws[f] = make_double2(fl0, fmax(a, bb));
-            w.gf[f] = make_double4_32a(fl1 - pc * nx, fl2 - pc * ny, 0., 0.);
-            continue;
-        }
-        CellRec rn;
-        if (n >= 0) rn = w.rec[n];
-        int kind = n >= 0 ? 1 : 2;
-        if (rc.h <= dry && (n < 0 || rn.h <= dry)) kind = 0;
-        unsigned bad = 0;
-        const Side L = face_side<F>(rc, m.disp[f], m.disp[2 * nf + f], dry, kind == 0, bad);
-        Side R = {0., 0., 0., 0., 0.};
-        if (n >= 0) R = face_side<F>(rn, m.disp[nf + f], m.disp[3 * nf + f], dry, kind == 0, bad);
-        double water = 0., speed = 0., l1 = 0., l2 = 0., r1 = 0., r2 = 0.;
-        if (kind != 0) {
-            double hL = L.h, xL = L.hu, yL = L.hv, bL = L.b;
-            double hR = R.h, xR = R.hu, yR = R.hv, bR = R.b;
-            double rawR = R.raw;
-            if (kind == 2) {
-                hR = hL; xR = xL; yR = yL; bR = bL; rawR = L.raw;   // mirrored trace
-            }
-            // rotation to the face frame (prepare)
-            double xRr = xR, yRr = yR;
-            if (kind == 2) {
-                const double dot = xL * nx + yL * ny;
-                xRr = xL - 2.0 * dot * nx; yRr = yL - 2.0 * dot * ny;
-            }
-            const double unL = xL * nx + yL * ny, utL = xL * (-ny) + yL * nx;
-            const double unR = xRr * nx + yRr * ny, utR = xRr * (-ny) + yRr * nx;
-            double loc[8] = {hL, unL, utL, bL, hR, unR, utR, bR};
-            if (kind == 1) {
-                const double top = fmax(bL, bR);
-                const double tol = 16. * EPS * fmax(dry, fmax(fabs(top), fmax(fabs(hL + bL), fabs(hR + bR))));
-                double hl = fmax(0., hL + bL - top), hr = fmax(0., hR + bR - top);
-                if (hl <= dry + tol) hl = 0.;
-                if (hr <= dry + tol) hr = 0.;
-                loc[0] = hl; loc[3] = top; loc[4] = hr; loc[7] = top;
-                loc[1] = hL > dry ? unL * (hl / hL) : 0.;
-                loc[2] = hL > dry ? utL * (hl / hL) : 0.;
-                loc[5] = hR > dry ? unR * (hr / hR) : 0.;
-                loc[6] = hR > dry ? utR * (hr / hR) : 0.;
-            }
-            if (trace && n >= 0 && hkt[m.face_sid[f]]) put_trace(trace, nf, f, loc, rc.flags & 1, rn.flags & 1);
-            bool closed = false;
-            if (kind == 1 && !(fmin(rc.h, rn.h) > dry)) {
-                const double dc = m.distance[f], dn = m.distance[nf + f];
-                double shared;
-                if (dc + dn > DBL_MIN_)
-                    shared = (dn * (rc.b + rc.h) + dc * (rn.b + rn.h)) / (dc + dn) - fmax(rc.b, rn.b);
-                else
-                    shared = 0.5 * ((rc.b + rc.h) + (rn.b + rn.h)) - fmax(rc.b, rn.b);
-                closed = shared <= dry;
-                if (closed) {
-                    bool opens = false;
-                    if (hL > dry && hR <= dry && unL / hL > 0.0) {
-                        const RType<F> t = riemann_type<F>(F(hL), F(hL), F(unL / hL), F(-unL / hL), F(dry), F(grav));
-                        opens = t.hm > hL + dry && t.hm + bL > bR + dry;
-                    } else if (hR > dry && hL <= dry && -unR / hR > 0.0) {
-                        const RType<F> t = riemann_type<F>(F(hR), F(hR), F(-unR / hR), F(unR / hR), F(dry), F(grav));
-                        opens = t.hm > hR + dry && t.hm + bR > bL + dry;
-                    }
-                    closed = !opens;
-                }
-            }
-            double l[3] = {0., 0., 0.}, r[3] = {0., 0., 0.};
-            FWaveOut<F> fwo;
-            F locf[8];
-#pragma unroll
-            for (int j = 0; j < 8; ++j) locf[j] = F(loc[j]);
-            const int fst = fwave<F>(locf, F(grav), F(dry), fwo);
-            if (fst) bad = 1;
-            if (closed) {
-                l[1] = 0.5 * grav * (hL * hL) * nx; l[2] = 0.5 * grav * (hL * hL) * ny;
-                r[1] = 0.5 * grav * (hR * hR) * nx; r[2] = 0.5 * grav * (hR * hR) * ny;
-                if (hL > dry) speed = fmax(speed, fabs(loc[1] / hL) + sqrt(grav * hL));
-                if (hR > dry) speed = fmax(speed, fabs(loc[5] / hR) + sqrt(grav * hR));
-            } else {
-                const double starL = loc[0], starR = loc[4];
-                double pl[3] = {0., 0., 0.}, pr[3] = {0., 0., 0.};
-                if (starL > dry) {
-                    const double hu = loc[1], hv = loc[2];
-                    pl[0] = hu; pl[1] = double(F(hu) * F(hu) / F(starL)) + 0.5 * grav * (starL * starL);
-                    pl[2] = double(F(hu) * F(hv) / F(starL));
-                }
-                if (starR > dry) {
-                    const double hu = loc[5], hv = loc[6];
-                    pr[0] = hu; pr[1] = double(F(hu) * F(hu) / F(starR)) + 0.5 * grav * (starR * starR);
-                    pr[2] = double(F(hu) * F(hv) / F(starR));
-                }
-#pragma unroll
-                for (int j = 0; j < 3; ++j) { pl[j] += double(fwo.amdq[j]); pr[j] -= double(fwo.apdq[j]); }
-                l[0] = pl[0]; l[1] = pl[1] * nx + pl[2] * (-ny); l[2] = pl[1] * ny + pl[2] * nx;
-                r[0] = pr[0]; r[1] = pr[1] * nx + pr[2] * (-ny); r[2] = pr[1] * ny + pr[2] * nx;
-                // left/right mass fluxes agree to the Riemann solve's precision (1e-10 in FP64)
-                const double consistency = sizeof(F) == 8 ? 1.e-10 : 2.e-5;
-                if (fabs(l[0] - r[0]) > consistency * fmax(1.0, fmax(fabs(l[0]), fabs(r[0])))) bad = 1;
-                l[0] = 0.5 * (l[0] + r[0]); r[0] = l[0];
-                speed = double(fmax(fabs(fwo.s[0]), fmax(fabs(fwo.s[1]), fabs(fwo.s[2]))));
-                if (kind == 1) {
-                    const double cl = .5 * grav * (hL * hL - starL * starL), cr = .5 * grav * (hR * hR - starR * starR);
-                    l[1] += cl * nx; l[2] += cl * ny; r[1] += cr * nx; r[2] += cr * ny;
-                }
-                if (kind == 2) {
-                    l[0] = 0.0;
-                    const double pressure = wall_pressure<double>(hL, loc[1], grav, dry);
-                    l[1] = pressure * nx; l[2] = pressure * ny;
-                    r[0] = l[0]; r[1] = l[1]; r[2] = l[2];
-                }
-            }
-            if (rc.h > dry) {
-                const double corr = (rc.flags & 1) ? 0.5 * grav * (rc.h * rc.h - hL * hL)
-                                                   : 0.5 * grav * (rc.h + L.raw) * (bL - rc.b);
-                l[1] += corr * nx; l[2] += corr * ny;
-            }
-            if (n >= 0) {
-                if (rn.h > dry) {
-                    const double corr = (rn.flags & 1) ? 0.5 * grav * (rn.h * rn.h - hR * hR)
-                                                       : 0.5 * grav * (rn.h + rawR) * (bR - rn.b);
-                    r[1] += corr * nx; r[2] += corr * ny;
-                }
-            } else { r[0] = l[0]; r[1] = l[1]; r[2] = l[2]; }
-            if (!isfinite(l[0]) || !isfinite(l[1]) || !isfinite(l[2]) || !isfinite(r[0]) || !isfinite(r[1]) ||
-                !isfinite(r[2])) bad = 1;
-            water = l[0]; l1 = l[1]; l2 = l[2]; r1 = r[1]; r2 = r[2];
-        }
-        if (kind == 0 && trace && n >= 0 && hkt[m.face_sid[f]]) {
-            const double zero[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
-            put_trace(trace, nf, f, zero, rc.flags & 1, rn.flags & 1);
-        }
-        if (bad) raise_status(ct, stage, ST_SPATIAL);
-        w.ws[f] = make_double2(water, speed);
-        const double pn = n >= 0 ? .5 * grav * rn.h * rn.h : 0.;
-        w.gf[f] = make_double4_32a(l1 - pc * nx, l2 - pc * ny, r1 - pn * nx, r2 - pn * ny);
-    }
-}
-
-// ---------------------------------------------------------------------------
 // Gather: rate, donor inventory / boundary reservation, CFL frequency.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_gather(MeshDev m, StateDev s, Ctrl *ctrl, Work w, int stage)
