@@ -25,6 +25,7 @@
 #include "brx_kernels.cuh"
 #include "brx_cells64.cuh"
 #include "brx_faces64.cuh"
+#include "brx_update64.cuh"
 #include "brx_launch.h"
 #include "brx_turbine.cuh"
 #include "brx_exner.cuh"
@@ -349,17 +350,29 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
         TRY(s->alloc(&s->state.q[1], 3 * (size_t)nc)); TRY(s->alloc(&s->state.work, 3 * (size_t)nc));
         TRY(s->alloc(&s->state.q1, 3 * (size_t)nc));
         TRY(s->alloc(&s->work.rec, nc)); TRY(s->alloc(&s->work.ws, nf)); TRY(s->alloc(&s->work.gf, nf));
-        TRY(s->alloc(&s->work.lim, nf)); TRY(s->alloc(&s->work.rate, 3 * (size_t)nc));
+        TRY(s->alloc(&s->work.lim, nf));
+        if (precision == BRX_MIXED) TRY(s->alloc(&s->work.rate, 3 * (size_t)nc));
         TRY(s->alloc(&s->work.theta, nc));
         TRY(s->alloc(&s->d_ctrl, nscen));
         // active set of the current trial (rebuilt on the device by k_control)
         TRY(s->upload(&s->d_cell_off, s->cell_offset.data(), s->cell_offset.size()));
         TRY(s->upload(&s->d_face_off, s->face_offset.data(), s->face_offset.size()));
         ActiveDev &a = s->mesh.act;
-        TRY(s->alloc(&a.count, 3)); TRY(s->alloc(&a.cdelta, nscen)); TRY(s->alloc(&a.fdelta, nscen));
+        TRY(s->alloc(&a.count, 5)); TRY(s->alloc(&a.cdelta, nscen)); TRY(s->alloc(&a.fdelta, nscen));
         TRY(s->alloc(&a.cstart, nscen + 1)); TRY(s->alloc(&a.fstart, nscen + 1));
-        CK(cudaMemset(a.count, 0, sizeof(int) * 3));
+        CK(cudaMemset(a.count, 0, sizeof(int) * 5));
         a.cell_off = s->d_cell_off; a.face_off = s->d_face_off;
+        TRY(s->alloc(&s->work.limited, nc));
+        if (precision == BRX_FP64) {
+            double2 *p_cw;
+            double *p_rarea;
+            TRY(s->alloc(&p_cw, nadj)); TRY(s->alloc(&p_rarea, nc));
+            // on the default stream, which follows the uploads
+            k64_weights<<<std::max(1, std::min((nc + 255) / 256, s->sms * 32)), 256>>>(m, p_cw, p_rarea);
+            CK(cudaGetLastError());
+            CK(cudaStreamSynchronize(nullptr));
+            s->work.cw = p_cw; s->work.rarea = p_rarea;
+        }
         s->small64 = precision == BRX_FP64 && s->maxdeg <= 4;
         if (s->small64) {
             // the cell sweep's tables, formed on the device from the uploaded
@@ -1084,15 +1097,14 @@ static int max_block(const brx_solver *s, int kind)
     const bool small = s->maxdeg <= 4;
     const void *fn = nullptr;
     switch (kind) {
-    case K_DRAG: fn = (const void *)k_open_drag<double>; break;
+    case K_DRAG: fn = (const void *)k_open_drag; break;
     case K_CELLS:
         fn = s->maxdeg <= 3 ? (const void *)k64_cells<3> : small ? (const void *)k64_cells<4>
                             : (const void *)k_cells<double, MAX_CELL_FACES>;
         break;
     case K_FACES: fn = (const void *)k64_faces; break;
-    case K_GATHER: fn = (const void *)k_gather; break;
     case K_LIMIT: fn = (const void *)k_limit; break;
-    case K_UPDATE: fn = (const void *)k_update<double>; break;
+    case K_UPDATE: fn = (const void *)k64_update; break;
     case K_HKT_GRAD: fn = (const void *)k_hkt_gradients; break;
     case K_HKT_FACES: fn = (const void *)k_hkt_faces; break;
     case KH_CELLS_SHAPE:
@@ -1537,7 +1549,7 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
     if (s->precision == BRX_MIXED) return mixed_kernel(make_launch(s, st), kind, stage, rate_out);
     switch (kind) {
     case K_DRAG:
-        k_open_drag<double><<<SSHAPE(K_DRAG, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl,
+        k_open_drag<<<SSHAPE(K_DRAG, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl,
                                                              s->method == BRX_METHOD_FWAVE ? s->c64.prim[0] : nullptr);
         return 1;
     case K_BOUNDARY:
@@ -1555,16 +1567,16 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
         k64_faces<<<SSHAPE(K_FACES, s->nf), 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, s->work, stage,
                                                     s->has_turb ? s->turb.trace : nullptr, s->turb.hkt);
         return 1;
-    case K_GATHER:
-        k_gather<<<SSHAPE(K_GATHER, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
-        return 1;
     case K_LIMIT:
         k_limit<<<SSHAPE(K_LIMIT, s->nf), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
         return 1;
     case K_UPDATE:
-        k_update<double><<<SSHAPE(K_UPDATE, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage, rate_out,
-                                                        s->turb, s->has_turb, s->c64.prim[1]);
-        return 1;
+        // the gather is part of the update; then the cells it found limited
+        k64_update<<<SSHAPE(K_UPDATE, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage, rate_out, s->turb,
+                                                       s->has_turb, s->c64.prim[1]);
+        k_limited<<<std::max(1, std::min((s->nc + 63) / 64, 2 * s->sms)), 64, 0, st>>>(
+            s->mesh, s->state, s->d_ctrl, s->work, stage, rate_out, s->turb, s->has_turb, s->c64.prim[1]);
+        return 2;
     }
     return 0;
 }
@@ -1606,7 +1618,8 @@ static void enqueue_stage(brx_solver *s, int stage, double *rate_out)
         // the mixed face sweep computes the rotor face terms in its tail: it
         // needs the rotor cell terms (wet gradients, actuator sink) first
         if (fork && mixed) cudaStreamWaitEvent(s->stream, s->join2, 0);
-        // the donor limiter runs inside the update (owner computes): no limit pass
+        // the donor limiter runs inside the update (owner computes): no limit
+        // pass, and in the FP64 form no separate gather
         for (int kind : {(int)K_FACES, (int)K_GATHER})
             s->launches += launch_kernel(s, kind, stage, nullptr);
         if (fork && !mixed) cudaStreamWaitEvent(s->stream, s->join2, 0);
@@ -1699,7 +1712,7 @@ static void host_set_trial(Ctrl &c)
     c.truncated = c.trial < c.hint * (1 - 1e-12);
     c.status1 = c.status2 = 0;
     c.peak1 = c.peak2 = 0ull;
-    c.g16r = 1. / (16. * c.grav);
+    c.g16r = 1. / (16. * c.grav); c.rrough = 1. / c.roughness_value;
     c.gravf = float(c.grav); c.dryf = float(c.dry); c.trialf = float(c.trial);
     c.roughf = float(c.roughness_value); c.cfl1 = 0;
 }
@@ -2196,8 +2209,7 @@ constexpr size_t NA_REC = 0;
 constexpr size_t NA_WS = NA_REC + noalloc_align(sizeof(CellRec) * NOALLOC_MAX_CELLS);
 constexpr size_t NA_GF = NA_WS + noalloc_align(sizeof(double2) * NOALLOC_MAX_FACES);
 constexpr size_t NA_LIM = NA_GF + noalloc_align(sizeof(double4_32a) * NOALLOC_MAX_FACES);
-constexpr size_t NA_RATE = NA_LIM + noalloc_align(sizeof(double4_32a) * NOALLOC_MAX_FACES);
-constexpr size_t NA_THETA = NA_RATE + noalloc_align(sizeof(double) * 3 * NOALLOC_MAX_CELLS);
+constexpr size_t NA_THETA = NA_LIM + noalloc_align(sizeof(double4_32a) * NOALLOC_MAX_FACES);
 constexpr size_t NA_CSID = NA_THETA + noalloc_align(sizeof(double) * NOALLOC_MAX_CELLS);
 constexpr size_t NA_CFLAGS = NA_CSID + noalloc_align(sizeof(int) * NOALLOC_MAX_CELLS);
 constexpr size_t NA_FSID = NA_CFLAGS + noalloc_align(sizeof(int) * NOALLOC_MAX_CELLS);
@@ -2206,7 +2218,8 @@ constexpr size_t NA_BMODE = NA_BSLOT + noalloc_align(sizeof(int) * NOALLOC_MAX_F
 constexpr size_t NA_DUNIT = NA_BMODE + noalloc_align(sizeof(int) * NOALLOC_MAX_FACES);
 constexpr size_t NA_CTRL = NA_DUNIT + noalloc_align(sizeof(double) * 4 * NOALLOC_MAX_FACES);
 constexpr size_t NA_ACT = NA_CTRL + noalloc_align(sizeof(Ctrl));
-constexpr size_t NOALLOC_BYTES = NA_ACT + noalloc_align(sizeof(int) * 16);   // about 7.4 MB
+constexpr size_t NA_LIMITED = NA_ACT + noalloc_align(sizeof(int) * 16);
+constexpr size_t NOALLOC_BYTES = NA_LIMITED + noalloc_align(sizeof(int) * NOALLOC_MAX_CELLS);   // about 7.1 MB
 
 static __device__ __align__(256) unsigned char brx_noalloc_scratch[NOALLOC_BYTES];
 
@@ -2262,13 +2275,13 @@ static int noalloc_address(unsigned char **out)
 }
 
 // The control block and the one-scenario active set: one run {count 1, nc,
-// nf}, cell run {start 0, nc; delta 0}, face run {0, nf; 0}, packed ranges
-// {0, nc} and {0, nf}.
+// nf} with no limited cells, cell run {start 0, nc; delta 0}, face run {0, nf;
+// 0}, packed ranges {0, nc} and {0, nf}.
 __global__ void k_noalloc_ctrl(Ctrl *ctrl, Ctrl init, int *act, int nc, int nf)
 {
     *ctrl = init;
-    const int v[13] = {1, nc, nf, 0, nc, 0, 0, nf, 0, 0, nc, 0, nf};
-    for (int i = 0; i < 13; ++i) act[i] = v[i];
+    const int v[15] = {1, nc, nf, 0, 0, 0, nc, 0, 0, nf, 0, 0, nc, 0, nf};
+    for (int i = 0; i < 15; ++i) act[i] = v[i];
 }
 
 // Derived per-cell/per-face tables of a closed single-scenario mesh, and a
@@ -2347,9 +2360,9 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     m.normal = normal; m.length = length; m.area = area; m.ls_matrix = ls_matrix; m.ls_weight = ls_weight;
     m.ls_delta = ls_delta; m.disp = displacement; m.disp_unit = disp_unit; m.disp_len = displacement_length;
     m.distance = distance;
-    int *act = (int *)(base + NA_ACT);   // count[3] cstart[2] cdelta[1] fstart[2] fdelta[1] cell_off[2] face_off[2]
-    m.act.count = act; m.act.cstart = act + 3; m.act.cdelta = act + 5; m.act.fstart = act + 6;
-    m.act.fdelta = act + 8; m.act.cell_off = act + 9; m.act.face_off = act + 11;
+    int *act = (int *)(base + NA_ACT);   // count[5] cstart[2] cdelta[1] fstart[2] fdelta[1] cell_off[2] face_off[2]
+    m.act.count = act; m.act.cstart = act + 5; m.act.cdelta = act + 7; m.act.fstart = act + 8;
+    m.act.fdelta = act + 10; m.act.cell_off = act + 11; m.act.face_off = act + 13;
     StateDev sd{};
     sd.q[0] = const_cast<double *>(q);
     sd.work = const_cast<double *>(q);    // the residual reads its stage state here and never writes it
@@ -2359,13 +2372,13 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     w.ws = (double2 *)(base + NA_WS);
     w.gf = (double4_32a *)(base + NA_GF);
     w.lim = (double4_32a *)(base + NA_LIM);
-    w.rate = (double *)(base + NA_RATE);
     w.theta = (double *)(base + NA_THETA);
+    w.limited = (int *)(base + NA_LIMITED);
     BoundaryDev b{};
     Ctrl init{};
     init.grav = gravity; init.dry = dry; init.cfl = cfl; init.speed_limit = 50.0;
     init.roughness_mode = 1; init.roughness_value = 1.0; init.active = 1;
-    init.g16r = 1. / (16. * gravity);
+    init.g16r = 1. / (16. * gravity); init.rrough = 1.;
     init.dt_outer = dt; init.hint = dt; init.trial = dt; init.max_substeps = 1;
     // Every field the residual reads is rewritten here: the array keeps the
     // previous call's contents, and calls that overlap on the GPU race on it.
@@ -2374,9 +2387,9 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     k_noalloc_tables<<<(n + 255) / 256, 256, 0, st>>>(m, ctrl, cell_sid, cflags, face_sid, bslot, bmode, disp_unit);
     k_cells<double, MAX_CELL_FACES><<<(nc + 127) / 128, 128, 0, st>>>(m, sd, ctrl, w, 1);
     k64_faces<<<(nf + 127) / 128, 128, 0, st>>>(m, sd, b, ctrl, w, 1, nullptr, nullptr);
-    k_gather<<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1);
+    k64_update<<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);
+    k_limited<<<(nc + 63) / 64, 64, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);
     k_limit<<<(nf + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1);
-    k_update<double><<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);
     k_noalloc_water<<<(nf + 255) / 256, 256, 0, st>>>(m, w, ctrl, water);
     CK(cudaGetLastError());
     Ctrl out{};

@@ -79,7 +79,7 @@ struct Ctrl {
     // inequality), which scales its roundoff allowance
     double bflux[2], ledger;
     double bgross[2], gross;
-    double g16r;                            // 1 / (16 grav), the two-rarefaction depth's factor
+    double g16r, rrough;                    // 1 / (16 grav) (two-rarefaction depth), 1 / roughness_value
     // FP32 copies for the mixed form's sweeps, refreshed with every trial
     float gravf, dryf, trialf, roughf;
     int cfl1, pad1;                         // stage 1 exceeded the CFL limit (mixed form, set after its gather)
@@ -95,7 +95,7 @@ struct Ctrl {
 // host sets it at the start of an interval; k_control rebuilds it after every
 // trial (ascending scenario order).
 struct ActiveDev {
-    int *count;              // [0] runs, [1] cells, [2] faces
+    int *count;              // [0] runs, [1] cells, [2] faces; [3], [4] cells limited in stage 1, 2
     int *cstart, *cdelta;    // (nscen+1), (nscen): per run, its first packed active cell index, and cell id - index
     int *fstart, *fdelta;    // the same for faces
     const int *cell_off, *face_off;   // (nscen+1) packed ranges of every scenario
@@ -247,6 +247,9 @@ struct Work {
     double4_32a *lim;            // (nf) limited water, momentum correction x,y
     double *rate;            // (3,nc)
     double *theta;           // (nc)
+    int *limited;            // (nc) cells whose outflow the stage's update limits, in any order
+    const double2 *cw;       // (nadj) signed length / area, length; null: formed per use
+    const double *rarea;     // (nc) RN(1 / area), with cw
 };
 
 __device__ __forceinline__ void atomic_max_nonneg(unsigned long long *addr, double v)

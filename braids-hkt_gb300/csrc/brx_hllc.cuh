@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(256) k_hllc_update(MeshDev m, StateDev s, Hllc
             bad = bad || !isfinite(v1) || !isfinite(v2);
         }
         if (bad) { raise_status(ct, 1, ST_ENDPOINT); continue; }
-        drag_cell<double>(ct, .5 * dt, v0, v1, v2);
+        drag_cell(ct, .5 * dt, v0, v1, v2);
         double *out = ct.cur ? s.q[0] : s.q[1];
         out[c] = v0; out[nc + c] = v1; out[2 * nc + c] = v2;
     }

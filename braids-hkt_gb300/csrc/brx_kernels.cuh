@@ -29,21 +29,26 @@ __device__ __forceinline__ F chezy(int method, F depth, F value)
     return F(18.) * log10(F(12.) * fmax(F(.5), depth / value));
 }
 
-// Depth stays FP64; the friction factor is evaluated in F.
-template <class F>
+// The depth's sixth root of Manning's law is cbrt(sqrt(h)) (25 FP64
+// instructions, good to about one ulp) instead of pow (88, two ulp), and the
+// quotients go through quotient(), correctly rounded as the divisions they
+// replace: 61 instructions instead of 145. Error of the factor over depths 1e-6
+// to 20 m: rms 1.2e-16, largest 7.5e-16 (with pow 1.8e-16 and 1.1e-15). The
+// opening half-step takes 57 us instead of 97 on 302k cells, 13 instead of 18
+// on 360.
 __device__ __forceinline__ void drag_cell(const Ctrl &ct, double dt, double &h, double &hu, double &hv)
 {
-    if (h <= ct.dry) { hu = 0.; hv = 0.; return; }
-    const F hf = F(h), uf = F(hu), vf = F(hv);
-    const F c = chezy<F>(ct.roughness_mode, hf, F(ct.roughness_value));
-    const F speed = sqrt(uf * uf + vf * vf) / hf;
-    const F factor = F(1.) / (F(1.) + F(dt) * F(ct.grav) * speed / (c * c * hf));
+    if (!greater(h, ct.dry)) { hu = 0.; hv = 0.; return; }
+    const double c = ct.roughness_mode == 2 ? quotient(cbrt(sqrt(h)), ct.roughness_value, ct.rrough)
+                                            : chezy<double>(ct.roughness_mode, h, ct.roughness_value);
+    const double speed = quotient(sqrt(hu * hu + hv * hv), h, reciprocal(h)), stiff = c * c * h;
+    const double y = 1. + quotient(dt * ct.grav * speed, stiff, reciprocal(stiff));
+    const double factor = quotient(1., y, reciprocal(y));
     hu *= factor;
     hv *= factor;
 }
 
 // work = drag(accepted, trial/2); prim (may be null): the first stage's primitives
-template <class F>
 __global__ void k_open_drag(MeshDev m, StateDev s, Ctrl *ctrl, Prim64 *prim)
 {
     const int nc = m.nc;
@@ -52,7 +57,7 @@ __global__ void k_open_drag(MeshDev m, StateDev s, Ctrl *ctrl, Prim64 *prim)
         if (!ct.active || ct.done) continue;
         const double *q = ct.cur ? s.q[1] : s.q[0];
         double h = q[c], hu = q[nc + c], hv = q[2 * nc + c];
-        drag_cell<F>(ct, .5 * ct.trial, h, hu, hv);
+        drag_cell(ct, .5 * ct.trial, h, hu, hv);
         s.work[c] = h; s.work[nc + c] = hu; s.work[2 * nc + c] = hv;
         if (prim) put_prim64(prim, c, h, hu, hv, s.z[c], ct.dry);
     }
@@ -1732,65 +1737,6 @@ __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl
     }
 }
 
-// ---------------------------------------------------------------------------
-// Gather: rate, donor inventory / boundary reservation, CFL frequency.
-// ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_gather(MeshDev m, StateDev s, Ctrl *ctrl, Work w, int stage)
-{
-    const int nc = m.nc;
-    const int stride = gridDim.x * blockDim.x;
-    // warp-uniform trip count: every lane reaches the warp reduction below
-    const int na = m.act.count[1];
-    for (int first = blockIdx.x * blockDim.x; first < na; first += stride) {   // warp-uniform trip count
-        const int c = first + (int)threadIdx.x < na ? active_cell(m.act, first + threadIdx.x) : nc;
-        bool have = false;
-        double fr = 0.;
-        int sid = 0;
-        if (c < nc) {
-            sid = m.cell_sid[c];
-            Ctrl &ct = ctrl[sid];
-            if (!skip_stage(ct, stage)) {
-                const double *base = stage == 1 ? s.work : s.q1;
-                const double dt = ct.trial, area = m.area[c];
-                const bool active = w.rec[c].flags & 2;
-                double sum0 = 0., sum1 = 0., sum2 = 0., out = 0., freq = 0., ext = 0., interior = 0.;
-                const bool owns_open = m.cflags[c] & 1;
-                for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
-                    const int f = m.faces[k];
-                    const double len = m.length[f];
-                    const double wt = len / area;
-                    const double2 ws = w.ws[f];
-                    const double4_32a gf = w.gf[f];
-                    if (m.signs[k] > 0) { sum0 += wt * ws.x; sum1 += wt * gf.x; sum2 += wt * gf.y; }
-                    else { sum0 -= wt * ws.x; sum1 -= wt * gf.z; sum2 -= wt * gf.w; }
-                    const double debit = fmax(m.signs[k] * ws.x, 0.) * len;
-                    out += debit;
-                    if (owns_open) { if (m.bslot[f] >= 0) ext += debit; else interior += debit; }
-                    freq += len * ws.y;
-                }
-                double r0 = 0., r1 = 0., r2 = 0.;
-                if (active) { r0 = -sum0; r1 = -sum1; r2 = -sum2; }
-                w.rate[c] = r0; w.rate[nc + c] = r1; w.rate[2 * nc + c] = r2;
-                double theta = 1.;
-                if (out > 0. && dt * out >= base[c] * area)
-                    theta = fmin(1., base[c] * area / (dt * out)) * (1. - 32. * 2.2204460492503131e-16);
-                if (owns_open) {
-                    const double available = base[c] * area / dt;
-                    if (ext > available) raise_status(ct, stage, ST_BUDGET);
-                    const double factor = fmin(1., (available - ext) / fmax(interior, 1e-300)) * (1. - 32. * EPS);
-                    theta = (interior > 0. && interior >= available - ext) ? factor : 1.;
-                }
-                w.theta[c] = theta;
-                fr = freq / area;
-                if (isnan(fr)) raise_status(ct, stage, ST_FREQ);
-                else have = true;
-            }
-        }
-        unsigned long long *peak0 = stage == 1 ? &ctrl[0].peak1 : &ctrl[0].peak2;
-        warp_max_peak(peak0, sizeof(Ctrl), sid, have, fr);
-    }
-}
-
 // midpoint_faces: limit donor outflow, carry the removed advective momentum.
 __global__ void __launch_bounds__(256) k_limit(MeshDev m, StateDev s, Ctrl *ctrl, Work w, int stage)
 {
@@ -1900,73 +1846,6 @@ __device__ __forceinline__ void add_viscosity(const MeshDev &m, const ViscDev &v
     r2 += 1. * y / area;
 }
 
-// midpoint_gather + stage combination (+ closing drag on the second stage).
-// With rate_out set, the final rate is stored there and no state is written.
-// Owner computes: each cell forms the donor-limited flux of its faces itself
-// (midpoint_faces, river_midpoint.h:30-41), with the same operations as
-// k_limit, so both cells of a face use the same value and no limited-flux
-// buffer goes through memory (k_limit still fills one for the water output
-// of a single residual).
-template <class F>
-__global__ void __launch_bounds__(256) k_update(MeshDev m, StateDev s, Ctrl *ctrl, Work w, int stage,
-                                                double *rate_out, TurbDev t, int turb, Prim64 *prim)
-{
-    const int nc = m.nc;
-    const double *q = stage == 1 ? s.work : s.q1;
-    FOR_ACTIVE_CELLS(m.act, c) {
-        const int sid = m.cell_sid[c];
-        Ctrl &ct = ctrl[sid];
-        if (skip_stage(ct, stage)) continue;
-        const double area = m.area[c];
-        double mass = 0., mx = 0., my = 0.;
-        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
-            const int f = m.faces[k];
-            const double wt = m.signs[k] * m.length[f] / area;
-            double water = w.ws[f].x;
-            if (water != 0. && m.bslot[f] < 0) {
-                const int donor = water < 0. ? m.neighbour[f] : m.owner[f];
-                if (donor >= 0) {
-                    const double th = w.theta[donor];
-                    if (th != 1.) {
-                        const double delta = (th - 1.) * water;
-                        water *= th;
-                        const double hd = q[donor];
-                        if (hd > ct.dry) {
-                            mx -= wt * (delta * q[nc + donor] / hd);
-                            my -= wt * (delta * q[2 * nc + donor] / hd);
-                        }
-                    }
-                }
-            }
-            mass -= wt * water;
-        }
-        const double r0 = mass;
-        double r1 = w.rate[nc + c] + mx, r2 = w.rate[2 * nc + c] + my;
-        if (turb && t.hkt[sid]) add_rotor_momentum(m, t, sid, c, area, r1, r2);
-        if (w.visc.nu && w.visc.nu[sid] > 0.) add_viscosity(m, w.visc, c, area, r1, r2);
-        if (!isfinite(r0) || !isfinite(r1) || !isfinite(r2)) raise_status(ct, stage, ST_RATE);
-        if (rate_out) { rate_out[c] = r0; rate_out[nc + c] = r1; rate_out[2 * nc + c] = r2; continue; }
-        const double dt = ct.trial, dry = ct.dry;
-        if (stage == 1) {
-            const double h = s.work[c] + dt * r0;
-            double hu = s.work[nc + c] + dt * r1, hv = s.work[2 * nc + c] + dt * r2;
-            if (h < 0) raise_status(ct, 1, ST_ENDPOINT);
-            if (h <= dry) { hu = 0.; hv = 0.; }
-            s.q1[c] = h; s.q1[nc + c] = hu; s.q1[2 * nc + c] = hv;
-            if (prim) put_prim64(prim, c, h, hu, hv, s.z[c], dry);   // the second stage's
-        } else {
-            double h = .5 * s.work[c] + .5 * (s.q1[c] + dt * r0);
-            double hu = .5 * s.work[nc + c] + .5 * (s.q1[nc + c] + dt * r1);
-            double hv = .5 * s.work[2 * nc + c] + .5 * (s.q1[2 * nc + c] + dt * r2);
-            if (!isfinite(h) || !isfinite(hu) || !isfinite(hv) || h < 0) raise_status(ct, 2, ST_ENDPOINT);
-            if (h <= dry) { hu = 0.; hv = 0.; }
-            drag_cell<F>(ct, .5 * dt, h, hu, hv);
-            double *qn = ct.cur ? s.q[0] : s.q[1];
-            qn[c] = h; qn[nc + c] = hu; qn[2 * nc + c] = hv;
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
 // Control: accept/reject the trial and set the next one (RiverExplicit.advance).
 // ---------------------------------------------------------------------------
@@ -2018,6 +1897,7 @@ __device__ void active_rebuild(const Ctrl *ctrl, int nscen, const ActiveDev &a)
     if (lane == 0) {
         a.cstart[nrun] = ncell; a.fstart[nrun] = nface;
         a.count[0] = nrun; a.count[1] = ncell; a.count[2] = nface;
+        a.count[3] = a.count[4] = 0;
     }
 }
 

@@ -37,6 +37,17 @@ __device__ __forceinline__ double quotient(double x, double y, double r)
     return __fma_rn(__fma_rn(-y, q, x), r, q);
 }
 
+// 1 / y to about an ulp, for quotient(): the hardware's approximation (PTX
+// rcp.approx.ftz.f64, relative error below 2^-20) and two Newton-Raphson steps;
+// four FP64 instructions instead of a division's ten. y normal and finite.
+__device__ __forceinline__ double reciprocal(double y)
+{
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(y));
+    r = __fma_rn(__fma_rn(-y, r, 1.), r, r);
+    return __fma_rn(__fma_rn(-y, r, 1.), r, r);
+}
+
 // FP32 image of a double by truncation, on the integer pipe (a conversion
 // instruction runs on the FP64 pipe): relative error below 2^-23, values
 // below the FP32 normal range become 0, those above it the largest float.
@@ -59,7 +70,7 @@ __device__ __forceinline__ void put_prim64(Prim64 *P, int c, double h, double hu
     Prim64 p;
     p.eta = h + z; p.h = h;
     if (greater(h, dry)) {
-        const double r = 1. / h;
+        const double r = reciprocal(h);
         p.u = quotient(hu, h, r); p.v = quotient(hv, h, r);
     } else {
         // a nonfinite momentum of a dry cell fails the stage as in a wet one

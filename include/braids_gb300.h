@@ -428,7 +428,7 @@ int brx_fma_rate(int precision, double *tflops, double *ms);
  * out as for brx_solver_create and brx_rate; status and freq are host
  * pointers (may be NULL). At most 16384 cells and 32768 faces: larger meshes
  * get BRX_ERR_UNSUPPORTED. The stage scratch is one static device array of
- * about 7.4 MB that every GPU loading this library holds until process exit.
+ * about 7.1 MB that every GPU loading this library holds until process exit.
  * The first call in each CUDA context (each device's primary context, and
  * again after a cudaDeviceReset, which loads the module anew) looks up that
  * array's device address (cudaGetSymbolAddress) with the device current;
