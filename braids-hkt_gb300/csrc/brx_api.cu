@@ -73,6 +73,7 @@ struct brx_solver {
     std::vector<double> hint;
     std::vector<int> active;
     std::vector<int> cell_offset, face_offset, seg_offset;
+    std::vector<int> seg_faces;      // open faces per segment
     std::vector<int> h_bid, h_owner, h_neighbour, h_slot_face, h_offset;
     std::vector<double> h_length, h_area;   // host copies for the mixed HLLC stencil tables
     int *d_bmode_rw = nullptr;       // writable alias of mesh.bmode
@@ -248,6 +249,7 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
         s->face_offset.assign(face_offset, face_offset + nscen + 1);
         s->seg_offset.assign(nscen + 1, 0);
         if (nseg) s->seg_offset.assign(seg_offset, seg_offset + nscen + 1);
+        for (int sg = 0; sg < nseg; ++sg) s->seg_faces.push_back(boundary_offset[sg + 1] - boundary_offset[sg]);
         s->h_bid.assign(bid, bid + nf);
         s->h_owner.assign(owner, owner + nf);
         s->h_neighbour.assign(neighbour, neighbour + nf);
@@ -342,7 +344,8 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
         double *p_forcing, *p_terms, *p_trace, *p_flux, *p_sums;
         TRY(s->alloc(&p_forcing, 2 * (size_t)nseg)); TRY(s->alloc(&p_terms, 3 * (size_t)s->nslot));
         TRY(s->alloc(&p_trace, 3 * (size_t)s->nslot)); TRY(s->alloc(&p_flux, 3 * (size_t)s->nslot));
-        TRY(s->alloc(&p_sums, 3 * (size_t)nseg));
+        TRY(s->alloc(&p_sums, 3 * (size_t)nseg)); TRY(s->alloc(&b.own_sum, s->nown));
+        b.cluster = 1;
         b.seg_mode = s->d_seg_mode_rw; b.stage_policy = s->d_stage_policy_rw; b.ext_bed = s->d_ext_bed_rw;
         b.forcing = p_forcing; b.terms = p_terms; b.trace = p_trace; b.flux = p_flux; b.seg_sums = p_sums;
         b.table_len = 0; b.table_time = nullptr; b.table_value = nullptr;
@@ -551,7 +554,19 @@ extern "C" int brx_boundary_set(brx_solver *s, const int *seg_mode, const int *s
     }
     s->h_seg_mode.assign(seg_mode, seg_mode + nseg);
     const int inlet = std::count(seg_mode, seg_mode + nseg, 9) > 0;
-    if (inlet != s->bnd.inlet) { s->bnd.inlet = inlet; s->graph_dirty = true; }
+    // blocks per scenario of the boundary kernel: one for 128 faces (a block has
+    // a warp per sub-partition), at most the portable cluster of eight; section
+    // solves work in a single block
+    int sections = 0, widest = 0, cluster = 1;
+    for (int sg = 0; sg < nseg; ++sg) sections |= seg_mode[sg] != 2 && seg_mode[sg] != 3 && seg_mode[sg] != 6;
+    for (int i = 0; i < s->nscen; ++i) {
+        int faces = 0;
+        for (int sg = s->seg_offset[i]; sg < s->seg_offset[i + 1]; ++sg) faces += s->seg_faces[sg];
+        widest = std::max(widest, faces);
+    }
+    while (!sections && cluster < 8 && widest > 128 * cluster) cluster *= 2;
+    if (inlet != s->bnd.inlet || sections != s->bnd.sections || cluster != s->bnd.cluster) s->graph_dirty = true;
+    s->bnd.inlet = inlet; s->bnd.sections = sections; s->bnd.cluster = cluster;
     TRY(clear_inlet_lines(s));
     std::vector<int> bmode(nf, 0);
     std::vector<double> ext(std::max(s->nslot, 1));
@@ -1554,7 +1569,7 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
         return 1;
     case K_BOUNDARY:
         if (!s->nslot) return 0;
-        k_boundary<double><<<s->nscen, 256, 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, stage);
+        launch_boundary<double>(s->mesh, s->state, s->bnd, s->d_ctrl, s->nscen, stage, st);
         return 1;
     case K_CELLS:
         if (s->maxdeg <= 3)
@@ -1658,7 +1673,7 @@ static int launch_hllc(brx_solver *s, int kind, cudaStream_t st = nullptr)
         return 1;
     case KH_BOUNDARY:
         if (!s->nslot) return 0;
-        k_boundary<double><<<s->nscen, 256, 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, STAGE_HANCOCK);
+        launch_boundary<double>(s->mesh, s->state, s->bnd, s->d_ctrl, s->nscen, STAGE_HANCOCK, st);
         return 1;
     case KH_FACES:
         k_hllc_faces<<<SSHAPE(KH_FACES_SHAPE, s->nf), 0, st>>>(s->mesh, s->bnd, rec, s->work, s->turb, s->has_turb, s->d_ctrl);

@@ -189,7 +189,10 @@ struct BoundaryDev {
     const double *table_time;   // (table_len)
     const double *table_value;  // (2, nseg, table_len)
     const int *own_cell, *own_off, *own_slot;  // unique owners, CSR into slots (boundary order)
-    double *terms;           // (3, nslot) scratch: stage terms and weights
+    double *terms;           // (3, nslot) scratch: tile sums / inlet factors, -, conveyance weights
+    double2 *own_sum;        // (nown) water and gross sums of 32 owners from each
+    int cluster;             // blocks per scenario of the boundary kernel
+    int sections;            // a segment needs a section solve (modes 4, 5, 9, 10, 11)
     double *trace, *flux;    // (3, nslot) each
     double *seg_sums;        // (3, nseg): wetted stage sum, wetted width, weight total
     const int *rt_off;       // (nseg+1) Q-H rating knots per mode-11 segment

@@ -8,6 +8,7 @@
 // evaluate exactly the FP64 expressions of the reference.
 #pragma once
 #include "brx_common.cuh"
+#include <cooperative_groups.h>
 #include "brx_num64.cuh"
 
 #ifndef BRX_NS
@@ -79,13 +80,29 @@ __device__ __forceinline__ F exterior_chezy(int mode, F h, F parameter, F floor_
                  : sqrt(gravity) / F(.41) * log1p(F(30.) * d / (exp(F(1.)) * parameter));
 }
 
-__device__ __forceinline__ void stage_wave(double h, double un, double target, double gravity, double &depth,
+// Conveyance weight per unit width of an inlet face: section^1.5 times
+// Chezy's coefficient at depth h (at least the dry depth). In FP64 the powers
+// are section sqrt(section) and cbrt(sqrt(h)): 36 FP64 instructions instead of
+// 176, each good to about one ulp.
+template <class F>
+__device__ __forceinline__ double conveyance(int mode, int waqua, F section, F h, const Ctrl &ct)
+{
+    if constexpr (sizeof(F) == 8) {
+        const double chezy = mode == 2 ? quotient(cbrt(sqrt(h)), ct.roughness_value, ct.rrough)
+                                       : exterior_chezy<F>(mode, h, ct.roughness_value, ct.dry, ct.grav, waqua);
+        return section * sqrt(section) * chezy;
+    } else
+        return double(pow(section, F(1.5)) *
+                      exterior_chezy<F>(mode, h, F(ct.roughness_value), F(ct.dry), F(ct.grav), waqua));
+}
+
+// c = sqrt(gravity h)
+__device__ __forceinline__ void stage_wave(double h, double un, double target, double gravity, double c, double &depth,
                                            double &velocity)
 {
-    const double c = sqrt(gravity * h);
     depth = h; velocity = un;
     if (target > h) {
-        const double k = sqrt(.5 * gravity * (1. / target + 1. / h));
+        const double k = sqrt(.5 * gravity * (quotient(1., target, reciprocal(target)) + quotient(1., h, reciprocal(h))));
         const double shock = un - target * k;
         if (shock >= 0.) return;
         depth = target; velocity = un - (target - h) * k;
@@ -105,36 +122,40 @@ __device__ __forceinline__ bool is_outlet(int mode)
     return mode == 2 || mode == 3 || mode == 4 || mode == 5 || mode == 10 || mode == 11;
 }
 
-// Sums of field `row` of b.terms over each segment of the scenario, in the
-// 64-tile tree. Called by all threads of the CTA; result in b.seg_sums[out_row].
-__device__ void segment_sums(const BoundaryDev &b, int s0, int s1, int row, int out_row, double *tile_buf)
+// The scenario's slots in tiles of 64 from each segment start.
+__device__ __forceinline__ int tile_count(const BoundaryDev &b, int sg)
 {
-    // tile partials: one thread per (segment, tile)
-    int ntile_total = 0;
-    for (int s = s0; s < s1; ++s) ntile_total += max(1, (b.seg_off[s + 1] - b.seg_off[s] + 63) / 64);
-    for (int t = threadIdx.x; t < ntile_total; t += blockDim.x) {
-        int s = s0, rem = t;
-        while (rem >= max(1, (b.seg_off[s + 1] - b.seg_off[s] + 63) / 64)) {
-            rem -= max(1, (b.seg_off[s + 1] - b.seg_off[s] + 63) / 64);
-            ++s;
-        }
-        const int start = b.seg_off[s] + 64 * rem, end = min(b.seg_off[s + 1], start + 64);
-        double sum = 0.;
-        for (int k = start; k < end; ++k) sum += b.terms[(size_t)row * b.nslot + k];
-        tile_buf[t] = sum;
-    }
-    __syncthreads();
-    for (int s = s0 + threadIdx.x; s < s1; s += blockDim.x) {
-        int first = 0;
-        for (int u = s0; u < s; ++u) first += max(1, (b.seg_off[u + 1] - b.seg_off[u] + 63) / 64);
-        const int nt = max(1, (b.seg_off[s + 1] - b.seg_off[s] + 63) / 64);
-        double total = 0.;
-        for (int t = 0; t < nt; ++t) total += tile_buf[first + t];
-        b.seg_sums[(size_t)out_row * b.nseg + s] = total;
-    }
-    __syncthreads();
+    return max(1, (b.seg_off[sg + 1] - b.seg_off[sg] + 63) / 64);
 }
 
+struct SlotTile { int sg, first, end; };
+
+__device__ __forceinline__ SlotTile slot_tile(const BoundaryDev &b, int s0, int t)
+{
+    int sg = s0;
+    for (int n = tile_count(b, sg); t >= n; n = tile_count(b, sg)) { t -= n; ++sg; }
+    const int first = b.seg_off[sg] + 64 * t;
+    return {sg, first, min(b.seg_off[sg + 1], first + 64)};
+}
+
+constexpr int BOUNDARY_THREADS = 128;      // one warp per sub-partition: FP64 work does not overlap within one
+
+// The sum of a tile's terms in slot order, formed by one warp: lane l's terms
+// are those of slots first + l and first + 32 + l; rows are summed by as many
+// lanes at once. Result of row r in lane r.
+template <int ROWS>
+__device__ __forceinline__ double tile_sum(double (*buf)[64], int n, const double (&lo)[ROWS], const double (&hi)[ROWS])
+{
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) { buf[r][lane] = lo[r]; buf[r][lane + 32] = hi[r]; }
+    __syncwarp();
+    double sum = 0.;
+    if (lane < ROWS)
+        for (int i = 0; i < n; ++i) sum += buf[lane][i];
+    __syncwarp();
+    return sum;
+}
 
 // ---------------------------------------------------------------------------
 // Q-H rating outlet (mode 11): the common water elevation at which the
@@ -177,7 +198,7 @@ __device__ double rating_residual(const MeshDev &m, const BoundaryDev &b, int sg
 }
 
 // 0, or the section failure: 1 no bracket, 2 residual, 3 a fictitious zero-flow root.
-__device__ int rating_section(const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry, double speed,
+__device__ __noinline__ int rating_section(const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry, double speed,
                               const double *q, const double *z, bool &bad)
 {
     const int nc = m.nc, nf = m.nf;
@@ -320,7 +341,7 @@ __device__ double nout_residual(const MeshDev &m, const BoundaryDev &b, const in
 }
 
 // 0, or the chain's failure (a trial rejection in the reference).
-__device__ int normal_chain(const MeshDev &m, const BoundaryDev &b, int ch, double g, double dry, double speed,
+__device__ __noinline__ int normal_chain(const MeshDev &m, const BoundaryDev &b, int ch, double g, double dry, double speed,
                             int law, double rough, const double *q, const double *z, bool &bad)
 {
     const int nc = m.nc, nf = m.nf;
@@ -438,156 +459,166 @@ __device__ int normal_chain(const MeshDev &m, const BoundaryDev &b, int ch, doub
 constexpr int SECTION_LANES = 128;
 
 struct SectionWork {
-    double part[6][SECTION_LANES];
-    double lo, hi, eta, residual, area, width, rate;
-    double velocity, gross, derivative, scale;
-    int error, done, stagnant, changed, count;
+    double part[4][SECTION_LANES];
+    double sum[4];
+    int error;
 };
+
+// Sums of the first ROWS rows of w.part over lanes 0 .. n-1 in lane order, one
+// thread per row in a warp of its own (their FP64 chains then run side by
+// side); every thread gets them. Lanes from n on hold nothing: the section has
+// n < SECTION_LANES faces. Block-cooperative.
+template <int ROWS>
+__device__ __forceinline__ void lane_sums(SectionWork &w, int n, double (&sum)[ROWS])
+{
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0)
+        for (int r = threadIdx.x >> 5; r < ROWS; r += blockDim.x >> 5) {
+            double t = 0.;
+            for (int lane = 0; lane < n; ++lane) t += w.part[r][lane];
+            w.sum[r] = t;
+        }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < ROWS; ++r) sum[r] = w.sum[r];
+}
+
+// Shrink [lo, hi], f(lo) >= 0 >= f(hi) and f decreasing, to neighbouring
+// numbers, where bisection ends. Each round evaluates the secant point and then
+// twice the distance it is still off, which as a rule is just across the root:
+// the width falls with the square, some twelve evaluations instead of
+// bisection's fifty-odd. A round that does not halve the interval bisects.
+template <class Fn>
+__device__ __forceinline__ void shrink_bracket(double &lo, double &hi, double flo, double fhi, const Fn &f)
+{
+    for (int round = 0; round < 90; ++round) {
+        const double mid = lo + .5 * (hi - lo);
+        if (mid == lo || mid == hi) return;
+        const double width = hi - lo, fall = flo - fhi;
+        double x = fall > 0. ? lo + width * (flo / fall) : mid;
+        if (!(x > lo && x < hi)) x = mid;
+        const double fx = f(x);
+        const bool left = fx > 0.;
+        if (left) { lo = x; flo = fx; } else { hi = x; fhi = fx; }
+        const double off = fall > 0. ? fmax(2. * fabs(fx) * (width / fall), 4. * EPS * fabs(x)) : width;
+        const double y = left ? x + off : x - off;
+        if (y > lo && y < hi) {
+            const double fy = f(y);
+            if (fy > 0.) { lo = y; flo = fy; } else { hi = y; fhi = fy; }
+        }
+        if (hi - lo > .5 * width) {
+            const double v = lo + .5 * (hi - lo);
+            if (v == lo || v == hi) return;
+            const double fv = f(v);
+            if (fv > 0.) { lo = v; flo = fv; } else { hi = v; fhi = fv; }
+        }
+    }
+}
 
 __device__ __forceinline__ double weir_velocity(double h, double hi, double ui, double g)
 {
     return h > hi ? ui - (h - hi) * sqrt(.5 * g * (1. / h + 1. / hi)) : ui + 2. * (sqrt(g * hi) - sqrt(g * h));
 }
 
-// river_exterior_outlet.h:207-227
-__device__ void weir_residual(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int k0, int k1, double eta,
-                              double g, double dry, double crest, double factor, const double *q, const double *z)
+// river_exterior_outlet.h:207-227: discharge minus the weir's at stage eta,
+// the same in every thread.
+__device__ __noinline__ double weir_residual(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int k0, int k1, double eta,
+                                double g, double dry, double crest, double factor, const double *q, const double *z)
 {
-    for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
-        double area = 0., width = 0., rate = 0.;
+    const int n = min(k1 - k0, SECTION_LANES);
+    for (int lane = threadIdx.x; lane < n; lane += blockDim.x) {
+        double rate = 0.;
         for (int k = k0 + lane; k < k1; k += SECTION_LANES) {
             if (!b.branch[k]) continue;
             const int f = b.slot_face[k], c = m.owner[f];
             const double bed = b.ext_bed[k], h = fmax(eta - bed, 0.), hi = fmax(q[c] + z[c] - bed, 0.);
             if (h <= dry) continue;
             const double u = fmax(weir_velocity(h, hi, b.invariant[k], g), 0.);
-            if (u > 0.) { area += h * m.length[f]; width += m.length[f]; rate += h * u * m.length[f]; }
+            if (u > 0.) rate += h * u * m.length[f];
         }
-        w.part[0][lane] = area; w.part[1][lane] = width; w.part[2][lane] = rate;
+        w.part[0][lane] = rate;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        w.area = w.width = w.rate = 0.;
-        for (int lane = 0; lane < SECTION_LANES; ++lane) {
-            w.area += w.part[0][lane]; w.width += w.part[1][lane]; w.rate += w.part[2][lane];
-        }
-        const double head = fmax(eta - crest, 0.);
-        w.residual = w.rate - factor * head * sqrt(head);
-    }
-    __syncthreads();
+    double sum[1];
+    lane_sums<1>(w, n, sum);
+    const double head = fmax(eta - crest, 0.);
+    return sum[0] - factor * head * sqrt(head);
 }
 
 // Free weir on segment sg (river_exterior_outlet.h:229-360): the common
 // subcritical stage at which the outgoing Lax-curve discharge equals
 // coefficient x width x head^1.5. Returns 0 or the section failure (a trial
 // rejection in the reference); `bad` gets the speed-limit face status.
-__device__ int weir_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
+__device__ __noinline__ int weir_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
                             double speed, const double *q, const double *z, bool &bad)
 {
     const int nc = m.nc, nf = m.nf, nseg = b.nseg, k0 = b.seg_off[sg], k1 = b.seg_off[sg + 1];
     const size_t ns = b.nslot;
     const double tol = 128. * EPS, crest = b.weir[sg], factor = b.weir[nseg + sg] * b.weir[2 * nseg + sg];
-    if (threadIdx.x == 0) { w.error = 0; w.done = 0; w.eta = 0.; w.area = w.width = w.rate = 0.; }
-    for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
-        double width = 0.;
-        for (int k = k0 + lane; k < k1; k += SECTION_LANES) {
-            const int f = b.slot_face[k], c = m.owner[f];
-            b.branch[k] = 0; b.invariant[k] = 0.;
-            const double h0 = q[c], h = fmax(h0 + z[c] - b.ext_bed[k], 0.);
-            if (h0 <= dry || h <= dry) continue;
-            const double un = (q[nc + c] * m.normal[f] + q[2 * nc + c] * m.normal[nf + f]) / h0;
-            b.branch[k] = 1; b.invariant[k] = un; width += m.length[f];
-        }
-        w.part[1][lane] = width;
+    if (threadIdx.x == 0) w.error = 0;
+    // wet faces, each with its incoming normal speed; the bracket of the stage
+    // from their sonic depths and their own levels (maxima: in any order)
+    double lo = -INFINITY, hi = -INFINITY;
+    bool some = false;
+    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+        const int f = b.slot_face[k], c = m.owner[f];
+        b.branch[k] = 0; b.invariant[k] = 0.;
+        const double hc = q[c], h0 = fmax(hc + z[c] - b.ext_bed[k], 0.);
+        if (hc <= dry || h0 <= dry) continue;
+        const double u = (q[nc + c] * m.normal[f] + q[2 * nc + c] * m.normal[nf + f]) / hc;
+        b.branch[k] = 1; b.invariant[k] = u;
+        some = true;
+        double left = 0., right = fmax(h0, 1.);
+        for (int it = 0; it < 60 && weir_velocity(right, h0, u, g) > sqrt(g * right); ++it) right *= 2.;
+        const auto f_sonic = [&](double h) { return weir_velocity(h, h0, u, g) - sqrt(g * h); };
+        shrink_bracket(left, right, f_sonic(left), f_sonic(right), f_sonic);
+        lo = fmax(lo, b.ext_bed[k] + right);
+        hi = fmax(hi, hc + z[c]);
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double width = 0.;
-        for (int lane = 0; lane < SECTION_LANES; ++lane) width += w.part[1][lane];
-        if (width == 0.) w.done = 1;
-    }
-    __syncthreads();
-    if (w.done) {
-        for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) b.branch[k] = 0;
-        __syncthreads();
-    } else {
-        for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
-            double lo = -INFINITY, hi = -INFINITY;
-            for (int k = k0 + lane; k < k1; k += SECTION_LANES) {
-                if (b.branch[k] != 1) continue;
-                const int c = m.owner[b.slot_face[k]];
-                const double h0 = fmax(q[c] + z[c] - b.ext_bed[k], 0.), u = b.invariant[k];
-                double left = 0., right = fmax(h0, 1.);
-                for (int it = 0; it < 60 && weir_velocity(right, h0, u, g) > sqrt(g * right); ++it) right *= 2.;
-                for (int it = 0; it < 70; ++it) {
-                    const double mid = .5 * (left + right);
-                    if (weir_velocity(mid, h0, u, g) > sqrt(g * mid)) left = mid; else right = mid;
-                }
-                lo = fmax(lo, b.ext_bed[k] + right);
-                hi = fmax(hi, q[c] + z[c]);
-            }
-            w.part[0][lane] = lo; w.part[1][lane] = hi;
-        }
+    double eta = 0.;
+    if (__syncthreads_or(some)) {
+        const int n = min(k1 - k0, (int)blockDim.x);
+        if ((int)threadIdx.x < n) { w.part[0][threadIdx.x] = lo; w.part[1][threadIdx.x] = hi; }
         __syncthreads();
         if (threadIdx.x == 0) {
-            w.lo = -INFINITY; w.hi = -INFINITY;
-            for (int lane = 0; lane < SECTION_LANES; ++lane) { w.lo = fmax(w.lo, w.part[0][lane]); w.hi = fmax(w.hi, w.part[1][lane]); }
-            w.lo = fmax(w.lo, crest);
-            w.hi = fmax(w.hi, w.lo + 1.);
+            for (int i = 0; i < n; ++i) { lo = fmax(lo, w.part[0][i]); hi = fmax(hi, w.part[1][i]); }
+            w.sum[0] = lo; w.sum[1] = hi;
         }
         __syncthreads();
-        weir_residual(w, m, b, k0, k1, w.lo, g, dry, crest, factor, q, z);
-        if (threadIdx.x == 0 && (w.residual < 0. || !isfinite(w.residual))) w.error = 1;
+        lo = fmax(w.sum[0], crest);
+        hi = fmax(w.sum[1], lo + 1.);
         __syncthreads();
-        if (!w.error) {
-            weir_residual(w, m, b, k0, k1, w.hi, g, dry, crest, factor, q, z);
-            for (int j = 0; j < 60 && w.residual > 0.; ++j) {
-                if (threadIdx.x == 0) w.hi = w.lo + 2. * (w.hi - w.lo);
-                __syncthreads();
-                weir_residual(w, m, b, k0, k1, w.hi, g, dry, crest, factor, q, z);
-            }
-            if (threadIdx.x == 0 && (w.residual > 0. || !isfinite(w.residual))) w.error = 1;
-            __syncthreads();
+        const auto residual = [&](double at) { return weir_residual(w, m, b, k0, k1, at, g, dry, crest, factor, q, z); };
+        int error = 0;
+        const double rlo = residual(lo);
+        double rhi = 0.;
+        if (rlo < 0. || !isfinite(rlo)) error = 1;
+        else {
+            rhi = residual(hi);
+            for (int j = 0; j < 60 && rhi > 0.; ++j) { hi = lo + 2. * (hi - lo); rhi = residual(hi); }
+            if (rhi > 0. || !isfinite(rhi)) error = 1;
         }
-        if (!w.error) {
-            for (int j = 0; j < 90; ++j) {
-                if (threadIdx.x == 0) { w.eta = w.lo + .5 * (w.hi - w.lo); w.stagnant = w.eta == w.lo || w.eta == w.hi; }
-                __syncthreads();
-                if (w.stagnant) break;
-                weir_residual(w, m, b, k0, k1, w.eta, g, dry, crest, factor, q, z);
-                if (threadIdx.x == 0) { if (w.residual > 0.) w.lo = w.eta; else w.hi = w.eta; }
-                __syncthreads();
+        if (!error) {
+            shrink_bracket(lo, hi, rlo, rhi, residual);
+            eta = lo + .5 * (hi - lo);
+            const double r = residual(eta), head = fmax(eta - crest, 0.), requested = factor * head * sqrt(head);
+            if (!isfinite(r) || fabs(r) > 1e-10 * fmax(requested, 1.)) error = 2;
+            bool inward = false;
+            for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
+                if (b.branch[k] != 1) continue;
+                const int c = m.owner[b.slot_face[k]];
+                const double bed = b.ext_bed[k], h0 = fmax(q[c] + z[c] - bed, 0.), h = fmax(eta - bed, 0.);
+                const double u = weir_velocity(h, h0, b.invariant[k], g);
+                if (h <= dry || u <= 0.) { b.branch[k] = 0; continue; }
+                // a downstream-only shock may not enter the domain
+                if (h > h0 && b.invariant[k] - h * sqrt(.5 * g * (1. / h + 1. / h0)) > tol) inward = true;
             }
-            if (threadIdx.x == 0) w.eta = w.lo + .5 * (w.hi - w.lo);
-            __syncthreads();
-            weir_residual(w, m, b, k0, k1, w.eta, g, dry, crest, factor, q, z);
-            if (threadIdx.x == 0) {
-                const double head = fmax(w.eta - crest, 0.), requested = factor * head * sqrt(head);
-                if (!isfinite(w.residual) || fabs(w.residual) > 1e-10 * fmax(requested, 1.)) w.error = 2;
-            }
-            __syncthreads();
-            for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
-                double count = 0.;
-                for (int k = k0 + lane; k < k1; k += SECTION_LANES) {
-                    if (b.branch[k] != 1) continue;
-                    const int c = m.owner[b.slot_face[k]];
-                    const double bed = b.ext_bed[k], hi = fmax(q[c] + z[c] - bed, 0.), h = fmax(w.eta - bed, 0.);
-                    const double u = weir_velocity(h, hi, b.invariant[k], g);
-                    if (h <= dry || u <= 0.) { b.branch[k] = 0; continue; }
-                    // a downstream-only shock may not enter the domain
-                    if (h > hi && b.invariant[k] - h * sqrt(.5 * g * (1. / h + 1. / hi)) > tol) count += 1.;
-                }
-                w.part[0][lane] = count;
-            }
-            __syncthreads();
-            if (threadIdx.x == 0)
-                for (int lane = 0; lane < SECTION_LANES; ++lane) if (w.part[0][lane] > 0.) w.error = 5;
-            __syncthreads();
+            if (__syncthreads_or(inward)) error = 5;
         }
+        if (error) return error;             // the same in every thread
+    } else {
+        for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) b.branch[k] = 0;
     }
-    const int error = w.error;
     __syncthreads();
-    if (error) return error;
     for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const int f = b.slot_face[k], c = m.owner[f];
         const double bed = b.ext_bed[k], h0 = q[c], geom = fmax(h0 + z[c] - bed, 0.);
@@ -609,7 +640,7 @@ __device__ int weir_section(SectionWork &w, const MeshDev &m, const BoundaryDev 
             }
             un = 0.;
         } else {
-            h = fmax(w.eta - bed, 0.);
+            h = fmax(eta - bed, 0.);
             un = weir_velocity(h, geom, b.invariant[k], g);
         }
         if (!isfinite(h) || !isfinite(un) || sqrt(un * un + tx * tx + ty * ty) > speed) { bad = true; continue; }
@@ -646,10 +677,14 @@ __device__ __forceinline__ double resolved_bed(const MeshDev &m, const BoundaryD
     return bed + (bounded - bed) * (1. - blend);
 }
 
-__device__ void crit_residual(SectionWork &w, const MeshDev &m, const BoundaryDev &b, const int *slots, int k0,
-                              int n, double eta, double g, double dry, const double *q, const double *z)
+// Controlled discharge minus sqrt(g A^3 / B) at stage eta, the same in every
+// thread; area, width out.
+__device__ __noinline__ double crit_residual(SectionWork &w, const MeshDev &m, const BoundaryDev &b, const int *slots, int k0,
+                                int n, double eta, double g, double dry, const double *q, const double *z, double &area,
+                                double &width_)
 {
-    for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
+    const int lanes = min(n, SECTION_LANES);
+    for (int lane = threadIdx.x; lane < lanes; lane += blockDim.x) {
         double a = 0., width = 0., rate = 0.;
         for (int i = lane; i < n; i += SECTION_LANES) {
             const int k = slots ? slots[i] : k0 + i;
@@ -661,14 +696,10 @@ __device__ void crit_residual(SectionWork &w, const MeshDev &m, const BoundaryDe
         }
         w.part[0][lane] = a; w.part[1][lane] = width; w.part[2][lane] = rate;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0., width = 0., rate = 0.;
-        for (int lane = 0; lane < SECTION_LANES; ++lane) { a += w.part[0][lane]; width += w.part[1][lane]; rate += w.part[2][lane]; }
-        w.area = a; w.width = width; w.rate = rate;
-        w.residual = rate - (width > 0. ? sqrt(g * a * a * a / width) : 0.);
-    }
-    __syncthreads();
+    double sum[3];
+    lane_sums<3>(w, lanes, sum);
+    area = sum[0]; width_ = sum[1];
+    return sum[2] - (sum[1] > 0. ? sqrt(g * sum[0] * sum[0] * sum[0] / sum[1]) : 0.);
 }
 
 __device__ int crit_group(SectionWork &w, const MeshDev &m, const BoundaryDev &b, const int *slots, int k0, int n,
@@ -677,7 +708,6 @@ __device__ int crit_group(SectionWork &w, const MeshDev &m, const BoundaryDev &b
     const int nc = m.nc, nf = m.nf;
     const size_t ns = b.nslot;
     const double tol = 128. * EPS;
-    if (threadIdx.x == 0) { w.error = 0; w.done = 0; w.eta = 0.; w.area = w.width = w.rate = 0.; }
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int k = slots ? slots[i] : k0 + i, f = b.slot_face[k], c = m.owner[f];
         b.branch[k] = 0; b.invariant[k] = 0.;
@@ -689,87 +719,62 @@ __device__ int crit_group(SectionWork &w, const MeshDev &m, const BoundaryDev &b
         b.branch[k] = 1; b.invariant[k] = un + 2. * wave;
     }
     __syncthreads();
-    for (int active = 0; active <= n; ++active) {
-        for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
-            double lo = INFINITY, hi = -INFINITY, count = 0.;
-            for (int i = lane; i < n; i += SECTION_LANES) {
-                const int k = slots ? slots[i] : k0 + i;
-                if (b.branch[k] != 1) continue;
-                const int c = m.owner[b.slot_face[k]];
-                lo = fmin(lo, resolved_bed(m, b, k, q, z)); hi = fmax(hi, q[c] + z[c]); count += 1.;
-            }
-            w.part[0][lane] = lo; w.part[1][lane] = hi; w.part[2][lane] = count;
+    int error = 0;
+    bool done = false;
+    double eta = 0., area = 0., width = 0.;
+    const auto residual = [&](double at) { return crit_residual(w, m, b, slots, k0, n, at, g, dry, q, z, area, width); };
+    for (int active = 0; active <= n && !done && !error; ++active) {
+        double lo = INFINITY, hi = -INFINITY;
+        bool some = false;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const int k = slots ? slots[i] : k0 + i;
+            if (b.branch[k] != 1) continue;
+            const int c = m.owner[b.slot_face[k]];
+            lo = fmin(lo, resolved_bed(m, b, k, q, z)); hi = fmax(hi, q[c] + z[c]);
+            some = true;
         }
+        if (!__syncthreads_or(some)) { done = true; break; }
+        const int used = min(n, (int)blockDim.x);
+        if ((int)threadIdx.x < used) { w.part[0][threadIdx.x] = lo; w.part[1][threadIdx.x] = hi; }
         __syncthreads();
         if (threadIdx.x == 0) {
-            w.lo = INFINITY; w.hi = -INFINITY; w.count = 0;
-            for (int lane = 0; lane < SECTION_LANES; ++lane) {
-                w.lo = fmin(w.lo, w.part[0][lane]); w.hi = fmax(w.hi, w.part[1][lane]); w.count += int(w.part[2][lane]);
-            }
-            if (w.count) w.lo += fmax(2. * dry, tol * fmax(1., fabs(w.lo)));
-            else { w.done = 1; w.area = w.width = w.rate = 0.; }
+            for (int i = 0; i < used; ++i) { lo = fmin(lo, w.part[0][i]); hi = fmax(hi, w.part[1][i]); }
+            w.sum[0] = lo; w.sum[1] = hi;
         }
         __syncthreads();
-        if (w.done) break;
-        crit_residual(w, m, b, slots, k0, n, w.lo, g, dry, q, z);
-        if (w.residual < 0.) {                     // unresolved controlled depth: the opening closes
+        lo = w.sum[0]; hi = w.sum[1];
+        __syncthreads();
+        lo += fmax(2. * dry, tol * fmax(1., fabs(lo)));
+        const double rlo = residual(lo);
+        if (rlo < 0.) {                            // unresolved controlled depth: the opening closes
             for (int i = threadIdx.x; i < n; i += blockDim.x) {
                 const int k = slots ? slots[i] : k0 + i;
                 if (b.branch[k] == 1) b.branch[k] = 0;
             }
-            if (threadIdx.x == 0) { w.done = 1; w.area = w.width = w.rate = 0.; w.eta = w.lo; }
-            __syncthreads();
+            eta = lo;
+            done = true;
             break;
         }
-        crit_residual(w, m, b, slots, k0, n, w.hi, g, dry, q, z);
-        for (int j = 0; j < 60 && w.residual > 0.; ++j) {
-            if (threadIdx.x == 0) w.hi = w.lo + 2. * (w.hi - w.lo);
-            __syncthreads();
-            crit_residual(w, m, b, slots, k0, n, w.hi, g, dry, q, z);
+        double rhi = residual(hi);
+        for (int j = 0; j < 60 && rhi > 0.; ++j) { hi = lo + 2. * (hi - lo); rhi = residual(hi); }
+        if (rhi > 0. || !isfinite(rhi)) { error = 1; break; }
+        shrink_bracket(lo, hi, rlo, rhi, residual);
+        eta = lo + .5 * (hi - lo);
+        bool changed = false;
+        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+            const int k = slots ? slots[i] : k0 + i;
+            if (b.branch[k] != 1) continue;
+            const double h = fmax(eta - resolved_bed(m, b, k, q, z), 0.), un = b.invariant[k] - 2. * sqrt(g * h);
+            if (h <= dry || un < -tol) { b.branch[k] = 0; changed = true; }
         }
-        if (w.residual > 0. || !isfinite(w.residual)) {
-            if (threadIdx.x == 0) w.error = 1;
-            __syncthreads();
-            break;
-        }
-        for (int j = 0; j < 90; ++j) {
-            if (threadIdx.x == 0) { w.eta = w.lo + .5 * (w.hi - w.lo); w.stagnant = w.eta == w.lo || w.eta == w.hi; }
-            __syncthreads();
-            if (w.stagnant) break;
-            crit_residual(w, m, b, slots, k0, n, w.eta, g, dry, q, z);
-            if (threadIdx.x == 0) { if (w.residual > 0.) w.lo = w.eta; else w.hi = w.eta; }
-            __syncthreads();
-        }
-        if (threadIdx.x == 0) w.eta = w.lo + .5 * (w.hi - w.lo);
-        __syncthreads();
-        for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
-            double changed = 0.;
-            for (int i = lane; i < n; i += SECTION_LANES) {
-                const int k = slots ? slots[i] : k0 + i;
-                if (b.branch[k] != 1) continue;
-                const double h = fmax(w.eta - resolved_bed(m, b, k, q, z), 0.), un = b.invariant[k] - 2. * sqrt(g * h);
-                if (h <= dry || un < -tol) { b.branch[k] = 0; changed += 1.; }
-            }
-            w.part[0][lane] = changed;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) { w.changed = 0; for (int lane = 0; lane < SECTION_LANES; ++lane) w.changed += int(w.part[0][lane]); }
-        __syncthreads();
-        if (w.changed) continue;
-        crit_residual(w, m, b, slots, k0, n, w.eta, g, dry, q, z);
-        if (threadIdx.x == 0) {
-            const double qc = w.width > 0. ? sqrt(g * w.area * w.area * w.area / w.width) : 0.;
-            if (w.area <= 0. || w.width <= 0. || !isfinite(w.residual) || fabs(w.residual) > 1e-10 * fmax(qc, 1.)) w.error = 2;
-            w.done = 1;
-        }
-        __syncthreads();
-        break;
+        if (__syncthreads_or(changed)) continue;
+        const double r = residual(eta), qc = width > 0. ? sqrt(g * area * area * area / width) : 0.;
+        if (area <= 0. || width <= 0. || !isfinite(r) || fabs(r) > 1e-10 * fmax(qc, 1.)) error = 2;
+        done = true;
     }
-    if (threadIdx.x == 0 && !w.done && !w.error) w.error = 3;
+    if (!done && !error) error = 3;
     __syncthreads();
-    const int error = w.error;
-    __syncthreads();
-    if (error) return error;
+    if (error) return error;                 // the same in every thread
     for (int i = threadIdx.x; i < n; i += blockDim.x) {
         const int k = slots ? slots[i] : k0 + i, f = b.slot_face[k], c = m.owner[f];
         const double rbed = resolved_bed(m, b, k, q, z), h0 = q[c], geom = fmax(h0 + z[c] - rbed, 0.);
@@ -779,7 +784,7 @@ __device__ int crit_group(SectionWork &w, const MeshDev &m, const BoundaryDev &b
         double un = ux * nx + uy * ny;
         const double tx = ux - un * nx, ty = uy - un * ny;
         if (b.branch[k] == 0) un = 0.;
-        else if (b.branch[k] == 1) { h = fmax(w.eta - rbed, 0.); un = b.invariant[k] - 2. * sqrt(g * h); }
+        else if (b.branch[k] == 1) { h = fmax(eta - rbed, 0.); un = b.invariant[k] - 2. * sqrt(g * h); }
         if (!isfinite(h) || !isfinite(un) || sqrt(un * un + tx * tx + ty * ty) > speed) { bad = true; continue; }
         double water = 0., fx = 0., fy = 0., t0 = 0., t1 = 0., t2 = 0.;
         if (h > dry) {
@@ -798,7 +803,7 @@ __device__ int crit_group(SectionWork &w, const MeshDev &m, const BoundaryDev &b
 // The critical owner of segment sg: the whole opening, then, when dry faces
 // split its chains into several wet groups, each group alone with the dry
 // faces closed at their owners' pressure (river_exterior_outlet.py:37-72).
-__device__ int crit_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
+__device__ __noinline__ int crit_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
                             double speed, const double *q, const double *z, bool &bad)
 {
     const int nf = m.nf, k0 = b.seg_off[sg], n = b.seg_off[sg + 1] - k0;
@@ -864,21 +869,23 @@ struct InletRiemann {
     int iterations, error;
 };
 
-__device__ __forceinline__ void inlet_wave(double h, double hk, double g, double &f, double &df)
+// Jump across the wave between h and the state of depth hk, and its
+// derivative; ck = sqrt(g hk), rk = 1 / hk, rh = 1 / h.
+__device__ __forceinline__ void inlet_wave(double h, double rh, double hk, double ck, double rk, double g, double &f,
+                                           double &df)
 {
-    if (h > hk) {
-        const double a = sqrt(.5 * g * (1. / h + 1. / hk));
+    if (greater(h, hk)) {
+        const double a = sqrt(.5 * g * (rh + rk)), den = a * h * h;
         f = (h - hk) * a;
-        df = a - .25 * g * (h - hk) / (a * h * h);
+        df = a - quotient(.25 * g * (h - hk), den, reciprocal(den));
     } else {
-        const double c = sqrt(g * h);
-        f = 2. * (c - sqrt(g * hk));
-        df = sqrt(g / h);
+        f = 2. * (sqrt(g * h) - ck);
+        df = sqrt(quotient(g, h, rh));
     }
 }
 
 // river_exterior_inlet.h:32-69: left = reservoir, right = interior (normal into the domain)
-__device__ InletRiemann inlet_exact(double hl, double ul, double hr, double ur, double g)
+__device__ __noinline__ InletRiemann inlet_exact(double hl, double ul, double hr, double ur, double g)
 {
     InletRiemann r = {0., 0., 0., 0, 0};
     const double cl = sqrt(g * hl), cr = sqrt(g * hr);
@@ -892,30 +899,30 @@ __device__ InletRiemann inlet_exact(double hl, double ul, double hr, double ur, 
     }
     double guess = .5 * (cl + cr) - .25 * (ur - ul);
     guess = guess * guess / g;
+    const double rl = quotient(1., hl, reciprocal(hl)), rr = quotient(1., hr, reciprocal(hr));
     double lo = 0., hi = fmax(fmax(hl, hr), guess), fl, fr, dl, dr;
-    inlet_wave(hi, hl, g, fl, dl);
-    inlet_wave(hi, hr, g, fr, dr);
-    for (int j = 0; j < 60 && fl + fr + ur - ul < 0.; ++j) {
-        hi *= 2.;
-        inlet_wave(hi, hl, g, fl, dl);
-        inlet_wave(hi, hr, g, fr, dr);
-    }
+    const auto waves = [&](double h) {
+        const double rh = quotient(1., h, reciprocal(h));
+        inlet_wave(h, rh, hl, cl, rl, g, fl, dl);
+        inlet_wave(h, rh, hr, cr, rr, g, fr, dr);
+    };
+    waves(hi);
+    for (int j = 0; j < 60 && fl + fr + ur - ul < 0.; ++j) { hi *= 2.; waves(hi); }
     if (!isfinite(hi) || fl + fr + ur - ul < 0.) { r.error = 1; return r; }
     const double scale = fmax(1., cl + cr + fabs(ul) + fabs(ur));
     double h = fmax(fmin(guess, hi), 1e-30), residual = 0.;
     for (int j = 0; j < 70; ++j) {
-        inlet_wave(h, hl, g, fl, dl);
-        inlet_wave(h, hr, g, fr, dr);
+        waves(h);
         residual = fl + fr + ur - ul;
         r.iterations = j + 1;
         if (fabs(residual) <= 4e-14 * scale) break;
         if (residual < 0.) lo = h; else hi = h;
-        double next = h - residual / (dl + dr);
+        const double slope = dl + dr;
+        double next = h - quotient(residual, slope, reciprocal(slope));
         if (!(next > lo && next < hi)) next = lo + .5 * (hi - lo);
         h = next;
     }
-    inlet_wave(h, hl, g, fl, dl);
-    inlet_wave(h, hr, g, fr, dr);
+    if (fabs(residual) > 4e-14 * scale) waves(h);
     residual = fl + fr + ur - ul;
     if (!isfinite(h) || fabs(residual) > 2e-11 * scale) { r.error = 2; return r; }
     const double u = .5 * (ul + ur + fr - fl), c = sqrt(g * h);
@@ -946,48 +953,46 @@ __device__ __forceinline__ void inlet_interior(const MeshDev &m, const BoundaryD
 }
 
 // river_exterior_inlet.h:71-95: section discharge, its derivative and the
-// gross throughflow at the common velocity w.velocity (lane sums, lane order).
-__device__ void inlet_rate(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int k0, int k1, double requested,
-                           double g, double dry, const double *q, const double *z)
+// gross throughflow at the common velocity (lane sums, lane order), the same
+// in every thread; returns whether a face's Riemann solution failed.
+__device__ __noinline__ bool inlet_rate(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int k0, int k1, double requested,
+                           double velocity, double g, double dry, const double *q, const double *z, double &rate,
+                           double &derivative, double &gross)
 {
-    for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
-        double rate = 0., derivative = 0., gross = 0.;
-        int error = 0;
+    const int n = min(k1 - k0, SECTION_LANES);
+    bool failed = false;
+    for (int lane = threadIdx.x; lane < n; lane += blockDim.x) {
+        double sum = 0., slope = 0., through = 0.;
         for (int k = k0 + lane; k < k1; k += SECTION_LANES) {
             double hi, ui;
             inlet_interior(m, b, k, dry, q, z, hi, ui);
             double hr = fmax(requested - b.ext_bed[k], 0.);
             if (hr <= dry) hr = 0.;
-            const InletRiemann r = inlet_exact(hr, w.velocity, hi, ui, g);
+            const InletRiemann r = inlet_exact(hr, velocity, hi, ui, g);
             const double len = m.length[b.slot_face[k]];
-            rate += r.h * r.u * len; derivative += r.derivative * len;
-            gross += fabs(r.h * r.u * len);
-            error = max(error, r.error);
+            sum += r.h * r.u * len; slope += r.derivative * len;
+            through += fabs(r.h * r.u * len);
+            failed = failed || r.error;
         }
-        w.part[0][lane] = rate; w.part[1][lane] = derivative; w.part[4][lane] = error; w.part[5][lane] = gross;
+        w.part[0][lane] = sum; w.part[1][lane] = slope; w.part[2][lane] = through;
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        w.rate = w.derivative = w.gross = 0.;
-        for (int lane = 0; lane < SECTION_LANES; ++lane) {
-            w.rate += w.part[0][lane]; w.derivative += w.part[1][lane]; w.gross += w.part[5][lane];
-            if (w.part[4][lane] != 0.) w.error = 5;
-        }
-    }
-    __syncthreads();
+    double sums[3];
+    lane_sums<3>(w, n, sums);
+    rate = sums[0]; derivative = sums[1]; gross = sums[2];
+    return __syncthreads_or(failed);
 }
 
 // river_exterior_inlet.h:97-186: the inlet of segment sg. Returns 0 or the
 // section failure (a trial rejection in the reference); `bad` gets the faces
 // whose Riemann solution failed or exceeds the speed limit (face status 3).
-__device__ int inlet_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
+__device__ __noinline__ int inlet_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
                              double speed, const double *q, const double *z, bool &bad)
 {
     const int nc = m.nc, nf = m.nf, nseg = b.nseg, k0 = b.seg_off[sg], k1 = b.seg_off[sg + 1];
     const size_t ns = b.nslot;
     const double Q = b.forcing[sg], requested = b.forcing[nseg + sg];
-    if (threadIdx.x == 0) w.error = 0;
-    for (int lane = threadIdx.x; lane < SECTION_LANES; lane += blockDim.x) {
+    const int n = min(k1 - k0, SECTION_LANES);
+    for (int lane = threadIdx.x; lane < n; lane += blockDim.x) {
         double area = 0., scale = 1.;
         for (int k = k0 + lane; k < k1; k += SECTION_LANES) {
             double hi, ui;
@@ -998,62 +1003,44 @@ __device__ int inlet_section(SectionWork &w, const MeshDev &m, const BoundaryDev
         }
         w.part[0][lane] = area; w.part[1][lane] = scale;
     }
+    double sums[1];
+    lane_sums<1>(w, n, sums);
+    double scale = 1.;
+    for (int lane = 0; lane < n; ++lane) scale = fmax(scale, w.part[1][lane]);
     __syncthreads();
-    if (threadIdx.x == 0) {
-        w.area = 0.; w.scale = 1.;
-        for (int lane = 0; lane < SECTION_LANES; ++lane) { w.area += w.part[0][lane]; w.scale = fmax(w.scale, w.part[1][lane]); }
-        if (!isfinite(Q) || Q < 0. || !isfinite(requested) || (Q > 0. && w.area <= 0.)) w.error = 1;
-        w.velocity = w.area > 0. ? Q / w.area : 0.;
-        w.scale = fmax(w.scale, 1. + fabs(w.velocity));
-    }
-    __syncthreads();
-    if (Q > 0. && !w.error) {
-        if (threadIdx.x == 0) { w.lo = w.velocity - w.scale; w.hi = w.velocity + w.scale; w.velocity = w.lo; }
-        __syncthreads();
-        inlet_rate(w, m, b, k0, k1, requested, g, dry, q, z);
-        for (int j = 0; j < 60 && w.rate > Q && !w.error; ++j) {
-            if (threadIdx.x == 0) { w.lo -= w.scale; w.scale *= 2.; w.velocity = w.lo; }
-            __syncthreads();
-            inlet_rate(w, m, b, k0, k1, requested, g, dry, q, z);
-        }
-        const bool low_bad = w.rate > Q;
-        __syncthreads();
-        if (threadIdx.x == 0) { if (low_bad) w.error = 2; w.velocity = w.hi; }
-        __syncthreads();
-        inlet_rate(w, m, b, k0, k1, requested, g, dry, q, z);
-        for (int j = 0; j < 60 && w.rate < Q && !w.error; ++j) {
-            if (threadIdx.x == 0) { w.hi += w.scale; w.scale *= 2.; w.velocity = w.hi; }
-            __syncthreads();
-            inlet_rate(w, m, b, k0, k1, requested, g, dry, q, z);
-        }
-        const bool high_bad = w.rate < Q;
-        __syncthreads();
-        if (threadIdx.x == 0) { if (high_bad) w.error = 2; w.velocity = fmin(w.hi, fmax(w.lo, Q / w.area)); }
-        __syncthreads();
-        for (int j = 0; j < 80 && !w.error; ++j) {
-            inlet_rate(w, m, b, k0, k1, requested, g, dry, q, z);
+    const double area = sums[0];
+    int error = 0;
+    if (!isfinite(Q) || Q < 0. || !isfinite(requested) || (Q > 0. && area <= 0.)) error = 1;
+    double velocity = area > 0. ? Q / area : 0.;
+    scale = fmax(scale, 1. + fabs(velocity));
+    if (Q > 0. && !error) {
+        double lo = velocity - scale, hi = velocity + scale, rate, derivative, gross;
+        const auto eval = [&](double at) {
+            velocity = at;
+            if (inlet_rate(w, m, b, k0, k1, requested, at, g, dry, q, z, rate, derivative, gross)) error = 5;
+        };
+        eval(lo);
+        for (int j = 0; j < 60 && rate > Q && !error; ++j) { lo -= scale; scale *= 2.; eval(lo); }
+        if (rate > Q) error = 2;
+        eval(hi);
+        for (int j = 0; j < 60 && rate < Q && !error; ++j) { hi += scale; scale *= 2.; eval(hi); }
+        if (rate < Q) error = 2;
+        double at = fmin(hi, fmax(lo, Q / area));
+        for (int j = 0; j < 80 && !error; ++j) {
+            eval(at);
             // net Q may be far below the signed face throughflow: relative
             // tolerance plus a double-precision budget on the gross flow
-            if (fabs(w.rate - Q) <= 3e-13 * Q + 256. * EPS * w.gross) break;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                if (w.rate < Q) w.lo = w.velocity; else w.hi = w.velocity;
-                double next = w.derivative > 0. ? w.velocity + (Q - w.rate) / w.derivative : w.lo + .5 * (w.hi - w.lo);
-                if (!(next > w.lo && next < w.hi)) next = w.lo + .5 * (w.hi - w.lo);
-                w.velocity = next;
-            }
-            __syncthreads();
+            if (fabs(rate - Q) <= 3e-13 * Q + 256. * EPS * gross) break;
+            if (rate < Q) lo = at; else hi = at;
+            double next = derivative > 0. ? at + (Q - rate) / derivative : lo + .5 * (hi - lo);
+            if (!(next > lo && next < hi)) next = lo + .5 * (hi - lo);
+            at = next;
         }
-        inlet_rate(w, m, b, k0, k1, requested, g, dry, q, z);
-        const bool final_bad = !isfinite(w.rate) || fabs(w.rate - Q) > 1e-10 * Q + 1024. * EPS * w.gross;
-        __syncthreads();
-        if (threadIdx.x == 0 && final_bad) w.error = 3;
-        __syncthreads();
+        if (velocity != at) eval(at);                // the loop ran out: its last point
+        velocity = at;
+        if (!isfinite(rate) || fabs(rate - Q) > 1e-10 * Q + 1024. * EPS * gross) error = 3;
     }
-    const int error = w.error;
-    const double velocity = w.velocity;
-    __syncthreads();
-    if (error) return error;
+    if (error) return error;                         // the same in every thread
     for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const int f = b.slot_face[k], c = m.owner[f];
         const double nx = m.normal[f], ny = m.normal[nf + f], h0 = q[c];
@@ -1203,7 +1190,7 @@ __device__ void line_normal_candidate(const MeshDev &m, const BoundaryDev &b, in
 
 // The line of segment sg (block-cooperative); false when the section has no
 // resolved root (the reference rejects the trial).
-__device__ bool line_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
+__device__ __noinline__ bool line_section(SectionWork &w, const MeshDev &m, const BoundaryDev &b, int sg, double g, double dry,
                              int law, double rough)
 {
     const int k0 = b.seg_off[sg], k1 = b.seg_off[sg + 1], kind = b.line_kind[sg];
@@ -1292,62 +1279,121 @@ __device__ void inlet_allocation(const MeshDev &m, const BoundaryDev &b, const C
     }
 }
 
-// The scenario's sum over its open faces of (outward water flux x length),
-// with each face's water as the update consumes it (the mixed form carries
-// it in FP32: F(flux)); per-thread strided sums, a butterfly within each
-// warp, then thread 0 adds the warp sums in warp order (a fixed order: the
-// same value on every run). The controller turns the stage sums into the
-// boundary ledger.
-constexpr int BOUNDARY_WARPS = 32;
-template <class F>
-__device__ void boundary_water(const MeshDev &m, const BoundaryDev &b, Ctrl &ct, int stage, int k0, int k1)
-{
-    __shared__ double part[BOUNDARY_WARPS], apart[BOUNDARY_WARPS];
-    __syncthreads();
-    double acc = 0., aacc = 0.;
-    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-        const double v = double(F(b.flux[k])) * m.length[b.slot_face[k]];
-        acc += v;
-        aacc += fabs(v);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        acc += __shfl_xor_sync(0xffffffffu, acc, o);
-        aacc += __shfl_xor_sync(0xffffffffu, aacc, o);
-    }
-    if ((threadIdx.x & 31) == 0) { part[threadIdx.x >> 5] = acc; apart[threadIdx.x >> 5] = aacc; }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double total = 0., gross = 0.;
-        for (int i = 0; i < (int)(blockDim.x >> 5); ++i) { total += part[i]; gross += apart[i]; }
-        ct.bflux[stage - 1] = total;
-        ct.bgross[stage - 1] = gross;
-    }
-}
-
 // stage 1 / 2: the SSPRK stages (state work / q1, its own stock, clock t or
 // t + dt); STAGE_HANCOCK: the HLLC predicted state q1 at t + dt/2, outlet
 // stock of the substep's start state work (hllc.py:91-97), status of stage 1.
 constexpr int STAGE_HANCOCK = 3;
 
-template <class F>
-__global__ void k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int stage_in)
+// Exterior trace and flux of slot k on a segment of mode 2, 3 or 6
+// (river_exterior_bed.h:94-174); returns the face status. total: the
+// segment's conveyance, w: the face's.
+__device__ __forceinline__ int plain_face(const MeshDev &m, const BoundaryDev &b, int k, int sg, const double *q,
+                                          const double *z, double dry, double grav, double speed_limit, double total,
+                                          double w, double tr[3], double fl[3])
 {
-    __shared__ double tile_buf[BOUNDARY_TILES];
-    const int sid = blockIdx.x;
+    const int nc = m.nc, f = b.slot_face[k], c = m.owner[f], mode = b.seg_mode[sg];
+    const double h0 = q[c], nx = m.normal[f], ny = m.normal[m.nf + f], bed = b.ext_bed[k];
+    const double Q = b.forcing[sg], stagev = b.forcing[b.nseg + sg];
+    double h = h0 + z[c] - bed, ux = 0., uy = 0.;
+    if (!greater(h, 0.)) h = 0.;
+    const double geometric = h;
+    const bool wet0 = greater(h0, dry);
+    if (wet0) {
+        const double r = reciprocal(h0);
+        ux = quotient(q[nc + c], h0, r); uy = quotient(q[2 * nc + c], h0, r);
+    }
+    const double un = ux * nx + uy * ny;
+    double tx = ux - un * nx, ty = uy - un * ny, speed = 0.;
+    if (mode == 6) {
+        if (Q > 0. && total <= 0.) return 1;
+        if (greater(h, dry) && Q > 0.) {
+            const double den = total * h * m.length[f];
+            speed = quotient(-Q * w, den, reciprocal(den));
+        }
+    } else if (mode == 3) {
+        if (!wet0) h = 0.;
+        else if (greater(h, dry)) {
+            if (un < sqrt(grav * h)) return 6;
+            speed = un;
+        }
+    } else if (mode == 2) {
+        const double target = greater(stagev - bed, 0.) ? stagev - bed : 0.;
+        const int policy = b.stage_policy[sg];
+        if (policy && (!wet0 || !greater(h, dry)) && greater(target, dry)) return 4;
+        if (!wet0) h = 0.;
+        if (greater(h, dry)) {
+            const double wave = sqrt(grav * h);
+            if (un <= -wave) {
+                if (policy) return 5;
+                tx = ty = 0.;
+            } else {
+                double hb, ub;
+                stage_wave(h, un, target, grav, wave, hb, ub);
+                if (ub < 0. && policy) {
+                    if (ub <= -sqrt(grav * hb)) return 5;
+                    h = hb; speed = ub; tx = ty = 0.;
+                } else if (ub < 0.) tx = ty = 0.;
+                else { h = hb; speed = ub; }
+            }
+        }
+    } else return 2;
+    if (!finite_bits(h) || !finite_bits(speed) || greater(0., h)) return 3;
+    // sqrt(s2) > limit, with the square root only where the squares are near
+    const double s2 = speed * speed + tx * tx + ty * ty;
+    if (!greater(speed_limit * speed_limit * .999999, s2) && sqrt(s2) > speed_limit) return 3;
+    double water = 0., fx = 0., fy = 0.;
+    if (greater(h, dry)) {
+        const double r = reciprocal(h);
+        tr[0] = h;
+        tr[1] = h * (speed * nx + tx);
+        tr[2] = h * (speed * ny + ty);
+        water = tr[1] * nx + tr[2] * ny;
+        fx = quotient(water * tr[1], h, r) + .5 * grav * h * h * nx;
+        fy = quotient(water * tr[2], h, r) + .5 * grav * h * h * ny;
+    }
+    const double pressure = wet0 ? .5 * grav * (h0 * h0 - geometric * geometric) : 0.;
+    fl[0] = water; fl[1] = fx + pressure * nx; fl[2] = fy + pressure * ny;
+    return 0;
+}
+
+// The open boundary of one scenario. What bounds it: a chain of short FP64
+// phases on one SM, where a warp's FP64 instruction takes 65 clocks and the
+// four sub-partitions are all there is. CLUSTER: a thread-block cluster shares
+// the scenario, a tile of 64 faces per pair of warps, with three cluster
+// barriers; used when no segment needs a section solve (those work in one
+// block) and the scenario is wider than one block's 128 faces. The sums keep
+// the reference's fixed tree (64-face tiles, then the tiles in order) and the
+// ledger its own, so no result depends on the cluster's size.
+template <class F, bool CLUSTER>
+__global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int stage_in)
+{
+    __shared__ double tile_buf[2][BOUNDARY_TILES], warp_buf[BOUNDARY_THREADS / 32][2][64];
+    int rank = 0, size = 1;
+    if constexpr (CLUSTER) {
+        rank = (int)cooperative_groups::this_cluster().block_rank();
+        size = (int)cooperative_groups::this_cluster().num_blocks();
+    }
+    auto team_sync = [&] {
+        if constexpr (CLUSTER) cooperative_groups::this_cluster().sync();
+        else __syncthreads();
+    };
+    const int sid = blockIdx.x / size, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Ctrl &ct = ctrl[sid];
     const bool hancock = stage_in == STAGE_HANCOCK;
     const int stage = hancock ? 1 : stage_in;
-    if (skip_stage(ct, stage)) return;
+    if (skip_stage(ct, stage)) return;            // the same for every block of the cluster
     const int s0 = b.scen_seg[sid], s1 = b.scen_seg[sid + 1];
     if (s0 == s1) return;
-    const int nc = m.nc;
+    const int nseg = b.nseg;
+    const size_t ns = b.nslot;
     const double *q = stage == 1 && !hancock ? s.work : s.q1;
     const double *base = hancock ? s.work : q;    // stock of the stage start (the substep start for Hancock)
     const double *z = s.z;
     const double dry = ct.dry, grav = ct.grav;
     const double t = ct.time0 + ct.elapsed + (stage == 2 ? ct.trial : hancock ? .5 * ct.trial : 0.0);
-    // forcing at the stage clock (piecewise linear tables, else constant)
-    if (b.table_len > 0)
+    // forcing at the stage clock (piecewise linear tables, else constant); each
+    // block of a cluster writes the same values
+    if (b.table_len > 0) {
         for (int sg = s0 + threadIdx.x; sg < s1; sg += blockDim.x)
             for (int row = 0; row < 2; ++row) {
                 const int L = b.table_len;
@@ -1365,11 +1411,13 @@ __global__ void k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int
                 }
                 b.forcing[(size_t)row * b.nseg + sg] = val;
             }
+        __syncthreads();
+    }
     // critical, then normal reference lines of the exact-discharge inlets
     // (river_exterior_bed.py:199-200); a section without a root rejects the trial
     __shared__ SectionWork section;
     bool line_failed = false;
-    if (b.line_kind) {
+    if (!CLUSTER && b.sections && b.line_kind) {
         for (int pass = 1; pass <= 2; ++pass)
             for (int sg = s0; sg < s1; ++sg)          // block-uniform
                 if (b.seg_mode[sg] == 9 && b.line_kind[sg] == pass &&
@@ -1377,189 +1425,220 @@ __global__ void k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int
                     line_failed = true;
         __syncthreads();
     }
-    const int k0 = b.seg_off[s0], k1 = b.seg_off[s1];
-    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-        const int f = b.slot_face[k], c = m.owner[f];
-        const double w = q[c] > dry ? m.length[f] : 0.;
-        b.terms[k] = (z[c] + q[c]) * w;
-        b.terms[(size_t)b.nslot + k] = w;
+    const int ntile = [&] { int n = 0; for (int sg = s0; sg < s1; ++sg) n += tile_count(b, sg); return n; }();
+    // wetted stage sum and wetted width of the conveyance inlets' segments
+    // (every block forms all of them: three instructions a face)
+    for (int i = warp; i < ntile; i += BOUNDARY_THREADS / 32) {
+        const SlotTile tile = slot_tile(b, s0, i);
+        if (b.seg_mode[tile.sg] != 6) continue;
+        double lo[2] = {0., 0.}, hi[2] = {0., 0.};
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int k = tile.first + lane + 32 * half;
+            if (k >= tile.end) continue;
+            const int f = b.slot_face[k], c = m.owner[f];
+            const double hc = q[c], w = greater(hc, dry) ? m.length[f] : 0.;
+            (half ? hi : lo)[0] = (z[c] + hc) * w;
+            (half ? hi : lo)[1] = w;
+        }
+        const double sum = tile_sum<2>(warp_buf[warp], tile.end - tile.first, lo, hi);
+        if (lane < 2) tile_buf[lane][i] = sum;
     }
     __syncthreads();
-    segment_sums(b, s0, s1, 0, 0, tile_buf);
-    segment_sums(b, s0, s1, 1, 1, tile_buf);
+    for (int sg = s0 + threadIdx.x; sg < s1; sg += blockDim.x) {
+        if (b.seg_mode[sg] != 6) continue;
+        int first = 0;
+        for (int u = s0; u < sg; ++u) first += tile_count(b, u);
+        double stage_sum = 0., width = 0.;
+        for (int i = 0; i < tile_count(b, sg); ++i) { stage_sum += tile_buf[0][first + i]; width += tile_buf[1][first + i]; }
+        b.seg_sums[sg] = stage_sum; b.seg_sums[nseg + sg] = width;
+    }
+    __syncthreads();
+    // conveyance weights, a tile per block of the cluster in turn
     const int rmode = ct.roughness_mode < 3 ? ct.roughness_mode : 3;
     const int waqua = ct.roughness_mode == 4;
-    const int nseg = b.nseg;
-    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-        const int f = b.slot_face[k], c = m.owner[f], sg = m.bid[f];
-        double w = 0.;
-        const double bed = b.ext_bed[k];
-        const int mode = b.seg_mode[sg];
-        if (mode == 6 && b.seg_sums[nseg + sg] > 0.) {
-            const double h = fmax(q[c] + z[c] - bed, 0.);
-            const double section = fmax(b.seg_sums[sg] / b.seg_sums[nseg + sg] - bed, 0.);
-            if (h > dry && section > 0.)
-                w = double(pow(F(section), F(1.5)) *
-                           exterior_chezy<F>(rmode, F(h), F(ct.roughness_value), F(dry), F(grav), waqua)) * m.length[f];
+    for (int i = rank + size * warp; i < ntile; i += size * (BOUNDARY_THREADS / 32)) {
+        const SlotTile tile = slot_tile(b, s0, i);
+        if (b.seg_mode[tile.sg] != 6) continue;
+        const double width = b.seg_sums[nseg + tile.sg];
+        const double level = width > 0. ? b.seg_sums[tile.sg] / width : 0.;
+        double lo[1] = {0.}, hi[1] = {0.};
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+            const int k = tile.first + lane + 32 * half;
+            if (k >= tile.end) continue;
+            const int f = b.slot_face[k], c = m.owner[f];
+            const double bed = b.ext_bed[k], h = q[c] + z[c] - bed, depth = level - bed;
+            double w = 0.;
+            if (width > 0. && greater(h, dry) && greater(depth, 0.))
+                w = conveyance<F>(rmode, waqua, F(depth), F(h), ct) * m.length[f];
+            b.terms[2 * ns + k] = w;
+            (half ? hi : lo)[0] = w;
         }
-        b.terms[2 * (size_t)b.nslot + k] = w;
+        const double sum = tile_sum<1>(warp_buf[warp], tile.end - tile.first, lo, hi);
+        if (lane == 0) b.terms[tile.first] = sum;
+    }
+    team_sync();
+    for (int sg = s0 + threadIdx.x; sg < s1; sg += blockDim.x) {
+        if (b.seg_mode[sg] != 6) continue;
+        double total = 0.;
+        for (int k = b.seg_off[sg]; k < b.seg_off[sg + 1]; k += 64) total += b.terms[k];
+        b.seg_sums[2 * (size_t)nseg + sg] = total;
     }
     __syncthreads();
-    segment_sums(b, s0, s1, 2, 2, tile_buf);
     unsigned bad = 0;
-    for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
-        const int f = b.slot_face[k], c = m.owner[f], sg = m.bid[f], mode = b.seg_mode[sg];
-        double tr0 = 0., tr1 = 0., tr2 = 0., fl0 = 0., fl1 = 0., fl2 = 0.;
-        const double h0 = q[c], nx = m.normal[f], ny = m.normal[m.nf + f], bed = b.ext_bed[k];
-        const double total = b.seg_sums[2 * (size_t)nseg + sg];
-        const double Q = b.forcing[sg], stagev = b.forcing[nseg + sg];
-        int st = 0;
-        if (!(mode == 4 || mode == 5 || mode == 9 || mode == 10 || mode == 11)) {
-            double h = fmax(h0 + z[c] - bed, 0.), geometric = h, ux = 0., uy = 0.;
-            if (h0 > dry) { ux = q[nc + c] / h0; uy = q[2 * nc + c] / h0; }
-            double un = ux * nx + uy * ny, tx = ux - un * nx, ty = uy - un * ny, normal_speed = 0.;
-            if (mode == 6) {
-                if (Q > 0. && total <= 0.) st = 1;
-                else if (h > dry && Q > 0.) normal_speed = -Q * b.terms[2 * (size_t)b.nslot + k] / (total * h * m.length[f]);
-            } else if (mode == 3) {
-                if (h0 <= dry) h = 0.;
-                else if (h > dry) {
-                    if (un < sqrt(grav * h)) st = 6;
-                    else normal_speed = un;
+    for (int i = rank + size * (threadIdx.x >> 6); i < ntile; i += size * (BOUNDARY_THREADS / 64)) {
+        const SlotTile tile = slot_tile(b, s0, i);
+        const int k = tile.first + (threadIdx.x & 63), mode = b.seg_mode[tile.sg];
+        if (k >= tile.end) continue;
+        double tr[3] = {0., 0., 0.}, fl[3] = {0., 0., 0.};
+        if (!(mode == 4 || mode == 5 || mode == 9 || mode == 10 || mode == 11) &&
+            plain_face(m, b, k, tile.sg, q, z, dry, grav, ct.speed_limit,
+                       mode == 6 ? b.seg_sums[2 * (size_t)nseg + tile.sg] : 0., mode == 6 ? b.terms[2 * ns + k] : 0., tr, fl))
+            bad = 1;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) { b.trace[r * ns + k] = tr[r]; b.flux[r * ns + k] = fl[r]; }
+    }
+    team_sync();
+    if constexpr (!CLUSTER) if (b.sections) {
+        // section owners of the remaining outlet modes, after the face loop, in
+        // the reference's order (river_exterior_bed.py:213-217): a normal-depth
+        // chain without a root rejects the trial before the rating owner runs; a
+        // rating section without a solution fails the scenario
+        __shared__ int section_reject;
+        if (threadIdx.x == 0) section_reject = line_failed;
+        __syncthreads();
+        if (b.inlet && !section_reject) {
+            bool inlet_failed = false;
+            for (int sg = s0; sg < s1; ++sg)              // block-uniform: the CTA solves one section at a time
+                if (b.seg_mode[sg] == 9) {
+                    bool sbad = false;
+                    if (inlet_section(section, m, b, sg, grav, dry, ct.speed_limit, q, z, sbad)) inlet_failed = true;
+                    if (sbad) bad = 1;
                 }
-            } else if (mode == 2) {
-                const double prescribed = fmax(stagev - bed, 0.);
-                const int policy = b.stage_policy[sg];
-                if (policy && (h0 <= dry || h <= dry) && prescribed > dry) st = 4;
-                else {
-                    if (h0 <= dry) h = 0.;
-                    if (h > dry) {
-                        const double wave = sqrt(grav * h);
-                        if (un <= -wave) {
-                            if (policy) st = 5;
-                            else { normal_speed = 0.; tx = ty = 0.; }
-                        } else {
-                            const double target = fmax(stagev - bed, 0.);
-                            double hb, ub;
-                            stage_wave(h, un, target, grav, hb, ub);
-                            if (ub < 0. && policy) {
-                                if (ub <= -sqrt(grav * hb)) st = 5;
-                                else { h = hb; normal_speed = ub; tx = ty = 0.; }
-                            } else if (ub < 0.) { normal_speed = 0.; tx = ty = 0.; }
-                            else { h = hb; normal_speed = ub; }
-                        }
-                    }
+            if (threadIdx.x == 0 && inlet_failed) section_reject = 1;
+            __syncthreads();
+        }
+        if (b.branch && !section_reject) {
+            bool crit_failed = false;
+            for (int sg = s0; sg < s1; ++sg)              // block-uniform: the CTA solves one section at a time
+                if (b.seg_mode[sg] == 4) {
+                    bool sbad = false;
+                    if (crit_section(section, m, b, sg, grav, dry, ct.speed_limit, q, z, sbad)) crit_failed = true;
+                    if (sbad) bad = 1;
                 }
-            } else st = 2;
-            if (!st && (!isfinite(h) || !isfinite(normal_speed) || h < 0. ||
-                        sqrt(normal_speed * normal_speed + tx * tx + ty * ty) > ct.speed_limit)) st = 3;
-            if (!st) {
-                double water = 0., fx = 0., fy = 0.;
-                if (h > dry) {
-                    tr0 = h;
-                    tr1 = h * (normal_speed * nx + tx);
-                    tr2 = h * (normal_speed * ny + ty);
-                    water = tr1 * nx + tr2 * ny;
-                    fx = water * tr1 / h + .5 * grav * h * h * nx;
-                    fy = water * tr2 / h + .5 * grav * h * h * ny;
+            if (threadIdx.x == 0 && crit_failed) section_reject = 1;
+            __syncthreads();
+        }
+        if (b.weir && !section_reject) {
+            for (int sg = s0; sg < s1; ++sg)              // block-uniform: the CTA solves one section at a time
+                if (b.seg_mode[sg] == 5) {
+                    bool sbad = false;
+                    const int e = weir_section(section, m, b, sg, grav, dry, ct.speed_limit, q, z, sbad);
+                    if (threadIdx.x == 0 && e) section_reject = 1;
+                    if (sbad) bad = 1;
                 }
-                double pressure = h0 > dry ? .5 * grav * (h0 * h0 - geometric * geometric) : 0.;
-                fl0 = water; fl1 = fx + pressure * nx; fl2 = fy + pressure * ny;
+            __syncthreads();
+        }
+        if (b.scen_chain && !section_reject) {
+            const int law = ct.roughness_mode;
+            for (int ch = b.scen_chain[sid] + threadIdx.x; ch < b.scen_chain[sid + 1]; ch += blockDim.x) {
+                bool sbad = false;
+                if (normal_chain(m, b, ch, grav, dry, ct.speed_limit, law, ct.roughness_value, q, z, sbad))
+                    atomicOr(&section_reject, 1);
+                if (sbad) bad = 1;
             }
         }
-        if (st) bad = 1;
-        b.trace[k] = tr0; b.trace[(size_t)b.nslot + k] = tr1; b.trace[2 * (size_t)b.nslot + k] = tr2;
-        b.flux[k] = fl0; b.flux[(size_t)b.nslot + k] = fl1; b.flux[2 * (size_t)b.nslot + k] = fl2;
-    }
-    __syncthreads();
-    // section owners of the remaining outlet modes, after the face loop, in
-    // the reference's order (river_exterior_bed.py:213-217): a normal-depth
-    // chain without a root rejects the trial before the rating owner runs; a
-    // rating section without a solution fails the scenario
-    __shared__ int section_reject;
-    if (threadIdx.x == 0) section_reject = line_failed;
-    __syncthreads();
-    if (b.inlet && !section_reject) {
-        bool inlet_failed = false;
-        for (int sg = s0; sg < s1; ++sg)              // block-uniform: the CTA solves one section at a time
-            if (b.seg_mode[sg] == 9) {
-                bool sbad = false;
-                if (inlet_section(section, m, b, sg, grav, dry, ct.speed_limit, q, z, sbad)) inlet_failed = true;
-                if (sbad) bad = 1;
-            }
-        if (threadIdx.x == 0 && inlet_failed) section_reject = 1;
+        __syncthreads();
+        if (!section_reject)
+            for (int sg = s0 + threadIdx.x; sg < s1; sg += blockDim.x)
+                if (b.seg_mode[sg] == 11) {
+                    bool sbad = false;
+                    if (rating_section(m, b, sg, grav, dry, ct.speed_limit, q, z, sbad)) raise_status(ct, stage, ST_FATAL);
+                    if (sbad) bad = 1;
+                }
+        if (section_reject) bad = 1;
         __syncthreads();
     }
-    if (b.branch && !section_reject) {
-        bool crit_failed = false;
-        for (int sg = s0; sg < s1; ++sg)              // block-uniform: the CTA solves one section at a time
-            if (b.seg_mode[sg] == 4) {
-                bool sbad = false;
-                if (crit_section(section, m, b, sg, grav, dry, ct.speed_limit, q, z, sbad)) crit_failed = true;
-                if (sbad) bad = 1;
-            }
-        if (threadIdx.x == 0 && crit_failed) section_reject = 1;
-        __syncthreads();
-    }
-    if (b.weir && !section_reject) {
-        for (int sg = s0; sg < s1; ++sg)              // block-uniform: the CTA solves one section at a time
-            if (b.seg_mode[sg] == 5) {
-                bool sbad = false;
-                const int e = weir_section(section, m, b, sg, grav, dry, ct.speed_limit, q, z, sbad);
-                if (threadIdx.x == 0 && e) section_reject = 1;
-                if (sbad) bad = 1;
-            }
-        __syncthreads();
-    }
-    if (b.scen_chain && !section_reject) {
-        const int law = ct.roughness_mode;
-        for (int ch = b.scen_chain[sid] + threadIdx.x; ch < b.scen_chain[sid + 1]; ch += blockDim.x) {
-            bool sbad = false;
-            if (normal_chain(m, b, ch, grav, dry, ct.speed_limit, law, ct.roughness_value, q, z, sbad))
-                atomicOr(&section_reject, 1);
-            if (sbad) bad = 1;
-        }
-    }
-    __syncthreads();
-    if (!section_reject)
-        for (int sg = s0 + threadIdx.x; sg < s1; sg += blockDim.x)
-            if (b.seg_mode[sg] == 11) {
-                bool sbad = false;
-                if (rating_section(m, b, sg, grav, dry, ct.speed_limit, q, z, sbad)) raise_status(ct, stage, ST_FATAL);
-                if (sbad) bad = 1;
-            }
-    if (section_reject) bad = 1;
     if (bad) raise_status(ct, stage, ST_SPATIAL);
-    __syncthreads();
     // outlet stock cap, one thread per unique owner, its faces in boundary order
     const int u0 = b.scen_own[sid], u1 = b.scen_own[sid + 1];
-    for (int u = u0 + threadIdx.x; u < u1; u += blockDim.x) {
+    const double rtrial = reciprocal(ct.trial);
+    for (int u = u0 + (int)threadIdx.x + BOUNDARY_THREADS * rank; u < u1; u += BOUNDARY_THREADS * size) {
         const int c = b.own_cell[u];
         double total = 0., reserved = 0.;
         for (int j = b.own_off[u]; j < b.own_off[u + 1]; ++j) {
             const int k = b.own_slot[j], f = b.slot_face[k];
-            const double debit = fmax(b.flux[k], 0.) * m.length[f];
+            const double flux = b.flux[k], debit = greater(flux, 0.) ? flux * m.length[f] : 0.;
             if (is_outlet(b.seg_mode[m.bid[f]])) total += debit; else reserved += debit;
         }
-        const double available = fmax(0., base[c] * m.area[c] / ct.trial - reserved);
-        const double ratio = fmin(1., available / fmax(total, 1e-300)) * (1. - 32. * EPS);
-        const double factor = total > available ? ratio : 1.;
+        const double left = quotient(base[c] * m.area[c], ct.trial, rtrial) - reserved;
+        const double available = greater(left, 0.) ? left : 0.;
+        if (!greater(total, available)) continue;             // nothing to cap
+        const double factor = fmin(1., available / fmax(total, 1e-300)) * (1. - 32. * EPS);
         for (int j = b.own_off[u]; j < b.own_off[u + 1]; ++j) {
             const int k = b.own_slot[j], f = b.slot_face[k];
             const double water = b.flux[k];
-            const double scale = (is_outlet(b.seg_mode[m.bid[f]]) && water > 0.) ? factor : 1.;
+            if (!is_outlet(b.seg_mode[m.bid[f]]) || !(water > 0.)) continue;
             const double depth = b.trace[k], denom = fmax(depth, 1e-300);
-            const double ux = depth > 0. ? b.trace[(size_t)b.nslot + k] / denom : 0.;
-            const double uy = depth > 0. ? b.trace[2 * (size_t)b.nslot + k] / denom : 0.;
-            b.flux[(size_t)b.nslot + k] += (scale * scale - 1.) * water * ux;
-            b.flux[2 * (size_t)b.nslot + k] += (scale * scale - 1.) * water * uy;
-            b.flux[k] = water * scale;
-            b.trace[(size_t)b.nslot + k] *= scale;
-            b.trace[2 * (size_t)b.nslot + k] *= scale;
+            const double ux = depth > 0. ? b.trace[ns + k] / denom : 0.;
+            const double uy = depth > 0. ? b.trace[2 * ns + k] / denom : 0.;
+            b.flux[ns + k] += (factor * factor - 1.) * water * ux;
+            b.flux[2 * ns + k] += (factor * factor - 1.) * water * uy;
+            b.flux[k] = water * factor;
+            b.trace[ns + k] *= factor;
+            b.trace[2 * ns + k] *= factor;
         }
     }
-    if (b.inlet) inlet_allocation(m, b, ct, base, s0, s1, u0, u1);
-    boundary_water<F>(m, b, ct, stage, k0, k1);
+    if (!CLUSTER && b.inlet) {
+        inlet_allocation(m, b, ct, base, s0, s1, u0, u1);
+        __syncthreads();
+    }
+    // The scenario's sum over its open faces of (outward water flux x length),
+    // with each face's water as the update consumes it (the mixed form carries
+    // it in FP32: F(flux)), and of its magnitude: 32 owners by a butterfly,
+    // then these partial sums in order. The controller turns the stage sums
+    // into the boundary ledger. An owner's faces are its own thread's above.
+    for (int first = u0 + 32 * (warp + rank * (BOUNDARY_THREADS / 32)); first < u1; first += BOUNDARY_THREADS * size) {
+        const int u = first + lane;
+        double acc = 0., gross = 0.;
+        if (u < u1)
+            for (int j = b.own_off[u]; j < b.own_off[u + 1]; ++j) {
+                const int k = b.own_slot[j];
+                const double v = double(F(b.flux[k])) * m.length[b.slot_face[k]];
+                acc += v;
+                gross += fabs(v);
+            }
+        for (int o = 16; o > 0; o >>= 1) {
+            acc += __shfl_xor_sync(0xffffffffu, acc, o);
+            gross += __shfl_xor_sync(0xffffffffu, gross, o);
+        }
+        if (lane == 0) b.own_sum[first] = make_double2(acc, gross);
+    }
+    team_sync();
+    if (rank == 0 && threadIdx.x < 2) {
+        double total = 0.;
+        for (int first = u0; first < u1; first += 32) total += threadIdx.x ? b.own_sum[first].y : b.own_sum[first].x;
+        if (threadIdx.x) ct.bgross[stage - 1] = total; else ct.bflux[stage - 1] = total;
+    }
+}
+
+// Launch over nscen scenarios, b.cluster blocks each.
+template <class F>
+inline void launch_boundary(const MeshDev &m, const StateDev &s, const BoundaryDev &b, Ctrl *ctrl, int nscen, int stage,
+                            cudaStream_t st)
+{
+    if (b.cluster <= 1) {
+        k_boundary<F, false><<<nscen, BOUNDARY_THREADS, 0, st>>>(m, s, b, ctrl, stage);
+        return;
+    }
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = b.cluster; attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(nscen * b.cluster); cfg.blockDim = dim3(BOUNDARY_THREADS); cfg.stream = st;
+    cfg.attrs = &attr; cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_boundary<F, true>, m, s, b, ctrl, stage);
 }
 
 // ---------------------------------------------------------------------------

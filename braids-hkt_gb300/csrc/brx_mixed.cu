@@ -1369,7 +1369,7 @@ int mixed_kernel(const Launch &L, int kind, int stage, double *out)
         return 1;
     case K_BOUNDARY:
         if (!L.nslot) return 0;
-        brx_mixb::k_boundary<float><<<L.nscen, 256, 0, st>>>(L.mesh, L.state, L.bnd, L.ctrl, stage);
+        brx_mixb::launch_boundary<float>(L.mesh, L.state, L.bnd, L.ctrl, L.nscen, stage, st);
         return 1;
     case K_CELLS:
         if (small)
