@@ -1633,10 +1633,8 @@ static void enqueue_stage(brx_solver *s, int stage, double *rate_out)
         // the mixed face sweep computes the rotor face terms in its tail: it
         // needs the rotor cell terms (wet gradients, actuator sink) first
         if (fork && mixed) cudaStreamWaitEvent(s->stream, s->join2, 0);
-        // the donor limiter runs inside the update (owner computes): no limit
-        // pass, and in the FP64 form no separate gather
-        for (int kind : {(int)K_FACES, (int)K_GATHER})
-            s->launches += launch_kernel(s, kind, stage, nullptr);
+        // gather and donor limiter are part of the update
+        s->launches += launch_kernel(s, K_FACES, stage, nullptr);
         if (fork && !mixed) cudaStreamWaitEvent(s->stream, s->join2, 0);
     }
     s->launches += launch_turbines(s, stage, s->stream, TURB_FACES);
@@ -2111,7 +2109,7 @@ extern "C" int brx_profile_substep(brx_solver *s, double dt, double time, int ca
         const bool mixed = s->precision == BRX_MIXED, tiled = mixed && s->tile_cells > 0;
         for (int stage = 1; stage <= 2; ++stage)
             for (int kind : {(int)K_BOUNDARY, mixed ? (int)K_TURB : -1, tiled ? (int)K_TILE : (int)K_CELLS,
-                             tiled ? -1 : (int)K_FACES, tiled ? -1 : (int)K_GATHER,
+                             tiled ? -1 : (int)K_FACES,
                              mixed ? -1 : (int)K_TURB, (int)K_VISC, (int)K_UPDATE})
                 if (kind >= 0)
                     if (const int nl = launch_kernel(s, kind, stage, nullptr)) { mark(kind); extra += nl - 1; }

@@ -882,19 +882,33 @@ __global__ void __launch_bounds__(128, BRX_FACES_MIN_BLOCKS) km_faces(MeshDev m,
 // have at most MAX_CELL_FACES faces.
 constexpr double DONOR_MARGIN = 64.0 * (double)FEPS;
 
-// Face values of a cell's entries for the gather: the grid sweep reads the
-// face sweep's arrays through the cell's face list.
-struct GlobalFaces {
-    const int *faces;
-    const float2 *ws;
-    const float4 *gf;
-    __device__ __forceinline__ float2 ws_at(int k) const { return ws[faces[k]]; }
-    __device__ __forceinline__ float4 gf_at(int k) const { return gf[faces[k]]; }
-};
+// Donor factor of one cell from its outward water rate out (FP32, of stage
+// depth hf), split into exterior and interior faces where it owns open ones:
+// an FP32 test that is conservative, the value in FP64.
+__device__ __forceinline__ float mx_theta(const StateDev &s, Ctrl &ct, int stage, int c, float hf, bool owns_open,
+                                          float out, float ext, float interior)
+{
+    float theta = 1.f;
+    if (out > 0.f && ct.trialf * out >= 0.999f * hf) {
+        const double hb = (stage == 1 ? s.work : s.q1)[c];
+        const double cap = ct.trial * double(out) * (1. + DONOR_MARGIN);
+        if (cap >= hb) theta = float(fmin(1., hb / cap) * (1. - 32. * EPS));
+    }
+    if (owns_open) {
+        const double hb = (stage == 1 ? s.work : s.q1)[c];
+        const double available = hb / ct.trial;
+        const double e = double(ext), e_hi = e * (1. + DONOR_MARGIN);
+        const double in_hi = double(interior) * (1. + DONOR_MARGIN);
+        if (e > available) raise_status(ct, stage, ST_BUDGET);
+        const double factor = fmin(1., (available - e_hi) / fmax(in_hi, 1e-300)) * (1. - 32. * EPS);
+        theta = (interior > 0.f && in_hi >= available - e_hi) ? float(fmax(factor, 0.)) : 1.f;
+    }
+    return theta;
+}
 
-// Gather of one cell (the body of the gather sweep): its momentum rates and
-// donor factor into rate32 / theta32 and its face-sum CFL frequency in fr;
-// hf = the record's (depth, flags). Returns whether fr is valid.
+// Gather of one cell of a tile: its momentum rates and donor factor into
+// rate32 / theta32 and its face-sum CFL frequency in fr; hf = the record's
+// (depth, flags). Returns whether fr is valid.
 template <class FaceAt>
 __device__ __forceinline__ bool mx_gather_cell(const MeshDev &m, const StateDev &s, Ctrl &ct, const MixedGeo &g,
                                                int stage, int c, float2 hf, const FaceAt &fa, float *rate32,
@@ -917,52 +931,10 @@ __device__ __forceinline__ bool mx_gather_cell(const MeshDev &m, const StateDev 
     }
     rate32[c] = active ? -sum1 : 0.f;
     rate32[nc + c] = active ? -sum2 : 0.f;
-    float theta = 1.f;
-    // donor factor: an FP32 test that is conservative, the value in FP64
-    if (out > 0.f && ct.trialf * out >= 0.999f * hf.x) {
-        const double hb = (stage == 1 ? s.work : s.q1)[c];
-        const double cap = ct.trial * double(out) * (1. + DONOR_MARGIN);
-        if (cap >= hb) theta = float(fmin(1., hb / cap) * (1. - 32. * EPS));
-    }
-    if (owns_open) {
-        const double hb = (stage == 1 ? s.work : s.q1)[c];
-        const double available = hb / ct.trial;
-        const double e = double(ext), e_hi = e * (1. + DONOR_MARGIN);
-        const double in_hi = double(interior) * (1. + DONOR_MARGIN);
-        if (e > available) raise_status(ct, stage, ST_BUDGET);
-        const double factor = fmin(1., (available - e_hi) / fmax(in_hi, 1e-300)) * (1. - 32. * EPS);
-        theta = (interior > 0.f && in_hi >= available - e_hi) ? float(fmax(factor, 0.)) : 1.f;
-    }
-    theta32[c] = theta;
+    theta32[c] = mx_theta(s, ct, stage, c, hf.x, owns_open, out, ext, interior);
     fr = freq;
     if (isnan(fr)) { raise_status(ct, stage, ST_FREQ); return false; }
     return true;
-}
-
-__global__ void __launch_bounds__(256) km_gather(MeshDev m, StateDev s, Ctrl *ctrl, Work w, MixedGeo g, int stage)
-{
-    const int nc = m.nc;
-    const MxRec *rec = reinterpret_cast<const MxRec *>(w.rec);
-    float *rate32 = reinterpret_cast<float *>(w.rate);      // (2, nc) momentum rates
-    float *theta32 = reinterpret_cast<float *>(w.theta);
-    const GlobalFaces fa{m.faces, reinterpret_cast<const float2 *>(w.ws), reinterpret_cast<const float4 *>(w.gf)};
-    const int stride = gridDim.x * blockDim.x;
-    const int na = m.act.count[1];
-    for (int first = blockIdx.x * blockDim.x; first < na; first += stride) {   // warp-uniform trip count
-        const int c = first + (int)threadIdx.x < na ? active_cell(m.act, first + threadIdx.x) : nc;
-        bool have = false;
-        float fr = 0.f;
-        int sid = 0;
-        if (c < nc) {
-            sid = m.cell_sid[c];
-            Ctrl &ct = ctrl[sid];
-            if (!mx_skip(ct, stage))
-                have = mx_gather_cell(m, s, ct, g, stage, c, *reinterpret_cast<const float2 *>(&rec[c]), fa, rate32,
-                                      theta32, fr);
-        }
-        unsigned long long *peak0 = stage == 1 ? &ctrl[0].peak1 : &ctrl[0].peak2;
-        warp_max_peak_f(peak0, sizeof(Ctrl), sid, have, fr);
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1126,15 +1098,108 @@ __device__ __forceinline__ void drag_f(const Ctrl &ct, float dtf, double &h, dou
     hv *= fd;
 }
 
-// Update (owner computes): each cell forms the donor-limited water flux of
-// its faces itself (river_midpoint.h:30-41) from the face sweep's FP32 water
-// and the donor's factor, exactly as the face pass km_limit does: both cells
-// of a face compute the same FP64 value double(w) * double(theta), so mass
-// still telescopes, and no limited-flux buffer goes through memory. After
+// Rotor, viscosity and stage terms of one cell with hydraulic rates mass
+// (FP64), f1, f2; the result into the stage's target. quiet: no endpoint
+// status (the cell is redone with its limited fluxes).
+__device__ __forceinline__ void mx_finish(const MeshDev &m, const StateDev &s, Ctrl &ct, const Work &w,
+                                          const MixedGeo &g, int stage, int sid, int c, double mass, float f1, float f2,
+                                          double *rate_out, const TurbDev &t, int turb, bool quiet)
+{
+    const int nc = m.nc;
+    MxPrim *P2 = reinterpret_cast<MxPrim *>(g.prim[1]);
+    double r1, r2;
+    if (turb && t.hkt[sid]) {
+        // ambient stress and balanced pressure (FP32 face sums, added in
+        // FP32), then the FP64 actuator sink of a support cell: one
+        // conversion per component
+        const int k0 = m.offset[c], k1 = m.offset[c + 1];
+        if (t.stress[sid]) {
+            float x = 0.f, y = 0.f;
+            for (int k = k0; k < k1; ++k) { const float2 v = g.hs[m.faces[k]]; x += g.cw4[k] * v.x; y += g.cw4[k] * v.y; }
+            f1 += x; f2 += y;
+        }
+        float x = 0.f, y = 0.f;
+        for (int k = k0; k < k1; ++k) { const float2 v = g.hp[m.faces[k]]; x += g.cw4[k] * v.x; y += g.cw4[k] * v.y; }
+        r1 = f2d(f1 + x);
+        r2 = f2d(f2 + y);
+        if (t.foot[c]) { r1 += t.raw[c]; r2 += t.raw[nc + c]; }
+    } else {
+        r1 = f2d(f1);
+        r2 = f2d(f2);
+    }
+    if (w.visc.nu && w.visc.nu[sid] > 0.) {
+        // the wet-bank viscosity's FP64 face stresses, FP64 signed weights
+        double x = 0., y = 0.;
+        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+            const int f = m.faces[k];
+            x += g.cw8[k] * w.visc.face[f];
+            y += g.cw8[k] * w.visc.face[m.nf + f];
+        }
+        r1 += x; r2 += y;
+    }
+    if (!finite64(mass) || !finite64(r1) || !finite64(r2)) raise_status(ct, stage, ST_RATE);
+    if (rate_out) { rate_out[c] = mass; rate_out[nc + c] = r1; rate_out[2 * nc + c] = r2; return; }
+    const double dt = ct.trial, dry = ct.dry;
+    if (stage == 1) {
+        const double h = s.work[c] + dt * mass;
+        double hu = s.work[nc + c] + dt * r1, hv = s.work[2 * nc + c] + dt * r2;
+        if (!quiet && lt_zero(h)) raise_status(ct, 1, ST_ENDPOINT);
+        if (le_threshold(h, dry)) { hu = 0.; hv = 0.; }
+        s.q1[c] = h; s.q1[nc + c] = hu; s.q1[2 * nc + c] = hv;
+        // the second stage's input; an invalid one fails that stage
+        if (!put_prim(P2, c, h, hu, hv, s.z[c], dry) && !lt_zero(h)) raise_status(ct, 2, ST_SPATIAL);
+    } else {
+        double h = .5 * s.work[c] + .5 * (s.q1[c] + dt * mass);
+        double hu = .5 * s.work[nc + c] + .5 * (s.q1[nc + c] + dt * r1);
+        double hv = .5 * s.work[2 * nc + c] + .5 * (s.q1[2 * nc + c] + dt * r2);
+        if (!quiet && (!finite64(h) || !finite64(hu) || !finite64(hv) || lt_zero(h))) raise_status(ct, 2, ST_ENDPOINT);
+        if (le_threshold(h, dry)) { hu = 0.; hv = 0.; }
+        drag_f(ct, .5f * ct.trialf, h, hu, hv);
+        double *qn = ct.cur ? s.q[0] : s.q[1];
+        qn[c] = h; qn[nc + c] = hu; qn[2 * nc + c] = hv;
+    }
+}
+
+// Donor-limited mass rate of one cell and the momentum its limited fluxes no
+// longer carry (owner computes, river_midpoint.h:30-41), from the face
+// sweep's FP32 water and the donors' factors, exactly as the face pass
+// km_limit does: both cells of a face compute the same FP64 value
+// double(w) * double(theta), so mass telescopes.
+__device__ __forceinline__ void mx_limited_mass(const MeshDev &m, const Work &w, const MixedGeo &g, int stage, int c,
+                                                double &mass, float &mx, float &my)
+{
+    const float2 *ws = reinterpret_cast<const float2 *>(w.ws);
+    const float *theta32 = reinterpret_cast<const float *>(w.theta);
+    const MxPrim *P = reinterpret_cast<const MxPrim *>((stage == 1 ? g.prim[0] : g.prim[1]));
+    mass = 0.;
+    mx = my = 0.f;
+    for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+        const float wf = ws[m.faces[k]].x;
+        const float wk = g.cw4[k];
+        double water = f2d(wf);
+        if (wf != 0.f) {
+            const int2 id = g.cidx[k];
+            // the donor is the owner for outward (positive) water, else the neighbour
+            const int donor = (wf > 0.f) == ((id.y & 16) != 0) ? c : id.x;
+            if (!(id.y & 8) && donor >= 0) {
+                const float th = theta32[donor];
+                if (th != 1.f) {
+                    const float delta = (th - 1.f) * wf;
+                    water = f2d(wf) * f2d(th);                // exact product
+                    const MxPrim pd = P[donor];
+                    if (pd.wet) { mx -= wk * (delta * pd.u); my -= wk * (delta * pd.v); }
+                }
+            }
+        }
+        mass -= g.cw8[k] * water;
+    }
+}
+
+// Update after the tile sweep, which gathered the rates and factors. After
 // the first gather, block 0 also evaluates each scenario's first-stage CFL
 // test (the second stage's kernels read it).
-__global__ void __launch_bounds__(256) km_update(MeshDev m, StateDev s, Ctrl *ctrl, Work w, MixedGeo g, int stage,
-                                                 double *rate_out, TurbDev t, int turb)
+__global__ void __launch_bounds__(256) km_update_gathered(MeshDev m, StateDev s, Ctrl *ctrl, Work w, MixedGeo g,
+                                                          int stage, double *rate_out, TurbDev t, int turb)
 {
     const int nc = m.nc;
     if (stage == 1 && blockIdx.x == 0)
@@ -1142,88 +1207,174 @@ __global__ void __launch_bounds__(256) km_update(MeshDev m, StateDev s, Ctrl *ct
             Ctrl &c = ctrl[i];
             c.cfl1 = c.trial * bits_to_double(c.peak1) > c.cfl * (1 + 1e-12);
         }
-    const float2 *ws = reinterpret_cast<const float2 *>(w.ws);
-    const float *theta32 = reinterpret_cast<const float *>(w.theta);
     const float *rate32 = reinterpret_cast<const float *>(w.rate);
-    const MxPrim *P = reinterpret_cast<const MxPrim *>((stage == 1 ? g.prim[0] : g.prim[1]));
-    MxPrim *P2 = reinterpret_cast<MxPrim *>(g.prim[1]);
     FOR_ACTIVE_CELLS(m.act, c) {
         const int sid = m.cell_sid[c];
         Ctrl &ct = ctrl[sid];
         if (mx_skip(ct, stage)) continue;
-        double mass = 0.;
-        float mx = 0.f, my = 0.f;
-        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
-            const float wf = ws[m.faces[k]].x;
-            const float wk = g.cw4[k];
-            double water = f2d(wf);
-            if (wf != 0.f) {
-                const int2 id = g.cidx[k];
-                // the donor is the owner for outward (positive) water, else the neighbour
-                const int donor = (wf > 0.f) == ((id.y & 16) != 0) ? c : id.x;
-                if (!(id.y & 8) && donor >= 0) {
-                    const float th = theta32[donor];
-                    if (th != 1.f) {
-                        const float delta = (th - 1.f) * wf;
-                        water = f2d(wf) * f2d(th);                // exact product
-                        const MxPrim pd = P[donor];
-                        if (pd.wet) { mx -= wk * (delta * pd.u); my -= wk * (delta * pd.v); }
-                    }
+        double mass;
+        float mx, my;
+        mx_limited_mass(m, w, g, stage, c, mass, mx, my);
+        mx_finish(m, s, ct, w, g, stage, sid, c, mass, rate32[c] + mx, rate32[nc + c] + my, rate_out, t, turb, false);
+    }
+}
+
+// Gather, donor factor, CFL frequency and stage update in one sweep. A donor
+// factor differs from one only where a cell would run dry within the substep,
+// so every cell is updated with the unlimited fluxes and the cells whose
+// factor is not one are listed; km_limited redoes those and the neighbours
+// they drain into. Bound by memory (it waits on gathers of face values): the
+// separate gather and update read the face waters, the entry weights and the
+// record flags twice and passed the rates through memory, 336 B of DRAM per
+// cell and stage against some 230 here.
+__global__ void __launch_bounds__(256) km_update(MeshDev m, StateDev s, Ctrl *ctrl, Work w, MixedGeo g, int stage,
+                                                 double *rate_out, TurbDev t, int turb)
+{
+    const int nc = m.nc;
+    const MxRec *rec = reinterpret_cast<const MxRec *>(w.rec);
+    const float2 *ws = reinterpret_cast<const float2 *>(w.ws);
+    const float4 *gf = reinterpret_cast<const float4 *>(w.gf);
+    float *theta32 = reinterpret_cast<float *>(w.theta);
+    const int stride = gridDim.x * blockDim.x;
+    const int na = m.act.count[1];
+    for (int first = blockIdx.x * blockDim.x; first < na; first += stride) {   // warp-uniform trip count
+        const int c = first + (int)threadIdx.x < na ? active_cell(m.act, first + threadIdx.x) : nc;
+        bool have = false;
+        float freq = 0.f;
+        int sid = 0;
+        if (c < nc) {
+            sid = m.cell_sid[c];
+            Ctrl &ct = ctrl[sid];
+            if (!mx_skip(ct, stage)) {
+                const float2 hf = *reinterpret_cast<const float2 *>(&rec[c]);
+                const bool active = __float_as_int(hf.y) & 2;
+                const bool owns_open = m.cflags[c] & 1;
+                float out = 0.f, ext = 0.f, interior = 0.f, sum1 = 0.f, sum2 = 0.f;
+                double mass = 0.;
+                for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+                    const int f = m.faces[k];
+                    const float wk = g.cw4[k];            // s * len / area
+                    const float2 wsf = ws[f];
+                    const float4 gff = gf[f];
+                    const float debit = fmaxf(wk * wsf.x, 0.f);   // outward water rate of this cell
+                    if (wk > 0.f) { sum1 += wk * gff.x; sum2 += wk * gff.y; }
+                    else { sum1 += wk * gff.z; sum2 += wk * gff.w; }
+                    out += debit;
+                    if (owns_open) { if (m.bslot[f] >= 0) ext += debit; else interior += debit; }
+                    freq += fabsf(wk) * wsf.y;
+                    mass -= g.cw8[k] * f2d(wsf.x);
                 }
+                const float theta = mx_theta(s, ct, stage, c, hf.x, owns_open, out, ext, interior);
+                theta32[c] = theta;
+                const bool limits = theta != 1.f;
+                if (limits) w.limited[atomicAdd(&m.act.count[2 + stage], 1)] = c;
+                if (isnan(freq)) raise_status(ct, stage, ST_FREQ);
+                else have = true;
+                mx_finish(m, s, ct, w, g, stage, sid, c, mass, active ? -sum1 : 0.f, active ? -sum2 : 0.f, rate_out, t,
+                          turb, limits);
             }
-            mass -= g.cw8[k] * water;
         }
-        float f1 = rate32[c] + mx, f2 = rate32[nc + c] + my;
-        double r1, r2;
-        if (turb && t.hkt[sid]) {
-            // ambient stress and balanced pressure (FP32 face sums, added in
-            // FP32), then the FP64 actuator sink of a support cell: one
-            // conversion per component
-            const int k0 = m.offset[c], k1 = m.offset[c + 1];
-            if (t.stress[sid]) {
-                float x = 0.f, y = 0.f;
-                for (int k = k0; k < k1; ++k) { const float2 v = g.hs[m.faces[k]]; x += g.cw4[k] * v.x; y += g.cw4[k] * v.y; }
-                f1 += x; f2 += y;
+        unsigned long long *peak0 = stage == 1 ? &ctrl[0].peak1 : &ctrl[0].peak2;
+        warp_max_peak_f(peak0, sizeof(Ctrl), sid, have, freq);
+    }
+}
+
+// One listed cell, or a neighbour one drains into, with its limited fluxes.
+// The few threads here wait on chains of dependent loads: D > 0 (cells of at
+// most D faces) requests every entry's data before using any.
+template <int D>
+__device__ __forceinline__ void mx_limited_cell(const MeshDev &m, const StateDev &s, Ctrl *ctrl, const Work &w,
+                                                const MixedGeo &g, int stage, int c, double *rate_out, const TurbDev &t,
+                                                int turb)
+{
+    const MxRec *rec = reinterpret_cast<const MxRec *>(w.rec);
+    const float4 *gf = reinterpret_cast<const float4 *>(w.gf);
+    const int sid = m.cell_sid[c];
+    const bool active = rec[c].flags & 2;
+    double mass = 0.;
+    float mx = 0.f, my = 0.f, sum1 = 0.f, sum2 = 0.f;
+    if constexpr (D > 0) {
+        const float2 *ws = reinterpret_cast<const float2 *>(w.ws);
+        const float *theta32 = reinterpret_cast<const float *>(w.theta);
+        const MxPrim *P = reinterpret_cast<const MxPrim *>((stage == 1 ? g.prim[0] : g.prim[1]));
+        const int k0 = m.offset[c], deg = m.offset[c + 1] - k0;
+        int f[D], donor[D];
+        float wk[D], wf[D], th[D];
+        double w8[D];
+        float4 gff[D];
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            const int k = j < deg ? k0 + j : k0;
+            f[j] = m.faces[k];
+            donor[j] = j < deg && !(g.cidx[k].y & 8) ? k : -1;
+            wk[j] = g.cw4[k]; w8[j] = g.cw8[k];
+        }
+#pragma unroll
+        for (int j = 0; j < D; ++j) { wf[j] = ws[f[j]].x; gff[j] = gf[f[j]]; }
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            if (wf[j] == 0.f) donor[j] = -1;
+            if (donor[j] >= 0) {
+                const int2 id = g.cidx[donor[j]];
+                donor[j] = (wf[j] > 0.f) == ((id.y & 16) != 0) ? c : id.x;
             }
-            float x = 0.f, y = 0.f;
-            for (int k = k0; k < k1; ++k) { const float2 v = g.hp[m.faces[k]]; x += g.cw4[k] * v.x; y += g.cw4[k] * v.y; }
-            r1 = f2d(f1 + x);
-            r2 = f2d(f2 + y);
-            if (t.foot[c]) { r1 += t.raw[c]; r2 += t.raw[nc + c]; }
-        } else {
-            r1 = f2d(f1);
-            r2 = f2d(f2);
+            th[j] = donor[j] >= 0 ? theta32[donor[j]] : 1.f;
         }
-        if (w.visc.nu && w.visc.nu[sid] > 0.) {
-            // the wet-bank viscosity's FP64 face stresses, FP64 signed weights
-            double x = 0., y = 0.;
-            for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
-                const int f = m.faces[k];
-                x += g.cw8[k] * w.visc.face[f];
-                y += g.cw8[k] * w.visc.face[m.nf + f];
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            if (j >= deg) continue;
+            if (wk[j] > 0.f) { sum1 += wk[j] * gff[j].x; sum2 += wk[j] * gff[j].y; }
+            else { sum1 += wk[j] * gff[j].z; sum2 += wk[j] * gff[j].w; }
+            double water = f2d(wf[j]);
+            if (th[j] != 1.f) {
+                const float delta = (th[j] - 1.f) * wf[j];
+                water = f2d(wf[j]) * f2d(th[j]);              // exact product
+                const MxPrim pd = P[donor[j]];
+                if (pd.wet) { mx -= wk[j] * (delta * pd.u); my -= wk[j] * (delta * pd.v); }
             }
-            r1 += x; r2 += y;
+            mass -= w8[j] * water;
         }
-        if (!finite64(mass) || !finite64(r1) || !finite64(r2)) raise_status(ct, stage, ST_RATE);
-        if (rate_out) { rate_out[c] = mass; rate_out[nc + c] = r1; rate_out[2 * nc + c] = r2; continue; }
-        const double dt = ct.trial, dry = ct.dry;
-        if (stage == 1) {
-            const double h = s.work[c] + dt * mass;
-            double hu = s.work[nc + c] + dt * r1, hv = s.work[2 * nc + c] + dt * r2;
-            if (lt_zero(h)) raise_status(ct, 1, ST_ENDPOINT);
-            if (le_threshold(h, dry)) { hu = 0.; hv = 0.; }
-            s.q1[c] = h; s.q1[nc + c] = hu; s.q1[2 * nc + c] = hv;
-            // the second stage's input; an invalid one fails that stage
-            if (!put_prim(P2, c, h, hu, hv, s.z[c], dry) && !lt_zero(h)) raise_status(ct, 2, ST_SPATIAL);
-        } else {
-            double h = .5 * s.work[c] + .5 * (s.q1[c] + dt * mass);
-            double hu = .5 * s.work[nc + c] + .5 * (s.q1[nc + c] + dt * r1);
-            double hv = .5 * s.work[2 * nc + c] + .5 * (s.q1[2 * nc + c] + dt * r2);
-            if (!finite64(h) || !finite64(hu) || !finite64(hv) || lt_zero(h)) raise_status(ct, 2, ST_ENDPOINT);
-            if (le_threshold(h, dry)) { hu = 0.; hv = 0.; }
-            drag_f(ct, .5f * ct.trialf, h, hu, hv);
-            double *qn = ct.cur ? s.q[0] : s.q[1];
-            qn[c] = h; qn[nc + c] = hu; qn[2 * nc + c] = hv;
+    } else {
+        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+            const float wk = g.cw4[k];
+            const float4 gff = gf[m.faces[k]];
+            if (wk > 0.f) { sum1 += wk * gff.x; sum2 += wk * gff.y; }
+            else { sum1 += wk * gff.z; sum2 += wk * gff.w; }
+        }
+        mx_limited_mass(m, w, g, stage, c, mass, mx, my);
+    }
+    mx_finish(m, s, ctrl[sid], w, g, stage, sid, c, mass, (active ? -sum1 : 0.f) + mx, (active ? -sum2 : 0.f) + my,
+              rate_out, t, turb, false);
+}
+
+// Redo the listed cells and the neighbours they drain into with the limited
+// fluxes. A cell reached from several list entries is redone by each with the
+// same result; nothing read here is written here (stage 1 reads work and
+// writes q1 and the second stage's primitives, stage 2 reads both states and
+// writes the inactive buffer). Block 0 also evaluates each scenario's
+// first-stage CFL test, which the second stage's kernels read.
+template <int D>
+__global__ void __launch_bounds__(64) km_limited(MeshDev m, StateDev s, Ctrl *ctrl, Work w, MixedGeo g, int stage,
+                                                 double *rate_out, TurbDev t, int turb)
+{
+    if (stage == 1 && blockIdx.x == 0)
+        for (int i = threadIdx.x; i < m.nscen; i += blockDim.x) {
+            Ctrl &c = ctrl[i];
+            c.cfl1 = c.trial * bits_to_double(c.peak1) > c.cfl * (1 + 1e-12);
+        }
+    const float2 *ws = reinterpret_cast<const float2 *>(w.ws);
+    const float *theta32 = reinterpret_cast<const float *>(w.theta);
+    // four threads per listed cell: itself, then its entries in turn; a
+    // neighbour that is listed too is left to its own entry
+    const int n = 4 * m.act.count[2 + stage];
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int c = w.limited[i >> 2], part = i & 3;
+        if (part == 0) mx_limited_cell<D>(m, s, ctrl, w, g, stage, c, rate_out, t, turb);
+        for (int k = m.offset[c] + (part + 3) % 4; k < m.offset[c + 1]; k += 4) {
+            const int2 id = g.cidx[k];
+            const float wf = ws[m.faces[k]].x;
+            if (id.x >= 0 && wf != 0.f && (wf > 0.f) == ((id.y & 16) != 0) && theta32[id.x] == 1.f)
+                mx_limited_cell<D>(m, s, ctrl, w, g, stage, id.x, rate_out, t, turb);
         }
     }
 }
@@ -1311,7 +1462,6 @@ int mixed_max_block(int kind, int maxdeg)
     case K_DRAG: fn = (const void *)brx_mx::km_open_drag; break;
     case K_CELLS: fn = small ? (const void *)brx_mx::km_cells<4> : (const void *)brx_mx::km_cells<MAX_CELL_FACES>; break;
     case K_FACES: fn = (const void *)brx_mx::km_faces; break;
-    case K_GATHER: fn = (const void *)brx_mx::km_gather; break;
     case K_LIMIT: fn = (const void *)brx_mx::km_limit; break;
     case K_UPDATE: fn = (const void *)brx_mx::km_update; break;
     case KH_CELLS: fn = (const void *)brx_mx::km_hllc_cells; break;
@@ -1383,9 +1533,6 @@ int mixed_kernel(const Launch &L, int kind, int stage, double *out)
         brx_mx::km_faces<<<SHAPE(K_FACES, nf), 0, st>>>(L.mesh, L.state, L.bnd, L.ctrl, L.work, L.mx, stage, L.turb,
                                                     L.has_turb);
         return 1;
-    case K_GATHER:
-        brx_mx::km_gather<<<SHAPE(K_GATHER, nc), 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage);
-        return 1;
     case K_TILE: {
         const int grid = std::max(1, std::min(L.tiles.ntiles, L.shape[K_TILE].per_sm * L.sms));
         brx_mx::km_tile<4><<<grid, TILE_THREADS, L.tile_smem, st>>>(L.mesh, L.state, L.bnd, L.ctrl, L.work, L.mx,
@@ -1396,9 +1543,23 @@ int mixed_kernel(const Launch &L, int kind, int stage, double *out)
         brx_mx::km_limit<<<SHAPE(K_LIMIT, nf), 0, st>>>(L.mesh, L.ctrl, L.work, L.mx, stage);
         return 1;
     case K_UPDATE:
+        if (L.tile_smem > 0) {
+            brx_mx::km_update_gathered<<<SHAPE(K_UPDATE, nc), 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage, out,
+                                                                       L.turb, L.has_turb);
+            return 1;
+        }
         brx_mx::km_update<<<SHAPE(K_UPDATE, nc), 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage, out, L.turb,
                                                      L.has_turb);
-        return 1;
+        {
+            const int grid = std::max(1, std::min((nc + 63) / 64, 4 * L.sms));
+            if (L.maxdeg <= 3)
+                brx_mx::km_limited<3><<<grid, 64, 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage, out, L.turb, L.has_turb);
+            else if (small)
+                brx_mx::km_limited<4><<<grid, 64, 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage, out, L.turb, L.has_turb);
+            else
+                brx_mx::km_limited<0><<<grid, 64, 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage, out, L.turb, L.has_turb);
+        }
+        return 2;
     case K_PRIM:
         brx_mx::km_prim<<<L.grid_c256, 256, 0, st>>>(L.mesh, L.state, L.ctrl, L.mx);
         return 1;

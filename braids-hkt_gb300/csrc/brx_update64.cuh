@@ -177,16 +177,17 @@ __device__ void limited_cell(const MeshDev &m, const StateDev &s, Ctrl *ctrl, co
 __global__ void __launch_bounds__(64) k_limited(MeshDev m, StateDev s, Ctrl *ctrl, Work w, int stage, double *rate_out,
                                                 TurbDev t, int turb, Prim64 *prim)
 {
-    const int n = m.act.count[2 + stage];
+    // four threads per listed cell: itself, then its entries in turn; a
+    // neighbour that is listed too is left to its own entry
+    const int n = 4 * m.act.count[2 + stage];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int c = w.limited[i];
-        if (skip_stage(ctrl[m.cell_sid[c]], stage)) continue;
-        limited_cell(m, s, ctrl, w, stage, c, rate_out, t, turb, prim);
-        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+        const int c = w.limited[i >> 2], part = i & 3;
+        if (part == 0) limited_cell(m, s, ctrl, w, stage, c, rate_out, t, turb, prim);
+        for (int k = m.offset[c] + (part + 3) % 4; k < m.offset[c + 1]; k += 4) {
             const int f = m.faces[k];
             const double water = w.ws[f].x;
             const int o = m.signs[k] > 0 ? m.neighbour[f] : m.owner[f];
-            if (o >= 0 && (m.signs[k] > 0 ? water > 0. : water < 0.))
+            if (o >= 0 && (m.signs[k] > 0 ? water > 0. : water < 0.) && w.theta[o] == 1.)
                 limited_cell(m, s, ctrl, w, stage, o, rate_out, t, turb, prim);
         }
     }
