@@ -344,8 +344,22 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
         double *p_forcing, *p_terms, *p_trace, *p_flux, *p_sums;
         TRY(s->alloc(&p_forcing, 2 * (size_t)nseg)); TRY(s->alloc(&p_terms, 3 * (size_t)s->nslot));
         TRY(s->alloc(&p_trace, 3 * (size_t)s->nslot)); TRY(s->alloc(&p_flux, 3 * (size_t)s->nslot));
-        TRY(s->alloc(&p_sums, 3 * (size_t)nseg)); TRY(s->alloc(&b.own_sum, s->nown));
-        b.cluster = 1;
+        TRY(s->alloc(&p_sums, 3 * (size_t)nseg)); TRY(s->alloc(&b.water_sum, s->nslot));
+        {
+            std::vector<unsigned char> several(s->nslot, 0);
+            std::vector<int> scen_several(nscen, 0);
+            for (int i = 0; i < nscen; ++i)
+                for (int u = scen_own[i]; u < scen_own[i + 1]; ++u)
+                    if (own_off[u + 1] - own_off[u] > 1) {
+                        scen_several[i] = 1;
+                        for (int j = own_off[u]; j < own_off[u + 1]; ++j) several[own_slot[j]] = 1;
+                    }
+            unsigned char *p_several;
+            int *p_scen_several;
+            TRY(s->upload(&p_several, several.data(), several.size()));
+            TRY(s->upload(&p_scen_several, scen_several.data(), nscen));
+            b.several = p_several; b.scen_several = p_scen_several;
+        }
         b.seg_mode = s->d_seg_mode_rw; b.stage_policy = s->d_stage_policy_rw; b.ext_bed = s->d_ext_bed_rw;
         b.forcing = p_forcing; b.terms = p_terms; b.trace = p_trace; b.flux = p_flux; b.seg_sums = p_sums;
         b.table_len = 0; b.table_time = nullptr; b.table_value = nullptr;
@@ -554,17 +568,18 @@ extern "C" int brx_boundary_set(brx_solver *s, const int *seg_mode, const int *s
     }
     s->h_seg_mode.assign(seg_mode, seg_mode + nseg);
     const int inlet = std::count(seg_mode, seg_mode + nseg, 9) > 0;
-    // blocks per scenario of the boundary kernel: one for 128 faces (a block has
-    // a warp per sub-partition), at most the portable cluster of eight; section
-    // solves work in a single block
+    // the boundary kernel: a thread per face where no segment needs a section
+    // solve and every scenario's tiles of 64 faces fit the portable cluster of
+    // eight blocks of two; else one block per scenario
     int sections = 0, widest = 0, cluster = 1;
     for (int sg = 0; sg < nseg; ++sg) sections |= seg_mode[sg] != 2 && seg_mode[sg] != 3 && seg_mode[sg] != 6;
     for (int i = 0; i < s->nscen; ++i) {
-        int faces = 0;
-        for (int sg = s->seg_offset[i]; sg < s->seg_offset[i + 1]; ++sg) faces += s->seg_faces[sg];
-        widest = std::max(widest, faces);
+        int tiles = 0;
+        for (int sg = s->seg_offset[i]; sg < s->seg_offset[i + 1]; ++sg) tiles += std::max(1, (s->seg_faces[sg] + 63) / 64);
+        widest = std::max(widest, tiles);
     }
-    while (!sections && cluster < 8 && widest > 128 * cluster) cluster *= 2;
+    while (cluster < 8 && widest > 2 * cluster) cluster *= 2;
+    if (sections || widest > 16) cluster = 0;
     if (inlet != s->bnd.inlet || sections != s->bnd.sections || cluster != s->bnd.cluster) s->graph_dirty = true;
     s->bnd.inlet = inlet; s->bnd.sections = sections; s->bnd.cluster = cluster;
     TRY(clear_inlet_lines(s));

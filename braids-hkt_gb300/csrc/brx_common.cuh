@@ -190,8 +190,10 @@ struct BoundaryDev {
     const double *table_value;  // (2, nseg, table_len)
     const int *own_cell, *own_off, *own_slot;  // unique owners, CSR into slots (boundary order)
     double *terms;           // (3, nslot) scratch: tile sums / inlet factors, -, conveyance weights
-    double2 *own_sum;        // (nown) water and gross sums of 32 owners from each
-    int cluster;             // blocks per scenario of the boundary kernel
+    double2 *water_sum;      // (nslot) water and gross sums of 32 faces from a multiple of 32 in their tile
+    const unsigned char *several;        // (nslot) the face's owner has several open faces
+    const int *scen_several;             // (nscen) some owner has
+    int cluster;             // blocks per scenario of k_boundary_plain; 0: k_boundary
     int sections;            // a segment needs a section solve (modes 4, 5, 9, 10, 11)
     double *trace, *flux;    // (3, nslot) each
     double *seg_sums;        // (3, nseg): wetted stage sum, wetted width, weight total

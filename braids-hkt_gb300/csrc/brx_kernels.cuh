@@ -1284,41 +1284,80 @@ __device__ void inlet_allocation(const MeshDev &m, const BoundaryDev &b, const C
 // stock of the substep's start state work (hllc.py:91-97), status of stage 1.
 constexpr int STAGE_HANCOCK = 3;
 
-// Exterior trace and flux of slot k on a segment of mode 2, 3 or 6
-// (river_exterior_bed.h:94-174); returns the face status. total: the
-// segment's conveyance, w: the face's.
-__device__ __forceinline__ int plain_face(const MeshDev &m, const BoundaryDev &b, int k, int sg, const double *q,
-                                          const double *z, double dry, double grav, double speed_limit, double total,
-                                          double w, double tr[3], double fl[3])
+// One open face: its ids, geometry and its owner's state.
+struct OpenFace {
+    int f, c, sg, mode;
+    double h, hu, hv, z, bed, nx, ny, len;
+};
+
+__device__ __forceinline__ OpenFace open_face(const MeshDev &m, const BoundaryDev &b, int k, int sg, const double *q,
+                                              const double *z)
 {
-    const int nc = m.nc, f = b.slot_face[k], c = m.owner[f], mode = b.seg_mode[sg];
-    const double h0 = q[c], nx = m.normal[f], ny = m.normal[m.nf + f], bed = b.ext_bed[k];
-    const double Q = b.forcing[sg], stagev = b.forcing[b.nseg + sg];
-    double h = h0 + z[c] - bed, ux = 0., uy = 0.;
+    OpenFace o;
+    o.f = b.slot_face[k]; o.c = m.owner[o.f]; o.sg = sg; o.mode = b.seg_mode[sg];
+    o.h = q[o.c]; o.hu = q[m.nc + o.c]; o.hv = q[2 * m.nc + o.c]; o.z = z[o.c];
+    o.bed = b.ext_bed[k]; o.nx = m.normal[o.f]; o.ny = m.normal[m.nf + o.f]; o.len = m.length[o.f];
+    return o;
+}
+
+// Forcing table row (0 discharge, 1 stage) of segment sg at time t:
+// piecewise linear, the end values outside.
+__device__ __forceinline__ double table_forcing(const BoundaryDev &b, int row, int sg, double t)
+{
+    const int L = b.table_len;
+    const double *y = b.table_value + ((size_t)row * b.nseg + sg) * L;
+    if (t <= b.table_time[0]) return y[0];
+    if (t >= b.table_time[L - 1]) return y[L - 1];
+    // last knot at or before t, capped at L - 2; (1 - w) y_i + w y_{i+1}
+    // (RiverHydraulicSchedule.sample, river_hydraulic_schedule.py:57-65)
+    int i = 0;
+    while (i < L - 2 && b.table_time[i + 1] <= t) ++i;
+    const double w = (t - b.table_time[i]) / (b.table_time[i + 1] - b.table_time[i]);
+    return (1. - w) * y[i] + w * y[i + 1];
+}
+
+// Conveyance weight of an inlet face under its segment's mean wetted stage.
+template <class F>
+__device__ __forceinline__ double face_weight(const Ctrl &ct, const OpenFace &o, double stage_sum, double width)
+{
+    if (!(width > 0.)) return 0.;
+    const double h = o.h + o.z - o.bed, depth = stage_sum / width - o.bed;
+    if (!greater(h, ct.dry) || !greater(depth, 0.)) return 0.;
+    const int rmode = ct.roughness_mode < 3 ? ct.roughness_mode : 3;
+    return conveyance<F>(rmode, ct.roughness_mode == 4, F(depth), F(h), ct) * o.len;
+}
+
+// Exterior trace and flux of a face on a segment of mode 2, 3 or 6 with
+// discharge Q or stage level (river_exterior_bed.h:94-174); returns the face
+// status. total: the segment's conveyance, w: the face's.
+__device__ __forceinline__ int plain_face(const OpenFace &o, double Q, double level, int policy, double dry, double grav,
+                                          double speed_limit, double total, double w, double tr[3], double fl[3])
+{
+    const double nx = o.nx, ny = o.ny, bed = o.bed;
+    double h = o.h + o.z - bed, ux = 0., uy = 0.;
     if (!greater(h, 0.)) h = 0.;
     const double geometric = h;
-    const bool wet0 = greater(h0, dry);
+    const bool wet0 = greater(o.h, dry);
     if (wet0) {
-        const double r = reciprocal(h0);
-        ux = quotient(q[nc + c], h0, r); uy = quotient(q[2 * nc + c], h0, r);
+        const double r = reciprocal(o.h);
+        ux = quotient(o.hu, o.h, r); uy = quotient(o.hv, o.h, r);
     }
     const double un = ux * nx + uy * ny;
     double tx = ux - un * nx, ty = uy - un * ny, speed = 0.;
-    if (mode == 6) {
+    if (o.mode == 6) {
         if (Q > 0. && total <= 0.) return 1;
         if (greater(h, dry) && Q > 0.) {
-            const double den = total * h * m.length[f];
+            const double den = total * h * o.len;
             speed = quotient(-Q * w, den, reciprocal(den));
         }
-    } else if (mode == 3) {
+    } else if (o.mode == 3) {
         if (!wet0) h = 0.;
         else if (greater(h, dry)) {
             if (un < sqrt(grav * h)) return 6;
             speed = un;
         }
-    } else if (mode == 2) {
-        const double target = greater(stagev - bed, 0.) ? stagev - bed : 0.;
-        const int policy = b.stage_policy[sg];
+    } else if (o.mode == 2) {
+        const double target = greater(level - bed, 0.) ? level - bed : 0.;
         if (policy && (!wet0 || !greater(h, dry)) && greater(target, dry)) return 4;
         if (!wet0) h = 0.;
         if (greater(h, dry)) {
@@ -1351,37 +1390,207 @@ __device__ __forceinline__ int plain_face(const MeshDev &m, const BoundaryDev &b
         fx = quotient(water * tr[1], h, r) + .5 * grav * h * h * nx;
         fy = quotient(water * tr[2], h, r) + .5 * grav * h * h * ny;
     }
-    const double pressure = wet0 ? .5 * grav * (h0 * h0 - geometric * geometric) : 0.;
+    const double pressure = wet0 ? .5 * grav * (o.h * o.h - geometric * geometric) : 0.;
     fl[0] = water; fl[1] = fx + pressure * nx; fl[2] = fy + pressure * ny;
     return 0;
 }
 
-// The open boundary of one scenario. What bounds it: a chain of short FP64
-// phases on one SM, where a warp's FP64 instruction takes 65 clocks and the
-// four sub-partitions are all there is. CLUSTER: a thread-block cluster shares
-// the scenario, a tile of 64 faces per pair of warps, with three cluster
-// barriers; used when no segment needs a section solve (those work in one
-// block) and the scenario is wider than one block's 128 faces. The sums keep
-// the reference's fixed tree (64-face tiles, then the tiles in order) and the
-// ledger its own, so no result depends on the cluster's size.
-template <class F, bool CLUSTER>
-__global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int stage_in)
+// Outlet faces' share of an owner's stock: total and reserved outward rates
+// against base area / trial; returns 1 where nothing is to be capped.
+__device__ __forceinline__ double cap_factor(double base, double area, double trial, double rtrial, double total,
+                                             double reserved)
 {
-    __shared__ double tile_buf[2][BOUNDARY_TILES], warp_buf[BOUNDARY_THREADS / 32][2][64];
-    int rank = 0, size = 1;
-    if constexpr (CLUSTER) {
-        rank = (int)cooperative_groups::this_cluster().block_rank();
-        size = (int)cooperative_groups::this_cluster().num_blocks();
+    const double left = quotient(base * area, trial, rtrial) - reserved;
+    const double available = greater(left, 0.) ? left : 0.;
+    if (!greater(total, available)) return 1.;
+    return fmin(1., available / fmax(total, 1e-300)) * (1. - 32. * EPS);
+}
+
+// Trace and flux of an outlet face capped by the owner's factor.
+__device__ __forceinline__ void cap_face(double factor, double tr[3], double fl[3])
+{
+    const double water = fl[0], depth = tr[0], denom = fmax(depth, 1e-300);
+    const double ux = depth > 0. ? tr[1] / denom : 0., uy = depth > 0. ? tr[2] / denom : 0.;
+    fl[1] += (factor * factor - 1.) * water * ux;
+    fl[2] += (factor * factor - 1.) * water * uy;
+    fl[0] = water * factor;
+    tr[1] *= factor;
+    tr[2] *= factor;
+}
+
+// The cap of every owner from u0 + first on, in steps (an owner's faces in boundary order).
+__device__ __forceinline__ void cap_owners(const MeshDev &m, const BoundaryDev &b, const double *base, double trial,
+                                           int first, int u1, int step, bool several)
+{
+    const size_t ns = b.nslot;
+    const double rtrial = reciprocal(trial);
+    for (int u = first; u < u1; u += step) {
+        const int j0 = b.own_off[u], j1 = b.own_off[u + 1], c = b.own_cell[u];
+        if (several && j1 - j0 < 2) continue;
+        double total = 0., reserved = 0.;
+        for (int j = j0; j < j1; ++j) {
+            const int k = b.own_slot[j], f = b.slot_face[k];
+            const double flux = b.flux[k], debit = greater(flux, 0.) ? flux * m.length[f] : 0.;
+            if (is_outlet(b.seg_mode[m.bid[f]])) total += debit; else reserved += debit;
+        }
+        const double factor = cap_factor(base[c], m.area[c], trial, rtrial, total, reserved);
+        if (factor == 1.) continue;
+        for (int j = j0; j < j1; ++j) {
+            const int k = b.own_slot[j];
+            double tr[3] = {b.trace[k], b.trace[ns + k], b.trace[2 * ns + k]};
+            double fl[3] = {b.flux[k], b.flux[ns + k], b.flux[2 * ns + k]};
+            if (!is_outlet(b.seg_mode[m.bid[b.slot_face[k]]]) || !(fl[0] > 0.)) continue;
+            cap_face(factor, tr, fl);
+#pragma unroll
+            for (int r = 0; r < 3; ++r) { b.trace[r * ns + k] = tr[r]; b.flux[r * ns + k] = fl[r]; }
+        }
     }
-    auto team_sync = [&] {
-        if constexpr (CLUSTER) cooperative_groups::this_cluster().sync();
-        else __syncthreads();
-    };
-    const int sid = blockIdx.x / size, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+}
+
+// Water and gross water of 32 faces by a butterfly; the result in every lane.
+__device__ __forceinline__ double2 warp_water(double v)
+{
+    double2 a = make_double2(v, fabs(v));
+    for (int o = 16; o > 0; o >>= 1) {
+        a.x += __shfl_xor_sync(0xffffffffu, a.x, o);
+        a.y += __shfl_xor_sync(0xffffffffu, a.y, o);
+    }
+    return a;
+}
+
+// The scenario's sum over its open faces of (outward water flux x length),
+// with each face's water as the update consumes it (the mixed form carries it
+// in FP32), and of its magnitude, from the sums of 32 faces in slot order. The
+// controller turns the stage sums into the boundary ledger. Threads 0 and 1.
+__device__ __forceinline__ void scenario_water(const BoundaryDev &b, Ctrl &ct, int stage, int s0, int ntile)
+{
+    if (threadIdx.x >= 2) return;
+    double total = 0.;
+    for (int i = 0; i < ntile; ++i) {
+        const SlotTile tile = slot_tile(b, s0, i);
+        for (int k = tile.first; k < tile.end; k += 32) total += threadIdx.x ? b.water_sum[k].y : b.water_sum[k].x;
+    }
+    if (threadIdx.x) ct.bgross[stage - 1] = total; else ct.bflux[stage - 1] = total;
+}
+
+// The open boundary of one scenario whose segments have modes 2, 3 and 6 and
+// at most 64 faces x 2 x cluster size: a thread per face, a thread-block
+// cluster per scenario. What bounds it: short FP64 phases (a warp's FP64
+// instruction takes 65 clocks, so a block has one warp per sub-partition and
+// wide openings more blocks) between dependent loads; each face's data is
+// loaded once, at the start. The sums keep the reference's fixed tree (64-face
+// tiles, then the tiles in order), so no result depends on the cluster's size.
+template <class F>
+__global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary_plain(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl,
+                                                                     int stage_in)
+{
+    __shared__ double buf[2][2][64];
+    const auto cluster = cooperative_groups::this_cluster();
+    const int rank = (int)cluster.block_rank(), size = (int)cluster.num_blocks();
+    const int sid = blockIdx.x / size, pair = threadIdx.x >> 6, at = threadIdx.x & 63;
     Ctrl &ct = ctrl[sid];
     const bool hancock = stage_in == STAGE_HANCOCK;
     const int stage = hancock ? 1 : stage_in;
-    if (skip_stage(ct, stage)) return;            // the same for every block of the cluster
+    const int s0 = b.scen_seg[sid], s1 = b.scen_seg[sid + 1];
+    if (s0 == s1 || skip_stage(ct, stage)) return;            // the same for every block of the cluster
+    const int nseg = b.nseg;
+    const size_t ns = b.nslot;
+    const double *q = stage == 1 && !hancock ? s.work : s.q1;
+    const double *base = hancock ? s.work : q;    // stock of the stage start (the substep start for Hancock)
+    int ntile = 0;
+    for (int sg = s0; sg < s1; ++sg) ntile += tile_count(b, sg);
+    const int i = 2 * rank + pair;
+    const SlotTile tile = i < ntile ? slot_tile(b, s0, i) : SlotTile{s0, 0, 0};
+    const int k = tile.first + at, n = tile.end - tile.first;
+    const bool on = at < n;
+    OpenFace o{};
+    double stock = 0., area = 0.;
+    bool several = false;
+    if (on) {
+        o = open_face(m, b, k, tile.sg, q, s.z);
+        stock = hancock ? base[o.c] : o.h;
+        area = m.area[o.c];
+        several = b.several[k];
+    }
+    const int mode = n > 0 ? b.seg_mode[tile.sg] : 0, policy = n > 0 ? b.stage_policy[tile.sg] : 0;
+    const double dry = ct.dry, trial = ct.trial;
+    double Q = 0., level = 0.;
+    if (b.table_len > 0) {
+        const double t = ct.time0 + ct.elapsed + (stage == 2 ? trial : hancock ? .5 * trial : 0.0);
+        const bool first = n > 0 && tile.first == b.seg_off[tile.sg] && at == 0;     // writes the sampled rows
+        if (n > 0 && (mode == 6 || first)) Q = table_forcing(b, 0, tile.sg, t);
+        if (n > 0 && (mode == 2 || first)) level = table_forcing(b, 1, tile.sg, t);
+        if (first) { b.forcing[tile.sg] = Q; b.forcing[nseg + tile.sg] = level; }
+    } else if (n > 0) { Q = b.forcing[tile.sg]; level = b.forcing[nseg + tile.sg]; }
+    // wetted stage sum and wetted width of the conveyance inlets' tiles: a row
+    // per warp, its first lane in slot order
+    const bool inlet = mode == 6;
+    if (inlet && on) {
+        const double w = greater(o.h, dry) ? o.len : 0.;
+        buf[pair][0][at] = (o.z + o.h) * w;
+        buf[pair][1][at] = w;
+    }
+    __syncthreads();
+    if (inlet && (threadIdx.x & 31) == 0) {
+        const int row = (threadIdx.x >> 5) & 1;
+        double sum = 0.;
+#pragma unroll 8
+        for (int j = 0; j < n; ++j) sum += buf[pair][row][j];
+        b.terms[row * ns + tile.first] = sum;
+    }
+    cluster.sync();
+    double w = 0., total = 0.;
+    if (inlet) {
+        double stage_sum = 0., width = 0.;
+        for (int j = b.seg_off[tile.sg]; j < b.seg_off[tile.sg + 1]; j += 64) { stage_sum += b.terms[j]; width += b.terms[ns + j]; }
+        if (on) { w = face_weight<F>(ct, o, stage_sum, width); buf[pair][0][at] = w; }
+    }
+    __syncthreads();
+    if (inlet && at == 0) {
+        double sum = 0.;
+#pragma unroll 8
+        for (int j = 0; j < n; ++j) sum += buf[pair][0][j];
+        b.terms[2 * ns + tile.first] = sum;
+    }
+    cluster.sync();
+    double tr[3] = {0., 0., 0.}, fl[3] = {0., 0., 0.};
+    bool bad = false;
+    if (inlet)
+        for (int j = b.seg_off[tile.sg]; j < b.seg_off[tile.sg + 1]; j += 64) total += b.terms[2 * ns + j];
+    if (on) {
+        bad = plain_face(o, Q, level, policy, dry, ct.grav, ct.speed_limit, total, w, tr, fl) != 0;
+        // outlet stock cap of an owner with one open face; the others below
+        if (!several && is_outlet(mode) && greater(fl[0], 0.)) {
+            const double factor = cap_factor(stock, area, trial, reciprocal(trial), fl[0] * o.len, 0.);
+            if (factor != 1.) cap_face(factor, tr, fl);
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) { b.trace[r * ns + k] = tr[r]; b.flux[r * ns + k] = fl[r]; }
+    }
+    if (bad) raise_status(ct, stage, ST_SPATIAL);
+    if (b.scen_several[sid]) {
+        cluster.sync();
+        if (rank == 0)
+            cap_owners(m, b, base, trial, b.scen_own[sid] + (int)threadIdx.x, b.scen_own[sid + 1], BOUNDARY_THREADS, true);
+        cluster.sync();
+        if (on && several) fl[0] = b.flux[k];
+    }
+    const double2 sum = warp_water(on ? double(F(fl[0])) * o.len : 0.);
+    if (on && (threadIdx.x & 31) == 0) b.water_sum[k] = sum;
+    cluster.sync();
+    if (rank == 0) scenario_water(b, ct, stage, s0, ntile);
+}
+
+// The open boundary of one scenario in one block: any modes, any width.
+template <class F>
+__global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int stage_in)
+{
+    __shared__ double tile_buf[2][BOUNDARY_TILES], warp_buf[BOUNDARY_THREADS / 32][2][64];
+    const int sid = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    Ctrl &ct = ctrl[sid];
+    const bool hancock = stage_in == STAGE_HANCOCK;
+    const int stage = hancock ? 1 : stage_in;
+    if (skip_stage(ct, stage)) return;
     const int s0 = b.scen_seg[sid], s1 = b.scen_seg[sid + 1];
     if (s0 == s1) return;
     const int nseg = b.nseg;
@@ -1390,34 +1599,18 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
     const double *base = hancock ? s.work : q;    // stock of the stage start (the substep start for Hancock)
     const double *z = s.z;
     const double dry = ct.dry, grav = ct.grav;
-    const double t = ct.time0 + ct.elapsed + (stage == 2 ? ct.trial : hancock ? .5 * ct.trial : 0.0);
-    // forcing at the stage clock (piecewise linear tables, else constant); each
-    // block of a cluster writes the same values
+    // forcing at the stage clock (piecewise linear tables, else constant)
     if (b.table_len > 0) {
+        const double t = ct.time0 + ct.elapsed + (stage == 2 ? ct.trial : hancock ? .5 * ct.trial : 0.0);
         for (int sg = s0 + threadIdx.x; sg < s1; sg += blockDim.x)
-            for (int row = 0; row < 2; ++row) {
-                const int L = b.table_len;
-                const double *y = b.table_value + ((size_t)row * b.nseg + sg) * L;
-                double val;
-                if (t <= b.table_time[0]) val = y[0];
-                else if (t >= b.table_time[L - 1]) val = y[L - 1];
-                else {
-                    // last knot at or before t, capped at L - 2; (1 - w) y_i + w y_{i+1}
-                    // (RiverHydraulicSchedule.sample, river_hydraulic_schedule.py:57-65)
-                    int i = 0;
-                    while (i < L - 2 && b.table_time[i + 1] <= t) ++i;
-                    const double w = (t - b.table_time[i]) / (b.table_time[i + 1] - b.table_time[i]);
-                    val = (1. - w) * y[i] + w * y[i + 1];
-                }
-                b.forcing[(size_t)row * b.nseg + sg] = val;
-            }
+            for (int row = 0; row < 2; ++row) b.forcing[(size_t)row * nseg + sg] = table_forcing(b, row, sg, t);
         __syncthreads();
     }
     // critical, then normal reference lines of the exact-discharge inlets
     // (river_exterior_bed.py:199-200); a section without a root rejects the trial
     __shared__ SectionWork section;
     bool line_failed = false;
-    if (!CLUSTER && b.sections && b.line_kind) {
+    if (b.sections && b.line_kind) {
         for (int pass = 1; pass <= 2; ++pass)
             for (int sg = s0; sg < s1; ++sg)          // block-uniform
                 if (b.seg_mode[sg] == 9 && b.line_kind[sg] == pass &&
@@ -1425,9 +1618,9 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
                     line_failed = true;
         __syncthreads();
     }
-    const int ntile = [&] { int n = 0; for (int sg = s0; sg < s1; ++sg) n += tile_count(b, sg); return n; }();
+    int ntile = 0;
+    for (int sg = s0; sg < s1; ++sg) ntile += tile_count(b, sg);
     // wetted stage sum and wetted width of the conveyance inlets' segments
-    // (every block forms all of them: three instructions a face)
     for (int i = warp; i < ntile; i += BOUNDARY_THREADS / 32) {
         const SlotTile tile = slot_tile(b, s0, i);
         if (b.seg_mode[tile.sg] != 6) continue;
@@ -1454,54 +1647,49 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
         b.seg_sums[sg] = stage_sum; b.seg_sums[nseg + sg] = width;
     }
     __syncthreads();
-    // conveyance weights, a tile per block of the cluster in turn
-    const int rmode = ct.roughness_mode < 3 ? ct.roughness_mode : 3;
-    const int waqua = ct.roughness_mode == 4;
-    for (int i = rank + size * warp; i < ntile; i += size * (BOUNDARY_THREADS / 32)) {
+    // conveyance weights
+    for (int i = warp; i < ntile; i += BOUNDARY_THREADS / 32) {
         const SlotTile tile = slot_tile(b, s0, i);
         if (b.seg_mode[tile.sg] != 6) continue;
-        const double width = b.seg_sums[nseg + tile.sg];
-        const double level = width > 0. ? b.seg_sums[tile.sg] / width : 0.;
         double lo[1] = {0.}, hi[1] = {0.};
 #pragma unroll
         for (int half = 0; half < 2; ++half) {
             const int k = tile.first + lane + 32 * half;
             if (k >= tile.end) continue;
-            const int f = b.slot_face[k], c = m.owner[f];
-            const double bed = b.ext_bed[k], h = q[c] + z[c] - bed, depth = level - bed;
-            double w = 0.;
-            if (width > 0. && greater(h, dry) && greater(depth, 0.))
-                w = conveyance<F>(rmode, waqua, F(depth), F(h), ct) * m.length[f];
+            const double w = face_weight<F>(ct, open_face(m, b, k, tile.sg, q, z), b.seg_sums[tile.sg], b.seg_sums[nseg + tile.sg]);
             b.terms[2 * ns + k] = w;
             (half ? hi : lo)[0] = w;
         }
         const double sum = tile_sum<1>(warp_buf[warp], tile.end - tile.first, lo, hi);
-        if (lane == 0) b.terms[tile.first] = sum;
+        if (lane == 0) tile_buf[0][i] = sum;
     }
-    team_sync();
+    __syncthreads();
     for (int sg = s0 + threadIdx.x; sg < s1; sg += blockDim.x) {
         if (b.seg_mode[sg] != 6) continue;
+        int first = 0;
+        for (int u = s0; u < sg; ++u) first += tile_count(b, u);
         double total = 0.;
-        for (int k = b.seg_off[sg]; k < b.seg_off[sg + 1]; k += 64) total += b.terms[k];
+        for (int i = 0; i < tile_count(b, sg); ++i) total += tile_buf[0][first + i];
         b.seg_sums[2 * (size_t)nseg + sg] = total;
     }
     __syncthreads();
     unsigned bad = 0;
-    for (int i = rank + size * (threadIdx.x >> 6); i < ntile; i += size * (BOUNDARY_THREADS / 64)) {
+    for (int i = threadIdx.x >> 6; i < ntile; i += BOUNDARY_THREADS / 64) {
         const SlotTile tile = slot_tile(b, s0, i);
         const int k = tile.first + (threadIdx.x & 63), mode = b.seg_mode[tile.sg];
         if (k >= tile.end) continue;
         double tr[3] = {0., 0., 0.}, fl[3] = {0., 0., 0.};
         if (!(mode == 4 || mode == 5 || mode == 9 || mode == 10 || mode == 11) &&
-            plain_face(m, b, k, tile.sg, q, z, dry, grav, ct.speed_limit,
+            plain_face(open_face(m, b, k, tile.sg, q, z), b.forcing[tile.sg], b.forcing[nseg + tile.sg],
+                       b.stage_policy[tile.sg], dry, grav, ct.speed_limit,
                        mode == 6 ? b.seg_sums[2 * (size_t)nseg + tile.sg] : 0., mode == 6 ? b.terms[2 * ns + k] : 0., tr, fl))
             bad = 1;
 #pragma unroll
         for (int r = 0; r < 3; ++r) { b.trace[r * ns + k] = tr[r]; b.flux[r * ns + k] = fl[r]; }
     }
-    team_sync();
-    if constexpr (!CLUSTER) if (b.sections) {
-        // section owners of the remaining outlet modes, after the face loop, in
+    __syncthreads();
+    if (b.sections) {
+    // section owners of the remaining outlet modes, after the face loop, in
         // the reference's order (river_exterior_bed.py:213-217): a normal-depth
         // chain without a root rejects the trial before the rating owner runs; a
         // rating section without a solution fails the scenario
@@ -1563,73 +1751,27 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
     if (bad) raise_status(ct, stage, ST_SPATIAL);
     // outlet stock cap, one thread per unique owner, its faces in boundary order
     const int u0 = b.scen_own[sid], u1 = b.scen_own[sid + 1];
-    const double rtrial = reciprocal(ct.trial);
-    for (int u = u0 + (int)threadIdx.x + BOUNDARY_THREADS * rank; u < u1; u += BOUNDARY_THREADS * size) {
-        const int c = b.own_cell[u];
-        double total = 0., reserved = 0.;
-        for (int j = b.own_off[u]; j < b.own_off[u + 1]; ++j) {
-            const int k = b.own_slot[j], f = b.slot_face[k];
-            const double flux = b.flux[k], debit = greater(flux, 0.) ? flux * m.length[f] : 0.;
-            if (is_outlet(b.seg_mode[m.bid[f]])) total += debit; else reserved += debit;
-        }
-        const double left = quotient(base[c] * m.area[c], ct.trial, rtrial) - reserved;
-        const double available = greater(left, 0.) ? left : 0.;
-        if (!greater(total, available)) continue;             // nothing to cap
-        const double factor = fmin(1., available / fmax(total, 1e-300)) * (1. - 32. * EPS);
-        for (int j = b.own_off[u]; j < b.own_off[u + 1]; ++j) {
-            const int k = b.own_slot[j], f = b.slot_face[k];
-            const double water = b.flux[k];
-            if (!is_outlet(b.seg_mode[m.bid[f]]) || !(water > 0.)) continue;
-            const double depth = b.trace[k], denom = fmax(depth, 1e-300);
-            const double ux = depth > 0. ? b.trace[ns + k] / denom : 0.;
-            const double uy = depth > 0. ? b.trace[2 * ns + k] / denom : 0.;
-            b.flux[ns + k] += (factor * factor - 1.) * water * ux;
-            b.flux[2 * ns + k] += (factor * factor - 1.) * water * uy;
-            b.flux[k] = water * factor;
-            b.trace[ns + k] *= factor;
-            b.trace[2 * ns + k] *= factor;
-        }
+    cap_owners(m, b, base, ct.trial, u0 + (int)threadIdx.x, u1, BOUNDARY_THREADS, false);
+    if (b.inlet) inlet_allocation(m, b, ct, base, s0, s1, u0, u1);
+    __syncthreads();
+    for (int i = warp; i < 2 * ntile; i += BOUNDARY_THREADS / 32) {
+        const SlotTile tile = slot_tile(b, s0, i >> 1);
+        const int first = tile.first + 32 * (i & 1), k = first + lane;
+        const double2 sum = warp_water(k < tile.end ? double(F(b.flux[k])) * m.length[b.slot_face[k]] : 0.);
+        if (lane == 0 && first < tile.end) b.water_sum[first] = sum;
     }
-    if (!CLUSTER && b.inlet) {
-        inlet_allocation(m, b, ct, base, s0, s1, u0, u1);
-        __syncthreads();
-    }
-    // The scenario's sum over its open faces of (outward water flux x length),
-    // with each face's water as the update consumes it (the mixed form carries
-    // it in FP32: F(flux)), and of its magnitude: 32 owners by a butterfly,
-    // then these partial sums in order. The controller turns the stage sums
-    // into the boundary ledger. An owner's faces are its own thread's above.
-    for (int first = u0 + 32 * (warp + rank * (BOUNDARY_THREADS / 32)); first < u1; first += BOUNDARY_THREADS * size) {
-        const int u = first + lane;
-        double acc = 0., gross = 0.;
-        if (u < u1)
-            for (int j = b.own_off[u]; j < b.own_off[u + 1]; ++j) {
-                const int k = b.own_slot[j];
-                const double v = double(F(b.flux[k])) * m.length[b.slot_face[k]];
-                acc += v;
-                gross += fabs(v);
-            }
-        for (int o = 16; o > 0; o >>= 1) {
-            acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            gross += __shfl_xor_sync(0xffffffffu, gross, o);
-        }
-        if (lane == 0) b.own_sum[first] = make_double2(acc, gross);
-    }
-    team_sync();
-    if (rank == 0 && threadIdx.x < 2) {
-        double total = 0.;
-        for (int first = u0; first < u1; first += 32) total += threadIdx.x ? b.own_sum[first].y : b.own_sum[first].x;
-        if (threadIdx.x) ct.bgross[stage - 1] = total; else ct.bflux[stage - 1] = total;
-    }
+    __syncthreads();
+    scenario_water(b, ct, stage, s0, ntile);
 }
 
-// Launch over nscen scenarios, b.cluster blocks each.
+// Launch over nscen scenarios: b.cluster blocks each where every scenario fits
+// a thread per face, else (b.cluster = 0) one block.
 template <class F>
 inline void launch_boundary(const MeshDev &m, const StateDev &s, const BoundaryDev &b, Ctrl *ctrl, int nscen, int stage,
                             cudaStream_t st)
 {
-    if (b.cluster <= 1) {
-        k_boundary<F, false><<<nscen, BOUNDARY_THREADS, 0, st>>>(m, s, b, ctrl, stage);
+    if (b.cluster == 0) {
+        k_boundary<F><<<nscen, BOUNDARY_THREADS, 0, st>>>(m, s, b, ctrl, stage);
         return;
     }
     cudaLaunchAttribute attr{};
@@ -1638,7 +1780,7 @@ inline void launch_boundary(const MeshDev &m, const StateDev &s, const BoundaryD
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(nscen * b.cluster); cfg.blockDim = dim3(BOUNDARY_THREADS); cfg.stream = st;
     cfg.attrs = &attr; cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, k_boundary<F, true>, m, s, b, ctrl, stage);
+    cudaLaunchKernelEx(&cfg, k_boundary_plain<F>, m, s, b, ctrl, stage);
 }
 
 // ---------------------------------------------------------------------------
