@@ -982,10 +982,16 @@ extern "C" int brx_turbines_set(brx_solver *s, int nrotor, const int *rotor_scen
         CK(cudaMemset(s->mx.hgrad, 0, sizeof(float) * 6 * (size_t)nc));
         CK(cudaMemset(s->mx.hp, 0, sizeof(float2) * nf)); CK(cudaMemset(s->mx.hs, 0, sizeof(float2) * nf));
     } else {
-        TRY(s->alloc(&t.grad, 8 * (size_t)nc)); TRY(s->alloc(&t.trace, 10 * (size_t)nf));
+        TRY(s->alloc(&t.grad, 6 * (size_t)nc));
         TRY(s->alloc(&t.pface, 2 * (size_t)nf)); TRY(s->alloc(&t.sface, 2 * (size_t)nf));
-        CK(cudaMemset(t.grad, 0, sizeof(double) * 8 * (size_t)nc));
-        CK(cudaMemset(t.trace, 0, sizeof(double) * 10 * (size_t)nf));
+        CK(cudaMemset(t.grad, 0, sizeof(double) * 6 * (size_t)nc));
+        double *p_wd;
+        TRY(s->alloc(&p_wd, 2 * (size_t)nadj));
+        // on the default stream, which follows the uploads
+        k_flow_weights<<<std::max(1, std::min((nadj + 255) / 256, s->sms * 32)), 256>>>(nadj, t.dxdy, p_wd);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(nullptr));
+        t.wdxdy = p_wd;
         CK(cudaMemset(t.pface, 0, sizeof(double) * 2 * (size_t)nf));
         CK(cudaMemset(t.sface, 0, sizeof(double) * 2 * (size_t)nf));
     }
@@ -1132,11 +1138,11 @@ static int max_block(const brx_solver *s, int kind)
         fn = s->maxdeg <= 3 ? (const void *)k64_cells<3> : small ? (const void *)k64_cells<4>
                             : (const void *)k_cells<double, MAX_CELL_FACES>;
         break;
-    case K_FACES: fn = (const void *)k64_faces; break;
+    case K_FACES: fn = s->has_turb ? (const void *)k64_faces<true> : (const void *)k64_faces<false>; break;
     case K_LIMIT: fn = (const void *)k_limit; break;
     case K_UPDATE: fn = (const void *)k64_update; break;
     case K_HKT_GRAD: fn = (const void *)k_hkt_gradients; break;
-    case K_HKT_FACES: fn = (const void *)k_hkt_faces; break;
+    case K_HKT_FACES: fn = (const void *)k_hkt_stress; break;
     case KH_CELLS_SHAPE:
         fn = small ? (const void *)k_hllc_cells<4> : (const void *)k_hllc_cells<MAX_CELL_FACES>;
         break;
@@ -1527,40 +1533,34 @@ static inline int sgrid(const brx_solver *s, int kind, int n)
 }
 #define SSHAPE(kind_, n_) sgrid(s, kind_, n_), s->shape[kind_].block
 
-// part: 1 the cell terms (wet gradients, rotor sample, actuator sink), which
-// need only the stage state; 2 the face terms (balanced pressure, ambient
-// stress), which also need the face sweep's traces; 3 both, in order.
-enum { TURB_CELLS = 1, TURB_FACES = 2, TURB_ALL = 3 };
-static int launch_turbines(brx_solver *s, int stage, cudaStream_t st, int part = TURB_ALL)
+// The cell terms (wet gradients, rotor sample, actuator sink), which need only
+// the stage state. The f-wave face sweeps of both forms add the face terms
+// (balanced pressure, ambient stress) in their tails; the HLLC owner, which has
+// no balanced pressure, forms its ambient stress here.
+static int launch_turbines(brx_solver *s, int stage, cudaStream_t st)
 {
     if (!s->has_turb) return 0;
     const double *q = stage == 1 ? s->state.work : s->state.q1;
     const TurbDev &t = s->turb;
     const bool mixed = s->precision == BRX_MIXED;
-    // the wet gradients feed only the face terms (balanced pressure, ambient
-    // stress); the HLLC owner without ambient stress has neither
-    const bool faces = t.balanced || s->any_stress;
     int n = 0;
-    if (part & TURB_CELLS) {
-        if (mixed) n += mixed_kernel(make_launch(s, st), K_HKT_GRAD, stage, nullptr);
-        else if (faces) {
-            k_hkt_gradients<<<SSHAPE(K_HKT_GRAD, s->nc), 0, st>>>(s->mesh, t, q, s->state.z, s->d_ctrl, stage);
-            ++n;
-        }
-        k_turbine_sample<<<t.nr, TURB_THREADS, 0, st>>>(s->mesh, t, q, s->state.z, s->d_ctrl, stage, t.diag);
+    // the mixed cell sweep forms the wet gradients in its tail; the HLLC owner
+    // without ambient stress uses none
+    if (!mixed && (t.balanced || s->any_stress)) {
+        const Prim64 *prim = s->small64 && s->method == BRX_METHOD_FWAVE ? s->c64.prim[stage - 1] : nullptr;
+        k_hkt_gradients<<<SSHAPE(K_HKT_GRAD, s->nc), 0, st>>>(s->mesh, t, q, s->state.z, s->d_ctrl, stage, prim);
         ++n;
-        if (t.nucell > 0) {            // cells shared by overlapping supports
-            k_turbine_raw<<<std::max(1, std::min((t.nucell + 255) / 256, s->sms * 8)), 256, 0, st>>>(s->mesh, t, q,
-                                                                                                   s->d_ctrl, stage);
-            ++n;
-        }
     }
-    if (part & TURB_FACES) {
-        if (mixed) n += mixed_kernel(make_launch(s, st), K_HKT_FACES, stage, nullptr);
-        else if (faces) {
-            k_hkt_faces<<<SSHAPE(K_HKT_FACES, s->nf), 0, st>>>(s->mesh, t, q, s->state.z, s->d_ctrl, stage);
-            ++n;
-        }
+    k_turbine_sample<<<t.nr, TURB_THREADS, 0, st>>>(s->mesh, t, q, s->state.z, s->d_ctrl, stage, t.diag);
+    ++n;
+    if (t.nucell > 0) {            // cells shared by overlapping supports
+        k_turbine_raw<<<std::max(1, std::min((t.nucell + 255) / 256, s->sms * 8)), 256, 0, st>>>(s->mesh, t, q,
+                                                                                               s->d_ctrl, stage);
+        ++n;
+    }
+    if (!mixed && s->method == BRX_METHOD_HLLC && s->any_stress) {
+        k_hkt_stress<<<SSHAPE(K_HKT_FACES, s->nf), 0, st>>>(s->mesh, t, q, s->state.z, s->d_ctrl, stage);
+        ++n;
     }
     return n;
 }
@@ -1594,8 +1594,10 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
         else k_cells<double, MAX_CELL_FACES><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
         return 1;
     case K_FACES:
-        k64_faces<<<SSHAPE(K_FACES, s->nf), 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, s->work, stage,
-                                                    s->has_turb ? s->turb.trace : nullptr, s->turb.hkt);
+        if (s->has_turb)
+            k64_faces<true><<<SSHAPE(K_FACES, s->nf), 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, s->work, stage, s->turb);
+        else
+            k64_faces<false><<<SSHAPE(K_FACES, s->nf), 0, st>>>(s->mesh, s->state, s->bnd, s->d_ctrl, s->work, stage, s->turb);
         return 1;
     case K_LIMIT:
         k_limit<<<SSHAPE(K_LIMIT, s->nf), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
@@ -1630,7 +1632,7 @@ static void enqueue_stage(brx_solver *s, int stage, double *rate_out)
         s->launches += launch_kernel(s, K_BOUNDARY, stage, nullptr, s->side);
         cudaEventRecord(s->join, s->side);
         cudaStreamWaitEvent(s->side2, s->fork, 0);
-        s->launches += launch_turbines(s, stage, s->side2, TURB_CELLS);
+        s->launches += launch_turbines(s, stage, s->side2);
         cudaEventRecord(s->join2, s->side2);
     }
     const bool mixed = s->precision == BRX_MIXED;
@@ -1645,14 +1647,12 @@ static void enqueue_stage(brx_solver *s, int stage, double *rate_out)
     } else {
         s->launches += launch_kernel(s, K_CELLS, stage, nullptr);
         if (fork) cudaStreamWaitEvent(s->stream, s->join, 0);
-        // the mixed face sweep computes the rotor face terms in its tail: it
-        // needs the rotor cell terms (wet gradients, actuator sink) first
-        if (fork && mixed) cudaStreamWaitEvent(s->stream, s->join2, 0);
+        // the face sweep computes the rotor face terms in its tail: it needs
+        // the rotor cell terms (wet gradients, actuator sink) first
+        if (fork) cudaStreamWaitEvent(s->stream, s->join2, 0);
         // gather and donor limiter are part of the update
         s->launches += launch_kernel(s, K_FACES, stage, nullptr);
-        if (fork && !mixed) cudaStreamWaitEvent(s->stream, s->join2, 0);
     }
-    s->launches += launch_turbines(s, stage, s->stream, TURB_FACES);
     s->launches += launch_kernel(s, K_VISC, stage, nullptr);
     s->launches += launch_kernel(s, K_UPDATE, stage, rate_out);
 }
@@ -1682,7 +1682,7 @@ static int launch_hllc(brx_solver *s, int kind, cudaStream_t st = nullptr)
         return s->has_turb ? launch_turbines(s, 1, st) : 0;
     case KH_PREDICT:
         if (!s->has_turb) return 0;
-        k_hllc_predict<<<SSHAPE(KH_PREDICT_SHAPE, s->nc), 0, st>>>(s->mesh, s->state, s->turb, rec, s->d_ctrl);
+        k_hllc_predict<<<SSHAPE(KH_PREDICT_SHAPE, s->nc), 0, st>>>(s->mesh, s->state, s->turb, rec, s->d_ctrl, s->work.rarea);
         return 1;
     case KH_BOUNDARY:
         if (!s->nslot) return 0;
@@ -2120,12 +2120,12 @@ extern "C" int brx_profile_substep(brx_solver *s, double dt, double time, int ca
         for (int kind : HLLC_SEQUENCE)
             if (const int nl = launch_hllc(s, kind)) { mark(kind); extra += nl - 1; }
     } else {
-        // the mixed face sweep reads the rotor cell terms: they come first there
+        // the face sweep reads the rotor cell terms: they come first
         const bool mixed = s->precision == BRX_MIXED, tiled = mixed && s->tile_cells > 0;
         for (int stage = 1; stage <= 2; ++stage)
-            for (int kind : {(int)K_BOUNDARY, mixed ? (int)K_TURB : -1, tiled ? (int)K_TILE : (int)K_CELLS,
+            for (int kind : {(int)K_BOUNDARY, (int)K_TURB, tiled ? (int)K_TILE : (int)K_CELLS,
                              tiled ? -1 : (int)K_FACES,
-                             mixed ? -1 : (int)K_TURB, (int)K_VISC, (int)K_UPDATE})
+                             (int)K_VISC, (int)K_UPDATE})
                 if (kind >= 0)
                     if (const int nl = launch_kernel(s, kind, stage, nullptr)) { mark(kind); extra += nl - 1; }
     }
@@ -2414,7 +2414,7 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     const int n = nc > nf ? nc : nf;
     k_noalloc_tables<<<(n + 255) / 256, 256, 0, st>>>(m, ctrl, cell_sid, cflags, face_sid, bslot, bmode, disp_unit);
     k_cells<double, MAX_CELL_FACES><<<(nc + 127) / 128, 128, 0, st>>>(m, sd, ctrl, w, 1);
-    k64_faces<<<(nf + 127) / 128, 128, 0, st>>>(m, sd, b, ctrl, w, 1, nullptr, nullptr);
+    k64_faces<false><<<(nf + 127) / 128, 128, 0, st>>>(m, sd, b, ctrl, w, 1, TurbDev{});
     k64_update<<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);
     k_limited<<<(nc + 63) / 64, 64, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);
     k_limit<<<(nf + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1);

@@ -167,10 +167,10 @@ struct TurbDev {
     const unsigned char *single;                    // (ns) 1: the entry's cell is in no other support entry
     const unsigned char *foot;                      // (nc) 1: a support cell (its actuator sink may be nonzero)
     const double *dxdy, *inverse, *xy, *mdisp, *nu; // (2,nadj) (3,nc) (2,nc) (4,nf) (nc)
-    double *grad;               // (8, nc) wet gradients: u, v, eta, b (x, y)
+    const double *wdxdy;        // (2, nadj) dxdy over its squared length: (1 / |d|^2) dx, (1 / |d|^2) dy (FP64 form)
+    double *grad;               // (6, nc) wet gradients: u, v, eta (x, y)
     double *kcell;              // (ns) sink coefficient
     double *raw;                // (2, nc) actuator momentum sink
-    double *trace;              // (10, nf) hydrostatically reconstructed face traces
     double *pface, *sface;      // (2, nf) pressure correction, ambient stress
     double *diag;               // (nr, 16) rotor diagnostics of the last sampled state
     int balanced;               // 1: balanced-pressure face term (f-wave owner); 0: HLLC owner
@@ -310,50 +310,6 @@ __device__ __forceinline__ bool skip_stage(const Ctrl &c, int stage)
 __device__ __forceinline__ void raise_status(Ctrl &c, int stage, unsigned bits)
 {
     atomicOr(stage == 1 ? &c.status1 : &c.status2, bits);
-}
-
-// Face traces of the hydrostatically reconstructed states for the rotor
-// pressure correction (river_turbine_flow.h:39-52): surfaces, normal
-// velocities and speeds of both sides, the common bed, constant flags.
-__device__ __forceinline__ void put_trace(double *tr, int nf, int f, const double loc[8], bool cl, bool cr)
-{
-    const double hl = loc[0], hr = loc[4];
-    tr[f] = hl + loc[3]; tr[nf + f] = hr + loc[7];
-    tr[2 * nf + f] = hl > 0. ? loc[1] / hl : 0.; tr[3 * nf + f] = hr > 0. ? loc[5] / hr : 0.;
-    tr[4 * nf + f] = hl > 0. ? hypot(loc[1], loc[2]) / hl : 0.;
-    tr[5 * nf + f] = hr > 0. ? hypot(loc[5], loc[6]) / hr : 0.;
-    tr[6 * nf + f] = loc[3]; tr[7 * nf + f] = loc[7];
-    tr[8 * nf + f] = cl ? 1. : 0.; tr[9 * nf + f] = cr ? 1. : 0.;
-}
-
-// Momentum terms of a rotor array, in the reference's add_momentum order
-// (river_turbine_flow.py:230-239): ambient stress, actuator sink, balanced
-// pressure; face terms gathered as sum(s len flux) / area
-// (flow2dh_fixed_bed_kernels.h:54-60 with unit depth weights). The HLLC
-// owner's rotor hook has no balanced pressure (river_turbines.py:27-36):
-// balanced = false.
-__device__ __forceinline__ void add_rotor_momentum(const MeshDev &m, const TurbDev &t, int sid, int c, double area,
-                                                   double &r1, double &r2, bool balanced = true)
-{
-    const int nc = m.nc, nf = m.nf;
-    if (t.stress[sid]) {
-        double x = 0., y = 0.;
-        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
-            const int f = m.faces[k];
-            x += m.signs[k] * m.length[f] * t.sface[f];
-            y += m.signs[k] * m.length[f] * t.sface[nf + f];
-        }
-        r1 += 1. * x / area; r2 += 1. * y / area;
-    }
-    r1 += t.raw[c]; r2 += t.raw[nc + c];
-    if (!balanced) return;
-    double x = 0., y = 0.;
-    for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
-        const int f = m.faces[k];
-        x += m.signs[k] * m.length[f] * t.pface[f];
-        y += m.signs[k] * m.length[f] * t.pface[nf + f];
-    }
-    r1 += 1. * x / area; r2 += 1. * y / area;
 }
 
 constexpr int BOUNDARY_TILES = 1024;   // tile slots of 64 faces per scenario (checked at set-up)

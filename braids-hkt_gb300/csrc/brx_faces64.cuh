@@ -20,6 +20,7 @@
 // whole sequence.
 #pragma once
 #include "brx_num64.cuh"
+#include "brx_turbine.cuh"
 
 namespace brx {
 
@@ -194,8 +195,12 @@ __device__ __noinline__ bool dry_face64(const double *loc, double hc, double zc,
 
 // Four resident blocks of 128 threads (at most 128 registers): a single
 // 75k-face scenario then fits the 152 SMs in one wave of 16 warps each.
+// ROTOR: a solver with rotors, whose face terms (balanced pressure, ambient
+// stress) are formed here from the traces in registers; they need the stage's
+// wet gradients and actuator sink first.
+template <bool ROTOR>
 __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, Work w, int stage,
-                                                    double *trace, const int *hkt)
+                                                    TurbDev t)
 {
     const int nf = m.nf, nc = m.nc;
     FOR_ACTIVE_FACES(m.act, f) {
@@ -220,36 +225,35 @@ __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, Bound
             w.gf[f] = make_double4_32a(fl1 - pc * nx, fl2 - pc * ny, 0., 0.);
             continue;
         }
-        CellRec rn;
-        if (n >= 0) rn = w.rec[n];
-        const bool wetc = greater(rc.h, dry), wetn = n >= 0 && greater(rn.h, dry);
-        const int kind = !wetc && !wetn ? 0 : n >= 0 ? 1 : 2;
+        // a wall reads its owner on both sides: interior and wall faces then go
+        // one way through the solve (a branch here splits the warp to the end)
+        const bool inner = n >= 0;
+        const CellRec rn = w.rec[inner ? n : c];
+        const bool wetc = greater(rc.h, dry), wetn = greater(rn.h, dry);
+        const bool idle = !wetc && !wetn;
         unsigned bad = 0;
-        const Side64 L = trace64(rc, m.disp[f], m.disp[2 * nf + f], dry, kind == 0, bad);
-        Side64 R = {0., 0., 0., 0., 0.};
-        if (n >= 0) R = trace64(rn, m.disp[nf + f], m.disp[3 * nf + f], dry, kind == 0, bad);
+        const Side64 L = trace64(rc, m.disp[f], m.disp[2 * nf + f], dry, idle, bad);
+        const int other = inner ? nf : 0;
+        const Side64 R = trace64(rn, m.disp[other + f], m.disp[2 * nf + other + f], dry, idle, bad);
         double water = 0., speed = 0., l1 = 0., l2 = 0., r1 = 0., r2 = 0.;
-        const bool rotor = trace && n >= 0 && hkt[m.face_sid[f]];
-        if (kind != 0) {
+        const bool rotor = ROTOR && inner && t.hkt[m.face_sid[f]];
+        double pressure = 0.;          // the rotors' balanced pressure along the normal
+        if (!idle) {
             // rotation to the face frame; a wall mirrors the state
             const double unL = L.hu * nx + L.hv * ny, utL = L.hu * (-ny) + L.hv * nx;
-            double hR = R.h, bR = R.b, xR = R.hu, yR = R.hv;
-            const double rawR = kind == 2 ? L.raw : R.raw;
-            if (kind == 2) { hR = L.h; bR = L.b; xR = L.hu - 2.0 * unL * nx; yR = L.hv - 2.0 * unL * ny; }
+            const double twice = inner ? 0. : 2.0 * unL;
+            const double xR = R.hu - twice * nx, yR = R.hv - twice * ny;
             const double unR = xR * nx + yR * ny, utR = xR * (-ny) + yR * nx;
-            const double hL = L.h, bL = L.b;
-            double loc[8] = {hL, unL, utL, bL, hR, unR, utR, bR};
-            if (kind == 1) {
-                const double top = greater(bL, bR) ? bL : bR, eL = hL + bL, eR = hR + bR;
-                const long long big = max(__double_as_longlong(dry), max(magnitude(top), max(magnitude(eL), magnitude(eR))));
-                const double thin = dry + 16. * EPS * __longlong_as_double(big);
-                double hl = eL - top, hr = eR - top;
-                if (!greater(hl, thin)) hl = 0.;
-                if (!greater(hr, thin)) hr = 0.;
-                loc[0] = hl; loc[3] = top; loc[4] = hr; loc[7] = top;
-                const double kl = greater(hL, dry) ? hl / hL : 0., kr = greater(hR, dry) ? hr / hR : 0.;
-                loc[1] = unL * kl; loc[2] = utL * kl; loc[5] = unR * kr; loc[6] = utR * kr;
-            }
+            const double hL = L.h, bL = L.b, hR = R.h, bR = R.b;
+            const double top = greater(bL, bR) ? bL : bR, eL = hL + bL, eR = hR + bR;
+            const long long big = max(__double_as_longlong(dry), max(magnitude(top), max(magnitude(eL), magnitude(eR))));
+            const double thin = dry + 16. * EPS * __longlong_as_double(big);
+            double hl = eL - top, hr = eR - top;
+            if (!greater(hl, thin)) hl = 0.;
+            if (!greater(hr, thin)) hr = 0.;
+            const double kl = greater(hL, dry) ? hl / hL : 0., kr = greater(hR, dry) ? hr / hR : 0.;
+            const double loc[8] = {inner ? hl : hL, inner ? unL * kl : unL, inner ? utL * kl : utL, inner ? top : bL,
+                                   inner ? hr : hR, inner ? unR * kr : unR, inner ? utR * kr : utR, inner ? top : bR};
             Solve64 o;
             bool closed = false;
             const bool wet = greater(loc[0], dry) && greater(loc[4], dry);
@@ -261,22 +265,16 @@ __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, Bound
                 for (int j = 0; j < 8; ++j) in[j] = loc[j];
                 Solve64 d;
                 bool shut;
-                if (dry_face64(in, rc.h, rc.b, n >= 0 ? rn.h : 0., n >= 0 ? rn.b : 0., kind, hL, bL, unL, hR, bR, unR,
+                if (dry_face64(in, rc.h, rc.b, rn.h, rn.b, inner ? 1 : 2, hL, bL, unL, hR, bR, unR,
                                m.distance[f], m.distance[nf + f], dry, grav, shut, d)) bad = 1;
                 o = d;
                 closed = shut;
             }
-            if (rotor) {
-                double *tr = trace;
-                tr[f] = loc[0] + loc[3]; tr[nf + f] = loc[4] + loc[7];
-                const bool vl = greater(loc[0], 0.), vr = greater(loc[4], 0.);
-                tr[2 * nf + f] = vl ? (wet ? o.ul : loc[1] / loc[0]) : 0.;
-                tr[3 * nf + f] = vr ? (wet ? o.ur : loc[5] / loc[4]) : 0.;
-                tr[4 * nf + f] = vl ? hypot(loc[1], loc[2]) / loc[0] : 0.;
-                tr[5 * nf + f] = vr ? hypot(loc[5], loc[6]) / loc[4] : 0.;
-                tr[6 * nf + f] = loc[3]; tr[7 * nf + f] = loc[7];
-                tr[8 * nf + f] = rc.flags & 1 ? 1. : 0.; tr[9 * nf + f] = rn.flags & 1 ? 1. : 0.;
-            }
+            if constexpr (ROTOR)
+                if (rotor && wet && wetc && wetn)
+                    pressure = balanced_pressure(m, t, f, c, n, rc, rn,
+                                                 FaceTrace{loc[0], loc[4], loc[3], o.ul, o.ur, loc[1], loc[2], loc[5], loc[6]},
+                                                 grav, dry, nx, ny);
             speed = o.speed;
             if (closed) {
                 const double p = hg * (hL * hL), q = hg * (hR * hR);
@@ -285,7 +283,7 @@ __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, Bound
                 // left / right mass fluxes agree to the solve's precision
                 const long long top = max(0x3ff0000000000000LL, max(magnitude(o.l[0]), magnitude(o.r[0])));
                 if (magnitude(o.l[0] - o.r[0]) > __double_as_longlong(1.e-10 * __longlong_as_double(top))) bad = 1;
-                if (kind == 2) {
+                if (!inner) {
                     const double pressure = wall_pressure<double>(hL, loc[1], grav, dry);
                     l1 = pressure * nx; l2 = pressure * ny;
                 } else {
@@ -300,20 +298,26 @@ __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, Bound
                 const double corr = (rc.flags & 1) ? hg * (rc.h * rc.h - hL * hL) : hg * (rc.h + L.raw) * (bL - rc.b);
                 l1 += corr * nx; l2 += corr * ny;
             }
-            if (n >= 0) {
+            if (inner) {
                 if (wetn) {
-                    const double corr = (rn.flags & 1) ? hg * (rn.h * rn.h - hR * hR) : hg * (rn.h + rawR) * (bR - rn.b);
+                    const double corr = (rn.flags & 1) ? hg * (rn.h * rn.h - hR * hR) : hg * (rn.h + R.raw) * (bR - rn.b);
                     r1 += corr * nx; r2 += corr * ny;
                 }
             } else { r1 = l1; r2 = l2; }
             if (!finite_bits(water) || !finite_bits(l1) || !finite_bits(l2) || !finite_bits(r1) || !finite_bits(r2)) bad = 1;
-        } else if (rotor) {
-            const double zero[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
-            put_trace(trace, nf, f, zero, rc.flags & 1, rn.flags & 1);
         }
+        if constexpr (ROTOR)
+            if (rotor) {
+                t.pface[f] = pressure * nx; t.pface[nf + f] = pressure * ny;
+                if (t.stress[m.face_sid[f]]) {
+                    double ox = 0., oy = 0.;
+                    if (wetc && wetn) rotor_stress(m, t, stage == 1 ? s.work : s.q1, s.z, f, c, n, nx, ny, ox, oy);
+                    t.sface[f] = ox; t.sface[nf + f] = oy;
+                }
+            }
         if (bad) raise_status(ct, stage, ST_SPATIAL);
         w.ws[f] = make_double2(water, speed);
-        if (n >= 0) {
+        if (inner) {
             const double pn = hg * rn.h * rn.h;
             w.gf[f] = make_double4_32a(l1 - pc * nx, l2 - pc * ny, r1 - pn * nx, r2 - pn * ny);
         } else w.gf[f] = make_double4_32a(l1 - pc * nx, l2 - pc * ny, r1, r2);

@@ -169,7 +169,8 @@ __global__ void __launch_bounds__(128) k_hllc_cells(MeshDev m, StateDev s, HllcD
 // Half-step rotor source on the predicted state of scenarios with rotors
 // (hllc.h:74-77); the rate is the HLLC owner's rotor momentum at the start
 // state (ambient stress, actuator sink).
-__global__ void __launch_bounds__(256) k_hllc_predict(MeshDev m, StateDev s, TurbDev t, HCell *rec, Ctrl *ctrl)
+__global__ void __launch_bounds__(256) k_hllc_predict(MeshDev m, StateDev s, TurbDev t, HCell *rec, Ctrl *ctrl,
+                                                      const double *rarea)
 {
     const int nc = m.nc;
     FOR_ACTIVE_CELLS(m.act, c) {
@@ -178,7 +179,7 @@ __global__ void __launch_bounds__(256) k_hllc_predict(MeshDev m, StateDev s, Tur
         const Ctrl &ct = ctrl[sid];
         if (!ct.active || ct.done) continue;
         double r1 = 0., r2 = 0.;
-        add_rotor_momentum(m, t, sid, c, m.area[c], r1, r2, false);
+        add_rotor_momentum(m, t, sid, c, m.area[c], r1, r2, false, rarea[c]);
         const double hh = s.q1[c];
         const double mu = s.q1[nc + c] + .5 * ct.trial * r1, mv = s.q1[2 * nc + c] + .5 * ct.trial * r2;
         s.q1[nc + c] = mu; s.q1[2 * nc + c] = mv;
@@ -363,7 +364,7 @@ __global__ void __launch_bounds__(256) k_hllc_update(MeshDev m, StateDev s, Hllc
         bad = bad || !isfinite(v0) || !isfinite(v1) || !isfinite(v2) || v0 < 0.;
         if (turb && t.hkt[sid]) {
             double r1 = 0., r2 = 0.;
-            add_rotor_momentum(m, t, sid, c, area, r1, r2, false);
+            add_rotor_momentum(m, t, sid, c, area, r1, r2, false, w.rarea[c]);
             v1 += dt * r1; v2 += dt * r2;
             bad = bad || !isfinite(v1) || !isfinite(v2);
         }

@@ -1572,10 +1572,6 @@ int mixed_kernel(const Launch &L, int kind, int stage, double *out)
     case K_WATER:
         brx_mx::km_water_out<<<L.grid_f256, 256, 0, st>>>(L.mesh, L.work, out);
         return 1;
-    case K_HKT_GRAD:        // fused into the cell sweep's tail
-        return 0;
-    case K_HKT_FACES:       // fused into the face sweep's tail
-        return 0;
     }
 #undef SHAPE
     return 0;

@@ -79,4 +79,34 @@ __device__ __forceinline__ void put_prim64(Prim64 *P, int c, double h, double hu
     P[c] = p;
 }
 
+// Momentum terms of a rotor array, in the reference's add_momentum order
+// (river_turbine_flow.py:230-239): ambient stress, actuator sink, balanced
+// pressure; face terms gathered as sum(s len flux) / area
+// (flow2dh_fixed_bed_kernels.h:54-60 with unit depth weights). The HLLC
+// owner's rotor hook has no balanced pressure (river_turbines.py:27-36):
+// balanced = false. rarea = RN(1 / area).
+__device__ __forceinline__ void add_rotor_momentum(const MeshDev &m, const TurbDev &t, int sid, int c, double area,
+                                                   double &r1, double &r2, bool balanced, double rarea)
+{
+    const int nc = m.nc, nf = m.nf;
+    if (t.stress[sid]) {
+        double x = 0., y = 0.;
+        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+            const int f = m.faces[k];
+            x += m.signs[k] * m.length[f] * t.sface[f];
+            y += m.signs[k] * m.length[f] * t.sface[nf + f];
+        }
+        r1 += quotient(x, area, rarea); r2 += quotient(y, area, rarea);
+    }
+    r1 += t.raw[c]; r2 += t.raw[nc + c];
+    if (!balanced) return;
+    double x = 0., y = 0.;
+    for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+        const int f = m.faces[k];
+        x += m.signs[k] * m.length[f] * t.pface[f];
+        y += m.signs[k] * m.length[f] * t.pface[nf + f];
+    }
+    r1 += quotient(x, area, rarea); r2 += quotient(y, area, rarea);
+}
+
 }  // namespace brx

@@ -48,7 +48,7 @@ __device__ __forceinline__ void finish_cell(const MeshDev &m, const StateDev &s,
                                             const TurbDev &t, int turb, Prim64 *prim, bool quiet)
 {
     const int nc = m.nc;
-    if (turb && t.hkt[sid]) add_rotor_momentum(m, t, sid, c, m.area[c], r1, r2);
+    if (turb && t.hkt[sid]) add_rotor_momentum(m, t, sid, c, m.area[c], r1, r2, true, w.rarea[c]);
     if (w.visc.nu && w.visc.nu[sid] > 0.) add_viscosity(m, w.visc, c, m.area[c], r1, r2);
     if (!finite_bits(r0) || !finite_bits(r1) || !finite_bits(r2)) raise_status(ct, stage, ST_RATE);
     if (rate_out) { rate_out[c] = r0; rate_out[nc + c] = r1; rate_out[2 * nc + c] = r2; return; }
