@@ -12,12 +12,16 @@
 //     reduce to one to five products;
 //   * the quotients by one depth share its reciprocal (quotient()), as do the
 //     three wave strengths, whose divisor is lam0 - lam2;
-//   * the middle state's square roots of g h are those of the wave speeds, the
-//     first trial depth of a mixed wave pattern gives the function value
-//     already known, and of a double shock's two terms one is zero.
-// About 400 FP64 instructions per wet face instead of 970. A face with a dry
-// side takes the general solver (dry_face64), which keeps the reference's
-// whole sequence.
+//   * the middle state's characteristics matter only to a flow near critical;
+//     bounds on its three wave patterns leave it out elsewhere, and with it the
+//     branch in which a warp ran all three. Where it is formed, its square
+//     roots of g h are those of the wave speeds, the first trial depth of a
+//     mixed pattern gives the function value already known, and of a double
+//     shock's two terms one is zero.
+// About 300 FP64 instructions per wet face instead of 970. Per launch, before
+// -> after: 302k cells 831 -> 306 us, 50k 158 -> 70 us, 360 cells 53 -> 29 us.
+// A face with a dry side takes the general solver (dry_face64), which keeps the
+// reference's whole sequence.
 #pragma once
 #include "brx_num64.cuh"
 #include "brx_turbine.cuh"
@@ -61,55 +65,73 @@ __device__ __forceinline__ bool wet_face64(double hL, double huL, double hvL, do
     bool bad = !(finite_bits(hL) && finite_bits(huL) && finite_bits(hvL) && finite_bits(hR) && finite_bits(huR) &&
                  finite_bits(hvR));
     const double hg = .5 * g;
-    const double rL = 1. / hL, rR = 1. / hR;
+    const double rL = reciprocal(hL), rR = reciprocal(hR);
     const double uL = quotient(huL, hL, rL), vL = quotient(hvL, hL, rL);
     const double uR = quotient(huR, hR, rR), vR = quotient(hvR, hR, rR);
     const double phiL = hg * (hL * hL) + quotient(huL * huL, hL, rL);
     const double phiR = hg * (hR * hR) + quotient(huR * huR, hR, rR);
-    const double sqL = sqrt(g * hL), sqR = sqrt(g * hR);
+    const double sqL = sqrt(g * hL), sqR = sqrt(g * hR), sq = sqR + sqL;
     const double mean = hg * (hR + hL);
-    const double uhat = (sqL * uL + sqR * uR) / (sqR + sqL), chat = sqrt(mean);
+    const double uhat = quotient(sqL * uL + sqR * uR, sq, reciprocal(sq)), chat = sqrt(mean);
     const double e1 = uhat - chat, e2 = uhat + chat, sL = uL - sqL, sR = uR + sqR;
-    // middle state (riemann_type, brx_fwave.cuh)
+    double lam0 = greater(sL, e1) ? e1 : sL, lam2 = greater(e2, sR) ? e2 : sR;
+    // The speeds are lam0 = min(lam0, s2m) and lam2 = max(lam2, s1m) with the
+    // middle state's characteristics s1m = u - c, s2m = u + c (riemann_type,
+    // brx_fwave.cuh). Only a flow near critical reaches s2m below lam0 or s1m
+    // above lam2; bounds on the three wave patterns rule that out in a dozen
+    // instructions, by a margin far above their rounding:
+    //   two rarefactions: the middle celerity is root / 4;
+    //   two shocks: the middle depth is at least the deeper side's;
+    //   a shock and a rarefaction: it lies between the two sides'.
     const bool right = __double_as_longlong(hR) >= __double_as_longlong(hL);       // R is the deeper side
-    const double hmin = right ? hL : hR, hmax = right ? hR : hL;
     const double sqmin = right ? sqL : sqR, sqmax = right ? sqR : sqL;
     const double delu = uR - uL;
     const double fmn = delu + 2. * (sqmin - sqmax);
-    const double aL = uL + 2. * sqL, aR = uR - 2. * sqR;
-    double s1m, s2m;
+    const double aL = uL + 2. * sqL, aR = uR - 2. * sqR, slack = 1.e-6 * sq;
+    const double up = lam0 + slack, down = lam2 - slack;
+    bool clear;
     if (greater(fmn, 0.)) {
-        const double root0 = -delu + 2. * (sqL + sqR), root = __double_as_longlong(root0) < 0 ? 0. : root0;
-        const double c = sqrt(g * (g16r * (root * root)));
-        s1m = aL - 3. * c;
-        s2m = aR + 3. * c;
+        const double root = 2. * sq - delu, q = .75 * root;
+        clear = __double_as_longlong(root) > 0 && greater(aR + q, up) && greater(down, aL - q);
     } else {
-        const double fmx = delu + (hmax - hmin) * sqrt(mean / (hmax * hmin));
-        if (!greater(fmx, 0.)) {
-            const double rmax = right ? rR : rL, rmin = right ? rL : rR;
-            const double gM = sqrt(hg * (rmax + rmax)), gm = sqrt(hg * (rmax + rmin)), gap = hmax - hmin;
-            const double F0 = delu + gap * gm;
-            const double q = (g * gap) / (4. * (hmax * hmax) * gm);
-            // ((gL - qL) + gR) - qR with the deeper side's q zero
-            const double dfdh = right ? (gm - q) + gM : (gM + gm) - q;
-            const double h0 = sqrt(hmax), root = h0 - F0 / (2. * h0 * dfdh);
-            const double hm = root * root, rm = 1. / hm, c = sqrt(g * hm);
-            s1m = uL - (hm - hL) * sqrt(hg * (rm + rL)) - c;
-            s2m = uR + (hm - hR) * sqrt(hg * (rm + rR)) + c;
-        } else {
-            const double slope = (fmx - fmn) / (hmax - hmin);
-            const double c = sqrt(g * (hmin - fmn / slope));
-            if (!right) { s1m = aL - 3. * c; s2m = aL - c; }
-            else { s2m = aR + 3. * c; s1m = aR + c; }
-        }
+        const double q = 3. * sqmin;
+        clear = greater(uR + sqmax, up) && greater(down, uL - sqmax) && (right ? greater(aR + q, up) : greater(down, aL - q));
     }
-    double lam0 = greater(sL, e1) ? e1 : sL, lam2 = greater(e2, sR) ? e2 : sR;
-    if (greater(lam0, s2m)) lam0 = s2m;
-    if (greater(s1m, lam2)) lam2 = s1m;
+    if (!clear) {
+        const double hmin = right ? hL : hR, hmax = right ? hR : hL;
+        double s1m, s2m;
+        if (greater(fmn, 0.)) {
+            const double root0 = -delu + 2. * (sqL + sqR), root = __double_as_longlong(root0) < 0 ? 0. : root0;
+            const double c = sqrt(g * (g16r * (root * root)));
+            s1m = aL - 3. * c;
+            s2m = aR + 3. * c;
+        } else {
+            const double fmx = delu + (hmax - hmin) * sqrt(mean / (hmax * hmin));
+            if (!greater(fmx, 0.)) {
+                const double iL = 1. / hL, iR = 1. / hR, rmax = right ? iR : iL, rmin = right ? iL : iR;
+                const double gM = sqrt(hg * (rmax + rmax)), gm = sqrt(hg * (rmax + rmin)), gap = hmax - hmin;
+                const double F0 = delu + gap * gm;
+                const double q = (g * gap) / (4. * (hmax * hmax) * gm);
+                // ((gL - qL) + gR) - qR with the deeper side's q zero
+                const double dfdh = right ? (gm - q) + gM : (gM + gm) - q;
+                const double h0 = sqrt(hmax), root = h0 - F0 / (2. * h0 * dfdh);
+                const double hm = root * root, rm = 1. / hm, c = sqrt(g * hm);
+                s1m = uL - (hm - hL) * sqrt(hg * (rm + iL)) - c;
+                s2m = uR + (hm - hR) * sqrt(hg * (rm + iR)) + c;
+            } else {
+                const double slope = (fmx - fmn) / (hmax - hmin);
+                const double c = sqrt(g * (hmin - fmn / slope));
+                if (!right) { s1m = aL - 3. * c; s2m = aL - c; }
+                else { s2m = aR + 3. * c; s1m = aR + c; }
+            }
+        }
+        if (greater(lam0, s2m)) lam0 = s2m;
+        if (greater(s1m, lam2)) lam2 = s1m;
+    }
     // wave strengths
     const double d0 = hR - hL, d1 = huR - huL, d2 = phiR - phiL;
     const double r20 = lam0 * lam0, r22 = lam2 * lam2;
-    const double det = lam0 - lam2, rdet = 1. / det;
+    const double det = lam0 - lam2, rdet = reciprocal(det);
     const double b0 = quotient(d1 - d0 * lam2, det, rdet);
     const double b1 = quotient(((d1 * r22 - lam2 * d2) - d0 * (lam0 * r22 - lam2 * r20)) + (lam0 * d2 - d1 * r20), det, rdet);
     const double b2 = quotient(d0 * lam0 - d1, det, rdet);
@@ -251,7 +273,8 @@ __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, Bound
             double hl = eL - top, hr = eR - top;
             if (!greater(hl, thin)) hl = 0.;
             if (!greater(hr, thin)) hr = 0.;
-            const double kl = greater(hL, dry) ? hl / hL : 0., kr = greater(hR, dry) ? hr / hR : 0.;
+            const double kl = greater(hL, dry) ? quotient(hl, hL, reciprocal(hL)) : 0.;
+            const double kr = greater(hR, dry) ? quotient(hr, hR, reciprocal(hR)) : 0.;
             const double loc[8] = {inner ? hl : hL, inner ? unL * kl : unL, inner ? utL * kl : utL, inner ? top : bL,
                                    inner ? hr : hR, inner ? unR * kr : unR, inner ? utR * kr : utR, inner ? top : bR};
             Solve64 o;
