@@ -389,6 +389,7 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
             CK(cudaGetLastError());
             CK(cudaStreamSynchronize(nullptr));
             s->work.cw = p_cw; s->work.rarea = p_rarea;
+            TRY(s->alloc(&s->c64.prim[0], nc));
         }
         s->small64 = precision == BRX_FP64 && s->maxdeg <= 4;
         if (s->small64) {
@@ -397,7 +398,7 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
             Cells64 &g = s->c64;
             TRY(s->alloc(&g.ls, nc)); TRY(s->alloc(&g.lsr, nc)); TRY(s->alloc(&g.par, nc)); TRY(s->alloc(&g.ccls, nc));
             TRY(s->alloc(&g.cidx, nadj)); TRY(s->alloc(&g.ent, nadj)); TRY(s->alloc(&g.unit, nadj));
-            TRY(s->alloc(&g.gbed, nc)); TRY(s->alloc(&g.prim[0], nc)); TRY(s->alloc(&g.prim[1], nc));
+            TRY(s->alloc(&g.gbed, nc)); TRY(s->alloc(&g.prim[1], nc));
             k64_tables<<<std::max(1, std::min((nc + 255) / 256, s->sms * 32)), 256>>>(m, g);
             CK(cudaGetLastError());
             CK(cudaStreamSynchronize(nullptr));
@@ -1041,6 +1042,15 @@ extern "C" int brx_hllc_set(brx_solver *s, const int *entry_face, const int *ent
     TRY(s->upload(&p_ent, ent.data(), nadj)); TRY(s->upload(&p_geo, geo.data(), nadj));
     TRY(s->upload(&p_inv, inverse, 3 * (size_t)nc));
     s->hllc.ent = p_ent; s->hllc.geo = p_geo; s->hllc.inverse = p_inv;
+    if (s->precision == BRX_FP64) {
+        double2 *p_square;
+        TRY(s->alloc(&p_square, nadj));
+        // on the default stream, which follows the uploads
+        k_hllc_squares<<<std::max(1, std::min((nadj + 255) / 256, s->sms * 32)), 256>>>(nadj, p_geo, p_square);
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(nullptr));
+        s->hllc.square = p_square; s->hllc.prim = s->c64.prim[0];
+    }
     if (s->precision == BRX_MIXED) {
         // FP32 stencil of the mixed form: LS offset over its squared length
         // (zero for coincident centres), midpoint offset, the LS inverse, and
@@ -1144,7 +1154,8 @@ static int max_block(const brx_solver *s, int kind)
     case K_HKT_GRAD: fn = (const void *)k_hkt_gradients; break;
     case K_HKT_FACES: fn = (const void *)k_hkt_stress; break;
     case KH_CELLS_SHAPE:
-        fn = small ? (const void *)k_hllc_cells<4> : (const void *)k_hllc_cells<MAX_CELL_FACES>;
+        fn = s->maxdeg <= 3 ? (const void *)k_hllc_cells<3>
+             : small ? (const void *)k_hllc_cells<4> : (const void *)k_hllc_cells<MAX_CELL_FACES>;
         break;
     case KH_PREDICT_SHAPE: fn = (const void *)k_hllc_predict; break;
     case KH_FACES_SHAPE: fn = (const void *)k_hllc_faces; break;
@@ -1580,7 +1591,8 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
     switch (kind) {
     case K_DRAG:
         k_open_drag<<<SSHAPE(K_DRAG, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl,
-                                                             s->method == BRX_METHOD_FWAVE ? s->c64.prim[0] : nullptr);
+                                                             s->small64 || s->method == BRX_METHOD_HLLC ? s->c64.prim[0]
+                                                                                                       : nullptr);
         return 1;
     case K_BOUNDARY:
         if (!s->nslot) return 0;
@@ -1675,7 +1687,8 @@ static int launch_hllc(brx_solver *s, int kind, cudaStream_t st = nullptr)
     HCell *rec = reinterpret_cast<HCell *>(s->work.rec);      // 96 of the 128 bytes per cell
     switch (kind) {
     case KH_CELLS:
-        if (s->maxdeg <= 4) k_hllc_cells<4><<<SSHAPE(KH_CELLS_SHAPE, s->nc), 0, st>>>(s->mesh, s->state, s->hllc, rec, s->d_ctrl);
+        if (s->maxdeg <= 3) k_hllc_cells<3><<<SSHAPE(KH_CELLS_SHAPE, s->nc), 0, st>>>(s->mesh, s->state, s->hllc, rec, s->d_ctrl);
+        else if (s->maxdeg <= 4) k_hllc_cells<4><<<SSHAPE(KH_CELLS_SHAPE, s->nc), 0, st>>>(s->mesh, s->state, s->hllc, rec, s->d_ctrl);
         else k_hllc_cells<MAX_CELL_FACES><<<SSHAPE(KH_CELLS_SHAPE, s->nc), 0, st>>>(s->mesh, s->state, s->hllc, rec, s->d_ctrl);
         return 1;
     case KH_TURB0:        // rotor terms on the start state (stage 1 reads work)
