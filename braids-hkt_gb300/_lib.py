@@ -44,6 +44,7 @@ SIGNATURES = {
     "brx_advance_poll": (I, [P, P, P]),
     "brx_solver_bytes": (C.c_longlong, [P]),
     "brx_totals": (I, [P, P]),
+    "brx_step_budget": (I, [P, P, P]),
     "brx_rating_set": (I, [P, P, P, P]),
     "brx_outlet_chains_set": (I, [P, I, P, P, P]),
     "brx_weir_set": (I, [P, P]),

@@ -106,7 +106,12 @@ struct brx_solver {
     bool has_exner = false;
     int *d_cell_off = nullptr, *d_face_off = nullptr;
     double *d_exdt = nullptr;
-    double *d_totals = nullptr;      // (nscen, 2) brx_totals output
+    double *d_totals = nullptr;      // (nscen, 3) sums, (nscen, 2) gravity and dry depth
+    double *h_totals = nullptr;      // (nscen, 3) pinned
+    int *d_totals_first = nullptr;   // (nscen+1) first block of each scenario
+    Pair *d_totals_part = nullptr;   // (blocks, 3) partial sums
+    unsigned *d_totals_tickets = nullptr;
+    int totals_widest = 0;           // most blocks of one scenario
     int tile_cells = 0;              // mixed f-wave: cells per tile of the tile sweep (0: separate sweeps)
     TileDev tiles{};                 // tile tables (valid when tile_smem > 0)
     int tile_smem = 0;
@@ -501,6 +506,7 @@ extern "C" int brx_solver_destroy(brx_solver *s)
     for (void *p : s->tile_allocs) cudaFree(p);
     if (s->h_ctrl) cudaFreeHost(s->h_ctrl);
     if (s->h_hist) cudaFreeHost(s->h_hist);
+    if (s->h_totals) cudaFreeHost(s->h_totals);
     if (s->fork) cudaEventDestroy(s->fork);
     if (s->polled) cudaEventDestroy(s->polled);
     if (s->join) cudaEventDestroy(s->join);
@@ -1884,21 +1890,59 @@ extern "C" int brx_advance_poll(brx_solver *s, int *done, brx_advance_stats *sta
     return finish_interval(s, stats);
 }
 
+// Scratch of the compensated sums (device partials and tickets, pinned values).
+static int ensure_totals(brx_solver *s)
+{
+    if (s->d_totals) return BRX_OK;
+    std::vector<int> first(s->nscen + 1, 0);
+    s->totals_widest = 1;
+    for (int i = 0; i < s->nscen; ++i) {
+        const int blocks = totals_blocks(s->cell_offset[i + 1] - s->cell_offset[i]);
+        first[i + 1] = first[i] + blocks;
+        s->totals_widest = std::max(s->totals_widest, blocks);
+    }
+    TRY(s->upload(&s->d_totals_first, first.data(), first.size()));
+    TRY(s->alloc(&s->d_totals_part, 3 * (size_t)first[s->nscen]));
+    TRY(s->alloc(&s->d_totals_tickets, s->nscen));
+    CK(cudaMemset(s->d_totals_tickets, 0, sizeof(unsigned) * s->nscen));
+    CK(cudaStreamSynchronize(nullptr));
+    CK(cudaMallocHost(&s->h_totals, sizeof(double) * 3 * s->nscen));
+    return s->alloc(&s->d_totals, 5 * (size_t)s->nscen);
+}
+
 extern "C" int brx_totals(brx_solver *s, double *out)
 {
     TRY(ensure_ready(s));
     if (!out) return fail(BRX_ERR_ARGUMENT, "null output");
     if (s->pending) return fail(BRX_ERR_STATE, "an asynchronous interval is in flight");
-    if (!s->d_totals) TRY(s->alloc(&s->d_totals, 4 * (size_t)s->nscen));
-    double *d = s->d_totals, *gd = s->d_totals + 2 * (size_t)s->nscen;
-    std::vector<double> h_gd(2 * (size_t)s->nscen);
-    for (int i = 0; i < s->nscen; ++i) { h_gd[2 * i] = s->h_ctrl[i].grav; h_gd[2 * i + 1] = s->h_ctrl[i].dry; }
-    CK(cudaMemcpyAsync(gd, h_gd.data(), sizeof(double) * h_gd.size(), cudaMemcpyHostToDevice, s->stream));
-    k_totals<<<s->nscen, 256, 0, s->stream>>>(s->mesh, s->state.q[0], s->state.z, gd, d);
+    TRY(ensure_totals(s));
+    double *d = s->d_totals, *gd = s->d_totals + 3 * (size_t)s->nscen;
+    for (int i = 0; i < s->nscen; ++i) { s->h_totals[2 * i] = s->h_ctrl[i].grav; s->h_totals[2 * i + 1] = s->h_ctrl[i].dry; }
+    CK(cudaMemcpyAsync(gd, s->h_totals, sizeof(double) * 2 * s->nscen, cudaMemcpyHostToDevice, s->stream));
+    k_totals<false><<<dim3(s->totals_widest, s->nscen), 256, 0, s->stream>>>(
+        s->mesh, s->state.q[0], nullptr, s->state.z, gd, s->d_totals_first, s->d_totals_part, s->d_totals_tickets, d);
     s->launches++;
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(out, d, sizeof(double) * 2 * s->nscen, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaMemcpyAsync(s->h_totals, d, sizeof(double) * 2 * s->nscen, cudaMemcpyDeviceToHost, s->stream));
     CK(cudaStreamSynchronize(s->stream));
+    memcpy(out, s->h_totals, sizeof(double) * 2 * s->nscen);
+    return BRX_OK;
+}
+
+extern "C" int brx_step_budget(brx_solver *s, const double *start_device, double *out)
+{
+    TRY(ensure_ready(s));
+    if (!start_device || !out) return fail(BRX_ERR_ARGUMENT, "null argument");
+    if (s->pending) return fail(BRX_ERR_STATE, "an asynchronous interval is in flight");
+    TRY(ensure_totals(s));
+    k_totals<true><<<dim3(s->totals_widest, s->nscen), 256, 0, s->stream>>>(
+        s->mesh, s->state.q[0], start_device, s->state.z, nullptr, s->d_totals_first, s->d_totals_part,
+        s->d_totals_tickets, s->d_totals);
+    s->launches++;
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync(s->h_totals, s->d_totals, sizeof(double) * 3 * s->nscen, cudaMemcpyDeviceToHost, s->stream));
+    CK(cudaStreamSynchronize(s->stream));
+    memcpy(out, s->h_totals, sizeof(double) * 3 * s->nscen);
     return BRX_OK;
 }
 

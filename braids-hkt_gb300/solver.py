@@ -625,12 +625,12 @@ class RiverSolver:
         check(self.lib.brx_ledger_gross_get(self.h, _ptr(out)))
         return out
 
-    def _inventory(self, h0, h1):
-        """sum(max(h0, h1) area) per scenario (shoreline_solver.py:356): the
-        water inventory that scales the roundoff allowance."""
-        a = self.packed["area"]
-        v = np.maximum(h0, h1) * a
-        return np.add.reduceat(v, self.packed["cell_offset"][:-1].astype(np.int64))
+    def _budget(self, q0):
+        """(volume of the start state q0, volume now, inventory sum(max(h0, h1) area)) per
+        scenario (shoreline_solver.py:353-357), compensated sums on the device."""
+        out = np.zeros((self.nscen, 3))
+        check(self.lib.brx_step_budget(self.h, C.c_void_p(q0.data_ptr()), _ptr(out)))
+        return out.T
 
     def step(self, dt):
         """Advance by dt from the owner clock with the owner's water-budget
@@ -642,15 +642,13 @@ class RiverSolver:
         WaterBudgetError raised; on success the ledger is committed."""
         self.torch.cuda.current_stream().synchronize()
         q0, z0, hints0 = self.q.clone(), self.z.clone(), self.hints()
-        v0 = np.atleast_2d(self.totals())[:, 0]
         try:
             diag = self.advance(dt, self.time[0])
         except BaseException:
             self.q.copy_(q0); self.z.copy_(z0); self.set_hints(hints0)
             raise
-        v1 = np.atleast_2d(self.totals())[:, 0]
+        v0, v1, inventory = self._budget(q0)
         ledger = self.ledger()
-        inventory = self._inventory(q0[0].cpu().numpy(), self.q[0].cpu().numpy())
         residual, roundoff, ok = water_budget(v0, v1, ledger, inventory, self.gross_boundary_volume())
         if not ok.all():
             self.q.copy_(q0); self.z.copy_(z0); self.set_hints(hints0)

@@ -319,6 +319,13 @@ int brx_advance_poll(brx_solver *s, int *done, brx_advance_stats *stats);
  * batch the same totals without copying the state. */
 int brx_totals(brx_solver *s, double *out);
 
+/* The volumes of the owner's water budget (ShorelineSolver.step,
+ * src/braids_core/sediment/shoreline_solver.py:353-357) per scenario, summed
+ * as brx_totals sums (out: nscen x 3, host): sum(A h0) of the start state,
+ * sum(A h) of the bound state, and the inventory sum(A max(h0, h)) that scales
+ * the roundoff allowance. start_device: (3, nc) start state in device memory. */
+int brx_step_budget(brx_solver *s, const double *start_device, double *out);
+
 /* Device bytes the solver holds (for admission against a memory budget). */
 long long brx_solver_bytes(const brx_solver *s);
 
