@@ -104,6 +104,7 @@ struct brx_solver {
     double *d_tdiag_out = nullptr;   // (nrotor, 16) diagnostics of brx_turbines_diagnose
     ExnerDev exner{};                // bed model (valid when has_exner)
     bool has_exner = false;
+    int exner_widest = 0;            // most chunks of one scenario
     int *d_cell_off = nullptr, *d_face_off = nullptr;
     double *d_exdt = nullptr;
     double *d_totals = nullptr;      // (nscen, 3) sums, (nscen, 2) gravity and dry depth
@@ -1389,9 +1390,25 @@ extern "C" int brx_exner_set(brx_solver *s, const int *enabled, const double *pa
     TRY(s->upload(&p_bc, bedbc, nf)); TRY(s->upload(&p_feed, feed, nf)); TRY(s->upload(&p_rock, rock, nc));
     TRY(s->upload(&p_dxdy, dxdy, 2 * (size_t)nadj)); TRY(s->upload(&p_inv, inverse, 3 * (size_t)nc));
     TRY(s->upload(&p_xy, xy, 2 * (size_t)nc));
+    // the offsets become weighted offsets in place, on the default stream, which follows the uploads
+    k_flow_weights<<<std::max(1, std::min((nadj + 255) / 256, s->sms * 32)), 256>>>(nadj, p_dxdy, p_dxdy);
+    CK(cudaGetLastError());
     e.enabled = p_en; e.param = p_par; e.bedbc = p_bc; e.feed = p_feed; e.rock = p_rock;
-    e.dxdy = p_dxdy; e.inverse = p_inv; e.xy = p_xy;
-    TRY(s->alloc(&e.cell, 6 * (size_t)nc)); TRY(s->alloc(&e.gz, 2 * (size_t)nc)); TRY(s->alloc(&e.flux, nf));
+    e.wdxdy = p_dxdy; e.inverse = p_inv; e.xy = p_xy;
+    std::vector<int> first(ns + 1, 0);
+    s->exner_widest = 1;
+    for (int i = 0; i < ns; ++i) {
+        const int blocks = exner_blocks(s->cell_offset[i + 1] - s->cell_offset[i]);
+        first[i + 1] = first[i] + blocks;
+        s->exner_widest = std::max(s->exner_widest, blocks);
+    }
+    int *p_first;
+    TRY(s->upload(&p_first, first.data(), first.size()));
+    e.first = p_first;
+    TRY(s->alloc(&e.part, 3 * (size_t)first[ns])); TRY(s->alloc(&e.tickets, ns)); TRY(s->alloc(&e.out_of_range, ns));
+    CK(cudaMemset(e.tickets, 0, sizeof(unsigned) * ns));
+    CK(cudaStreamSynchronize(nullptr));
+    TRY(s->alloc(&e.cell, 3 * (size_t)nc)); TRY(s->alloc(&e.gz, 2 * (size_t)nc)); TRY(s->alloc(&e.flux, nf));
     TRY(s->alloc(&e.fac, nc)); TRY(s->alloc(&e.ztrial, nc)); TRY(s->alloc(&e.stats, (size_t)ns * ES_N));
     TRY(s->alloc(&e.wet, nc)); TRY(s->alloc(&e.bad, ns));
     TRY(s->alloc(&s->d_exdt, ns));
@@ -1417,17 +1434,16 @@ extern "C" int brx_exner(brx_solver *s, const double *dt, double *stats)
     cudaStream_t st = s->stream;
     CK(cudaMemcpyAsync(s->d_exdt, dt, sizeof(double) * s->nscen, cudaMemcpyHostToDevice, st));
     CK(cudaMemsetAsync(e.bad, 0, sizeof(int) * s->nscen, st));
+    CK(cudaMemsetAsync(e.out_of_range, 0, sizeof(int) * s->nscen, st));
     CK(cudaMemsetAsync(e.stats, 0, sizeof(double) * s->nscen * ES_N, st));
     const double *q = s->state.q[0];
     double *z = const_cast<double *>(s->state.z);     // the caller's bound bed, updated in place
     k_ex_cells<<<s->grid_c256, 256, 0, st>>>(s->mesh, e, q, z);
     k_ex_faces<<<s->grid_f, 128, 0, st>>>(s->mesh, e, z);
     k_ex_donor<<<s->grid_c256, 256, 0, st>>>(s->mesh, e, z);
-    k_ex_limit<<<s->grid_f256, 256, 0, st>>>(s->mesh, e);
-    k_ex_trial<<<s->grid_c256, 256, 0, st>>>(s->mesh, e, z);
-    k_ex_reduce<<<s->nscen, 256, 0, st>>>(s->mesh, e, q, z, s->d_cell_off, s->d_face_off);
+    k_ex_trial<<<dim3(s->exner_widest, s->nscen), 256, 0, st>>>(s->mesh, e, s->bnd, q, z);
     k_ex_commit<<<s->grid_c256, 256, 0, st>>>(s->mesh, e, z);
-    s->launches += 7;
+    s->launches += 5;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(stats, e.stats, sizeof(double) * s->nscen * ES_N, cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
