@@ -189,6 +189,13 @@ __device__ __forceinline__ void warp_max_peak_f(unsigned long long *peak_of_sid0
     }
 }
 
+// a b + c d and a b - c d with the rounding written out. The compiler may fuse
+// either product, and chooses anew in each instance and unrolled copy: a
+// scenario would get other last bits in a batch whose widest cell selects
+// another instance of the sweep.
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
+__device__ __forceinline__ float diff2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
+
 // ---------------------------------------------------------------------------
 // Gradient bounds: the directional projection limiter on a set of slabs
 //     -bm[j] <= (ux[j], uy[j]) . g <= bp[j]      (entries j of one cell)
@@ -206,47 +213,72 @@ __device__ __forceinline__ bool slabs_feasible(const Slabs<N> &S, float x, float
 #pragma unroll (N <= 4 ? N : 1)
     for (int j = 0; j < N; ++j)
         if (S.mask >> j & 1u) {
-            const float t = S.ux[j] * x + S.uy[j] * y;
-            const float a = fabsf(S.ux[j] * x) + fabsf(S.uy[j] * y);
+            const float py = __fmul_rn(S.uy[j], y), t = __fmaf_rn(S.ux[j], x, py);
+            const float a = __fadd_rn(fabsf(__fmul_rn(S.ux[j], x)), fabsf(py));
             if (t > S.bp[j] + (2.e-14f + 16.f * FEPS * (a + S.bp[j]))) ok = false;
             if (-t > S.bm[j] + (2.e-14f + 16.f * FEPS * (a + S.bm[j]))) ok = false;
         }
     return ok;
 }
 
+// Entry i of a slab row: a chain of selects where the rows live in registers.
+template <int N>
+__device__ __forceinline__ float slab_entry(const float (&a)[N], int i)
+{
+    if constexpr (N <= 4) {
+        float v = a[0];
+#pragma unroll
+        for (int j = 1; j < N; ++j) v = i == j ? a[j] : v;
+        return v;
+    } else {
+        return a[i];
+    }
+}
+
 // Nearest feasible point: the best feasible candidate among single-side
 // projections and pairwise vertices. The polygon contains the origin (all
 // bounds >= 0) and is convex, so its nearest point is unique and lies on a
 // side the unlimited gradient violates: only violated sides seed candidates.
+// Each lane walks its own list of violated sides, so that lanes with different
+// ones share the code of a side (unrolled over the sides, a warp ran every
+// side that any lane violates, one after another); a feasible projection is the
+// nearest point of the side's half plane, which holds the polygon, and ends it.
 template <int N>
 __device__ __forceinline__ void slabs_project(const Slabs<N> &S, float &x, float &y)
 {
     const float rx = x, ry = y;
-    float bx = 0.f, by = 0.f, best = rx * rx + ry * ry;
+    unsigned todo = 0u, minus = 0u;
 #pragma unroll (N <= 4 ? N : 1)
     for (int i = 0; i < N; ++i) {
         if (!(S.mask >> i & 1u)) continue;
-        const float t = S.ux[i] * rx + S.uy[i] * ry;
-        float ax, ay, b;
-        if (t - S.bp[i] > 0.f) { ax = S.ux[i]; ay = S.uy[i]; b = S.bp[i]; }
-        else if (-t - S.bm[i] > 0.f) { ax = -S.ux[i]; ay = -S.uy[i]; b = S.bm[i]; }
-        else continue;
-        const float dot = ax * rx + ay * ry - b;
+        const float t = dot2(S.ux[i], rx, S.uy[i], ry);
+        if (t - S.bp[i] > 0.f) todo |= 1u << i;
+        else if (-t - S.bm[i] > 0.f) { todo |= 1u << i; minus |= 1u << i; }
+    }
+    float bx = 0.f, by = 0.f, best = dot2(rx, rx, ry, ry);
+    while (todo) {
+        const int i = __ffs(todo) - 1;
+        todo &= todo - 1;
+        float ax = slab_entry(S.ux, i), ay = slab_entry(S.uy, i), b = slab_entry(S.bp, i);
+        if (minus >> i & 1u) { ax = -ax; ay = -ay; b = slab_entry(S.bm, i); }
+        const float dot = dot2(ax, rx, ay, ry) - b;
         float cx = rx - dot * ax, cy = ry - dot * ay;
-        float d = (cx - rx) * (cx - rx) + (cy - ry) * (cy - ry);
-        if (d < best && slabs_feasible(S, cx, cy)) { bx = cx; by = cy; best = d; }
+        float d = dot2(cx - rx, cx - rx, cy - ry, cy - ry);
+        if (d < best && slabs_feasible(S, cx, cy)) { bx = cx; by = cy; break; }
 #pragma unroll (N <= 4 ? N : 1)
-        for (int j = 0; j < N; ++j) {
-            if (j == i || !(S.mask >> j & 1u)) continue;
+        for (int k = 0; k < N - 1; ++k) {
+            const int j = k + (k >= i);
+            if (!(S.mask >> j & 1u)) continue;
+            const float ux = slab_entry(S.ux, j), uy = slab_entry(S.uy, j);
 #pragma unroll
             for (int side = 0; side < 2; ++side) {
-                const float jx = side ? -S.ux[j] : S.ux[j], jy = side ? -S.uy[j] : S.uy[j];
-                const float jb = side ? S.bm[j] : S.bp[j];
-                const float det = ax * jy - ay * jx;
+                const float jx = side ? -ux : ux, jy = side ? -uy : uy;
+                const float jb = side ? slab_entry(S.bm, j) : slab_entry(S.bp, j);
+                const float det = diff2(ax, jy, ay, jx);
                 if (fabsf(det) < 1.e-12f) continue;
-                cx = (b * jy - ay * jb) / det;
-                cy = (ax * jb - b * jx) / det;
-                d = (cx - rx) * (cx - rx) + (cy - ry) * (cy - ry);
+                cx = diff2(b, jy, ay, jb) / det;
+                cy = diff2(ax, jb, b, jx) / det;
+                d = dot2(cx - rx, cx - rx, cy - ry, cy - ry);
                 if (d < best && slabs_feasible(S, cx, cy)) { bx = cx; by = cy; best = d; }
             }
         }
@@ -289,7 +321,7 @@ __global__ void __launch_bounds__(128) km_bed(MeshDev m, StateDev s, MixedGeo g)
         float2 gb = make_float2(0.f, 0.f);
         const float4 inv = g.cinv[c];
         if (inv.x != 0.f || inv.y != 0.f || inv.z != 0.f) {
-            float gx = inv.x * bx + inv.y * by, gy = inv.y * bx + inv.z * by;
+            float gx = dot2(inv.x, bx, inv.y, by), gy = dot2(inv.y, bx, inv.z, by);
             Slabs<MAXF> S{};
             const float bp = fmaxf(0.f, hi), bm = fmaxf(0.f, -lo);
 #pragma unroll (MAXF <= 4 ? MAXF : 1)
@@ -297,7 +329,7 @@ __global__ void __launch_bounds__(128) km_bed(MeshDev m, StateDev s, MixedGeo g)
                 if (j >= deg) continue;      // (a break would stop the unrolling)
                 if (g.cidx[k0 + j].y & 4) continue;          // walls do not bound the bed
                 const float4 ge = g.cent[k0 + j];
-                const float len = sqrtf(ge.z * ge.z + ge.w * ge.w);
+                const float len = sqrtf(dot2(ge.z, ge.z, ge.w, ge.w));
                 if (len <= 0.f) continue;
                 const float il = 1.f / len;
                 S.ux[j] = ge.z * il; S.uy[j] = ge.w * il; S.bp[j] = bp * il; S.bm[j] = bm * il;
@@ -335,18 +367,18 @@ __device__ __forceinline__ void hkt_cell_gradients(const MeshDev &m, const Mixed
             const MxPrim pn = nb.prim(n);
             if (!pn.wet) continue;
             const float2 d = g.hdxy[k];
-            const float w = 1.f / (d.x * d.x + d.y * d.y);
+            const float w = 1.f / dot2(d.x, d.x, d.y, d.y);
             xx += w * d.x * d.x; xy += w * d.x * d.y; yy += w * d.y * d.y;
             const float dv[3] = {pn.u - pc.u, pn.v - pc.v, (pn.ehi - pc.ehi) + (pn.elo - pc.elo)};
 #pragma unroll
             for (int p = 0; p < 3; ++p) { bx[p] += w * d.x * dv[p]; by[p] += w * d.y * dv[p]; }
         }
-    const float det = xx * yy - xy * xy;
+    const float det = diff2(xx, yy, xy, xy);
     const bool solve = det > 1e-6f * fmaxf(1.f, xx * yy);
 #pragma unroll
     for (int p = 0; p < 3; ++p) {
-        g.hgrad[(2 * p) * nc + c] = solve ? (yy * bx[p] - xy * by[p]) / det : 0.f;
-        g.hgrad[(2 * p + 1) * nc + c] = solve ? (xx * by[p] - xy * bx[p]) / det : 0.f;
+        g.hgrad[(2 * p) * nc + c] = solve ? diff2(yy, bx[p], xy, by[p]) / det : 0.f;
+        g.hgrad[(2 * p + 1) * nc + c] = solve ? diff2(xx, by[p], xy, bx[p]) / det : 0.f;
     }
 }
 
@@ -375,15 +407,26 @@ __device__ __forceinline__ MxRec mx_record(const MeshDev &m, const StateDev &s, 
         float lo[4] = {0.f, u, v, 0.f}, hi[4] = {0.f, u, v, 0.f};
         float bx[4] = {0.f, 0.f, 0.f, 0.f}, by[4] = {0.f, 0.f, 0.f, 0.f};
         bool active = wet;
-        for (int k = k0; k < k0 + deg; ++k) {
-            const int2 id = nb.id(k, k - k0);
+        // triangles: the three entries are requested at once, so their
+        // neighbours' loads wait for one, not each for its own
+        constexpr int AHEAD = MAXF == 3 ? MAXF : 1;
+        int2 ids[AHEAD];
+        if constexpr (MAXF == 3) {
+#pragma unroll
+            for (int j = 0; j < MAXF; ++j) ids[j] = j < deg ? nb.id(k0 + j, j) : make_int2(-1, 0);
+        }
+#pragma unroll (MAXF == 3 ? MAXF : 1)
+        for (int j = 0; j < MAXF; ++j) {
+            if (j >= deg) continue;
+            const int k = k0 + j;
+            const int2 id = MAXF == 3 ? ids[MAXF == 3 ? j : 0] : nb.id(k, j);
             const int n = id.x;
             if (n < 0) {
                 if (id.y & 1) active = true;
                 else if ((id.y & 4) && wet) {
                     // a wall bounds the velocities by the mirrored cell velocity
                     const float2 nn = g.fnorm[m.faces[k]];
-                    const float un = u * nn.x + v * nn.y;
+                    const float un = dot2(u, nn.x, v, nn.y);
                     const float mx = u - 2.f * un * nn.x, my = v - 2.f * un * nn.y;
                     lo[1] = fminf(lo[1], mx); hi[1] = fmaxf(hi[1], mx);
                     lo[2] = fminf(lo[2], my); hi[2] = fmaxf(hi[2], my);
@@ -419,13 +462,13 @@ __device__ __forceinline__ MxRec mx_record(const MeshDev &m, const StateDev &s, 
         if (active && (inv.x != 0.f || inv.y != 0.f || inv.z != 0.f)) {
 #pragma unroll
             for (int p = 0; p < 3; ++p) {
-                gx[p] = inv.x * bx[p] + inv.y * by[p];
-                gy[p] = inv.y * bx[p] + inv.z * by[p];
+                gx[p] = dot2(inv.x, bx[p], inv.y, by[p]);
+                gy[p] = dot2(inv.y, bx[p], inv.z, by[p]);
             }
             float bedtol = 0.f, sq = 0.f;
             if (outlet) {
-                gx[3] = inv.x * bx[3] + inv.y * by[3];
-                gy[3] = inv.y * bx[3] + inv.z * by[3];
+                gx[3] = dot2(inv.x, bx[3], inv.y, by[3]);
+                gy[3] = dot2(inv.y, bx[3], inv.z, by[3]);
                 bedtol = 64.f * FEPS * fmaxf(1.f, fabsf(float(s.z[c])));
                 sq = wet ? sqrtf(ct.gravf * hf) : 0.f;
             } else {
@@ -446,11 +489,11 @@ __device__ __forceinline__ MxRec mx_record(const MeshDev &m, const StateDev &s, 
                 if (outlet && (nb.id(k, j).y & 2) && wet) {
                     // an open stage outlet with a subcritical wet owner keeps its bed slope
                     const float2 nn = g.fnorm[m.faces[k]];
-                    if (fabsf(u * nn.x + v * nn.y) < sq && fabsf(gx[3] * rx + gy[3] * ry) > bedtol) continue;
+                    if (fabsf(dot2(u, nn.x, v, nn.y)) < sq && fabsf(dot2(gx[3], rx, gy[3], ry)) > bedtol) continue;
                 }
 #pragma unroll
                 for (int p = 1; p < 3; ++p) {
-                    const float dd = gx[p] * rx + gy[p] * ry;
+                    const float dd = dot2(gx[p], rx, gy[p], ry);
                     const float ctr = p == 1 ? u : v;
                     if (fabsf(dd) <= 64.f * FEPS * fmaxf(1.f, fmaxf(fabsf(ctr), fmaxf(fabsf(lo[p]), fabsf(hi[p])))))
                         continue;
@@ -458,7 +501,7 @@ __device__ __forceinline__ MxRec mx_record(const MeshDev &m, const StateDev &s, 
                     if (dd > 0.f) th = fminf(th, (hi[p] - ctr) / dd);
                     if (dd < 0.f) th = fminf(th, (lo[p] - ctr) / dd);
                 }
-                const float len = sqrtf(rx * rx + ry * ry);
+                const float len = sqrtf(dot2(rx, rx, ry, ry));
                 if (len <= 0.f) continue;
                 const float il = 1.f / len;
                 S.ux[j] = rx * il; S.uy[j] = ry * il; S.bp[j] = b0p * il; S.bm[j] = b0m * il;
@@ -477,9 +520,9 @@ __device__ __forceinline__ MxRec mx_record(const MeshDev &m, const StateDev &s, 
                     const float rx = ge.z, ry = ge.w;
                     if ((fl & 2) && wet) {
                         const float2 nn = g.fnorm[m.faces[k]];
-                        if (fabsf(u * nn.x + v * nn.y) < sq && fabsf(gx[3] * rx + gy[3] * ry) > bedtol) continue;
+                        if (fabsf(dot2(u, nn.x, v, nn.y)) < sq && fabsf(dot2(gx[3], rx, gy[3], ry)) > bedtol) continue;
                     }
-                    const float len = sqrtf(rx * rx + ry * ry);
+                    const float len = sqrtf(dot2(rx, rx, ry, ry));
                     if (len <= 0.f || (fl & 4)) continue;          // walls do not bound the bed
                     const float il = 1.f / len;
                     S.ux[j] = rx * il; S.uy[j] = ry * il; S.bp[j] = b3p * il; S.bm[j] = b3m * il;
@@ -494,7 +537,7 @@ __device__ __forceinline__ MxRec mx_record(const MeshDev &m, const StateDev &s, 
         if (!flatten) {
             for (int k = k0; k < k0 + deg; ++k) {
                 const float4 ge = g.cent[k];
-                const float de = gx[0] * ge.z + gy[0] * ge.w, db = gx[3] * ge.z + gy[3] * ge.w;
+                const float de = dot2(gx[0], ge.z, gy[0], ge.w), db = dot2(gx[3], ge.z, gy[3], ge.w);
                 if (hf + (de - db) <= dry || fabsf(db) >= hf) { flatten = true; break; }
             }
         }
@@ -509,6 +552,13 @@ __device__ __forceinline__ MxRec mx_record(const MeshDev &m, const StateDev &s, 
     }
 }
 
+// MAXF 3 (triangles), 4 or any: bound by instruction issue and by the chain of
+// loads offset -> entry -> neighbour, which only resident warps hide: at 6 blocks
+// of 80 registers 68 us, at 8 of 64 57 us, at 10 of 51 61 us per stage at 900k
+// triangles. Holding all of an entry's data (68 us) costs more registers than the
+// shorter chain is worth; the entries alone are requested ahead. Against four
+// slots and the limiter's sides unrolled: 900k 64 -> 57 us, 809k in a batch of
+// twelve 76 -> 65 us.
 template <int MAXF>
 __global__ void __launch_bounds__(128, BRX_CELLS_MIN_BLOCKS) km_cells(MeshDev m, StateDev s, Ctrl *ctrl, Work w,
                                                                       MixedGeo g, int stage, TurbDev t, int turb)
@@ -1460,7 +1510,10 @@ int mixed_max_block(int kind, int maxdeg)
     const void *fn = nullptr;
     switch (kind) {
     case K_DRAG: fn = (const void *)brx_mx::km_open_drag; break;
-    case K_CELLS: fn = small ? (const void *)brx_mx::km_cells<4> : (const void *)brx_mx::km_cells<MAX_CELL_FACES>; break;
+    case K_CELLS:
+        fn = maxdeg <= 3 ? (const void *)brx_mx::km_cells<3> : small ? (const void *)brx_mx::km_cells<4>
+                                                                     : (const void *)brx_mx::km_cells<MAX_CELL_FACES>;
+        break;
     case K_FACES: fn = (const void *)brx_mx::km_faces; break;
     case K_LIMIT: fn = (const void *)brx_mx::km_limit; break;
     case K_UPDATE: fn = (const void *)brx_mx::km_update; break;
@@ -1522,7 +1575,10 @@ int mixed_kernel(const Launch &L, int kind, int stage, double *out)
         brx_mixb::launch_boundary<float>(L.mesh, L.state, L.bnd, L.ctrl, L.nscen, stage, st);
         return 1;
     case K_CELLS:
-        if (small)
+        if (L.maxdeg <= 3)
+            brx_mx::km_cells<3><<<SHAPE(K_CELLS, nc), 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage, L.turb,
+                                                              L.has_turb);
+        else if (small)
             brx_mx::km_cells<4><<<SHAPE(K_CELLS, nc), 0, st>>>(L.mesh, L.state, L.ctrl, L.work, L.mx, stage, L.turb,
                                                               L.has_turb);
         else
