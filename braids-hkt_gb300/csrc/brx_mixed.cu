@@ -189,13 +189,6 @@ __device__ __forceinline__ void warp_max_peak_f(unsigned long long *peak_of_sid0
     }
 }
 
-// a b + c d and a b - c d with the rounding written out. The compiler may fuse
-// either product, and chooses anew in each instance and unrolled copy: a
-// scenario would get other last bits in a batch whose widest cell selects
-// another instance of the sweep.
-__device__ __forceinline__ float dot2(float a, float b, float c, float d) { return __fmaf_rn(a, b, __fmul_rn(c, d)); }
-__device__ __forceinline__ float diff2(float a, float b, float c, float d) { return __fmaf_rn(a, b, -__fmul_rn(c, d)); }
-
 // ---------------------------------------------------------------------------
 // Gradient bounds: the directional projection limiter on a set of slabs
 //     -bm[j] <= (ux[j], uy[j]) . g <= bp[j]      (entries j of one cell)
@@ -590,10 +583,10 @@ struct MxSide {
 
 __device__ __forceinline__ MxSide mx_side(const MxRec &r, float rx, float ry, float dry, bool dryface, unsigned &bad)
 {
-    float de = r.gx[0] * rx + r.gy[0] * ry;
-    float uu = r.u + (r.gx[1] * rx + r.gy[1] * ry);
-    float vv = r.v + (r.gx[2] * rx + r.gy[2] * ry);
-    float db = r.gx[3] * rx + r.gy[3] * ry;
+    float de = dot2(r.gx[0], rx, r.gy[0], ry);
+    float uu = r.u + (dot2(r.gx[1], rx, r.gy[1], ry));
+    float vv = r.v + (dot2(r.gx[2], rx, r.gy[2], ry));
+    float db = dot2(r.gx[3], rx, r.gy[3], ry);
     const float hf = r.h;
     const bool constant = r.flags & 1, wet = r.flags & 4;
     if (constant) {
@@ -645,16 +638,16 @@ __device__ __forceinline__ void hkt_face_terms(const MxRec &pa, const MxRec &pb,
     if (t.stress[sid]) {
         float h = fminf(pa.h, pb.h);
         h = fminf(h, fmaxf(0.f, .5f * (ea + eb) - fmaxf(0.f, zb)));
-        const float visc = wa * float(t.nu[a]) + wb * float(t.nu[b]);
+        const float visc = dot2(wa, float(t.nu[a]), wb, float(t.nu[b]));
         const float2 dd = g.hcc[f];
-        const float dn = dd.x * nx + dd.y * ny;
+        const float dn = dot2(dd.x, nx, dd.y, ny);
         const float du = pb.u - pa.u, dv = pb.v - pa.v;
         const float *G = g.hgrad;
-        float ux = wa * G[a] + wb * G[b], uy = wa * G[nc + a] + wb * G[nc + b];
-        float vx = wa * G[2 * nc + a] + wb * G[2 * nc + b], vy = wa * G[3 * nc + a] + wb * G[3 * nc + b];
+        float ux = dot2(wa, G[a], wb, G[b]), uy = dot2(wa, G[nc + a], wb, G[nc + b]);
+        float vx = dot2(wa, G[2 * nc + a], wb, G[2 * nc + b]), vy = dot2(wa, G[3 * nc + a], wb, G[3 * nc + b]);
         const float cu = (du - ux * dd.x - uy * dd.y) / dn, cv = (dv - vx * dd.x - vy * dd.y) / dn;
         ux += cu * nx; uy += cu * ny; vx += cv * nx; vy += cv * ny;
-        st = make_float2(visc * h * (2.f * ux * nx + (uy + vx) * ny), visc * h * ((uy + vx) * nx + 2.f * vy * ny));
+        st = make_float2(visc * h * dot2(2.f * ux, nx, uy + vx, ny), visc * h * dot2(uy + vx, nx, 2.f * vy, ny));
     }
     const int cf = __float_as_int(t0.w);
     const float top = t0.z, bed = fmaxf(fmaxf(0.f, zb), top);
@@ -664,20 +657,20 @@ __device__ __forceinline__ void hkt_face_terms(const MxRec &pa, const MxRec &pb,
     const float qg = .25f * gravity;
     const float ca = (cf & 1) ? qg * __fmul_rn(ha - hl, ha + hl) : 0.f;
     const float cb = (cf & 2) ? qg * __fmul_rn(hb - hr, hb + hr) : 0.f;
-    const float scale = qg * (hl * hl + hr * hr);                       // |po|, |pn| to first order
+    const float scale = qg * dot2(hl, hl, hr, hr);                       // |po|, |pn| to first order
     if (!(fminf(fminf(ha, hb), fminf(hl, hr)) <= dry) && !(fabsf(hr - hl) > .005f * h) &&
         !(fabsf(2.f * (ca - cb)) > 128.f * FEPS * fmaxf(1.f, scale))) {
         const float4 md = g.hmd[f];
-        const float sx = wa * md.x + wb * md.z, sy = wa * md.y + wb * md.w;
+        const float sx = dot2(wa, md.x, wb, md.z), sy = dot2(wa, md.y, wb, md.w);
         const float *G = g.hgrad;
-        float delta = qg * (__fmul_rn(hl - ha, hl + ha) + __fmul_rn(hr - hb, hr + hb)) +
-                      qg * ((da - db) / d) * __fmul_rn(ha - hb, ha + hb) + (ca + cb);
-        delta -= gravity * sx * (wa * ha * G[4 * nc + a] + wb * hb * G[4 * nc + b]);
-        delta -= gravity * sy * (wa * ha * G[5 * nc + a] + wb * hb * G[5 * nc + b]);
+        float delta = dot2(qg, __fadd_rn(__fmul_rn(hl - ha, hl + ha), __fmul_rn(hr - hb, hr + hb)), qg * ((da - db) / d),
+                           __fmul_rn(ha - hb, ha + hb)) + (ca + cb);
+        delta -= gravity * sx * dot2(wa * ha, G[4 * nc + a], wb * hb, G[4 * nc + b]);
+        delta -= gravity * sy * dot2(wa * ha, G[5 * nc + a], wb * hb, G[5 * nc + b]);
         // the actuator sink difference: FP64 rates, zero outside the rotor
         // support cells, so only faces touching one read and subtract them
         if (t.foot[a] | t.foot[b])
-            delta -= da * db / d * (float(t.raw[a] - t.raw[b]) * nx + float(t.raw[nc + a] - t.raw[nc + b]) * ny);
+            delta -= da * db / d * dot2(float(t.raw[a] - t.raw[b]), nx, float(t.raw[nc + a] - t.raw[nc + b]), ny);
         const float speed = sqrtf(gravity * h), theta = fminf(1.f, fmaxf(t1.z, t1.w) / speed);
         delta -= .5f * (1.f - theta) * speed * (2.f * hl * hr / (hl + hr)) * (t1.y - t1.x);
         pr = make_float2(delta * nx, delta * ny);
@@ -727,11 +720,11 @@ __device__ __forceinline__ MxFaceOut mx_face(const MeshDev &m, const StateDev &s
             if (kind == 2) { hR = hL; xR = xL; yR = yL; bRr = bLr; sR = sL; }
             float xRr = xR, yRr = yR;
             if (kind == 2) {
-                const float dot = xL * nx + yL * ny;
+                const float dot = dot2(xL, nx, yL, ny);
                 xRr = xL - 2.f * dot * nx; yRr = yL - 2.f * dot * ny;
             }
-            const float unL = xL * nx + yL * ny, utL = xL * (-ny) + yL * nx;
-            const float unR = xRr * nx + yRr * ny, utR = xRr * (-ny) + yRr * nx;
+            const float unL = dot2(xL, nx, yL, ny), utL = dot2(xL, -ny, yL, nx);
+            const float unR = dot2(xRr, nx, yRr, ny), utR = dot2(xRr, -ny, yRr, nx);
             float loc[8] = {hL, unL, utL, 0.f, hR, unR, utR, 0.f};
             float top_bed = 0.f;           // the face's common bed (kind 1), for the rotor terms
             if (kind == 1) {
@@ -826,13 +819,13 @@ __device__ __forceinline__ MxFaceOut mx_face(const MeshDev &m, const StateDev &s
                 }
             }
             // rotate the dynamic parts back; add the hydrostatic perturbation relative to each cell
-            const float lx = dl1 * nx - dl2 * ny + wallx * nx, ly = dl1 * ny + dl2 * nx + wallx * ny;
+            const float lx = diff2(dl1, nx, dl2, ny) + wallx * nx, ly = dot2(dl1, ny, dl2, nx) + wallx * ny;
             float hsL;
             if (hc > dry) hsL = (rc.flags & 1) ? 0.f : half_g * hydro_perturbation(L.dh, hL, hc, L.raw, L.db);
             else hsL = half_g * (hL - hc) * (hL + hc);
             gl1 = lx + hsL * nx; gl2 = ly + hsL * ny;
             if (n >= 0) {
-                const float rx_ = dr1 * nx - dr2 * ny, ry_ = dr1 * ny + dr2 * nx;
+                const float rx_ = diff2(dr1, nx, dr2, ny), ry_ = dot2(dr1, ny, dr2, nx);
                 float hsR;
                 if (hn > dry) hsR = (rn.flags & 1) ? 0.f : half_g * hydro_perturbation(R.dh, hR, hn, R.raw, R.db);
                 else hsR = half_g * (hR - hn) * (hR + hn);
