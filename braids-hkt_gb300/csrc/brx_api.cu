@@ -1812,7 +1812,9 @@ static void begin_interval(brx_solver *s, double dt, double time, bool fixed)
 // changed since the last call).
 static void refresh_bed(brx_solver *s)
 {
-    if (s->precision == BRX_MIXED) s->launches += mixed_kernel(make_launch(s, s->stream), K_BED, 0, nullptr);
+    if (s->precision == BRX_MIXED)
+        s->launches += s->method == BRX_METHOD_HLLC ? mixed_hllc_kernel(make_launch(s, s->stream), KH_BED)
+                                                    : mixed_kernel(make_launch(s, s->stream), K_BED, 0, nullptr);
     // the HLLC method limits its bed gradient with its own rule
     if (s->small64 && s->method == BRX_METHOD_FWAVE) {
         if (s->maxdeg <= 3) k64_bed<3><<<s->grid_c, 128, 0, s->stream>>>(s->mesh, s->c64, s->state.z);

@@ -83,6 +83,28 @@ __device__ __forceinline__ void hllc_riemann_f(float hl, float ul, float vl, flo
 }
 
 // ---------------------------------------------------------------------------
+// Bed-derived tables of the method, once per call (the bed may change between
+// calls): bed of the other cell of an entry and of a face less the own. The
+// f-wave method's tables (its entries and its limited bed gradient) are not formed
+// for it: 16 us at 450k cells, and 27 us less a call.
+// ---------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) km_hllc_bed(MeshDev m, StateDev s, MixedGeo g)
+{
+    const int stride = gridDim.x * blockDim.x, first = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int f = first; f < m.nf; f += stride) {
+        const int o = m.neighbour[f];
+        g.fdb[f] = o >= 0 ? float(s.z[o] - s.z[m.owner[f]]) : 0.f;
+    }
+    for (int c = first; c < m.nc; c += stride) {
+        const double zc = s.z[c];
+        for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
+            const int o = g.hent[k].y;
+            g.hcdb[k] = o >= 0 ? float(s.z[o] - zc) : 0.f;
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------
 // Cells: limited MUSCL gradients over the neighbours and mirrored walls (open
 // faces take no part), the half-step predictor; the predicted conserved
 // state in q1 (FP64) for the exterior owner at t + dt/2.

@@ -56,7 +56,7 @@ struct TileDev {
 };
 // HLLC kinds of one substep (their launch-shape slots), shared by both forms.
 enum HllcKind { KH_CELLS = 20, KH_PREDICT = 21, KH_BOUNDARY = 22, KH_FACES = 23, KH_BUDGET = 24, KH_TURB = 25,
-                KH_UPDATE = 26, KH_TURB0 = 27 };
+                KH_UPDATE = 26, KH_TURB0 = 27, KH_BED = 28 };
 
 // Launch shape of one kernel kind: threads per block and the grid cap in
 // resident blocks per SM (grid = min(ceil(n / block), per_sm * SMs); the

@@ -280,7 +280,8 @@ __device__ __forceinline__ void slabs_project(const Slabs<N> &S, float &x, float
 }
 
 // ---------------------------------------------------------------------------
-// Bed-derived tables (once per call: the bed may change between calls)
+// Bed-derived tables of the f-wave method (once per call: the bed may change
+// between calls); the HLLC method's are km_hllc_bed's
 // ---------------------------------------------------------------------------
 template <int MAXF>
 __global__ void __launch_bounds__(128) km_bed(MeshDev m, StateDev s, MixedGeo g)
@@ -306,11 +307,6 @@ __global__ void __launch_bounds__(128) km_bed(MeshDev m, StateDev s, MixedGeo g)
             }
             g.cdb[k] = d;
         }
-        if (g.hent)          // the HLLC incidence (faces ascending per cell)
-            for (int k = k0; k < k0 + deg; ++k) {
-                const int o = g.hent[k].y;
-                g.hcdb[k] = o >= 0 ? float(s.z[o] - zc) : 0.f;
-            }
         float2 gb = make_float2(0.f, 0.f);
         const float4 inv = g.cinv[c];
         if (inv.x != 0.f || inv.y != 0.f || inv.z != 0.f) {
@@ -1530,6 +1526,9 @@ int mixed_hllc_kernel(const Launch &L, int kind)
     brx_mx::HCellF *rec = reinterpret_cast<brx_mx::HCellF *>(L.work.rec);
 #define SHAPE(kind_, n_) shape_grid(L, kind_, n_), L.shape[kind_].block
     switch (kind) {
+    case KH_BED:
+        brx_mx::km_hllc_bed<<<std::max(L.grid_c256, L.grid_f256), 256, 0, st>>>(L.mesh, L.state, L.mx);
+        return 1;
     case KH_CELLS:
         brx_mx::km_hllc_cells<<<SHAPE(KH_CELLS, nc), 0, st>>>(L.mesh, L.state, L.ctrl, L.mx, rec);
         return 1;
@@ -1614,7 +1613,8 @@ int mixed_kernel(const Launch &L, int kind, int stage, double *out)
         return 1;
     case K_BED: {
         const int grid = L.grid_c > L.grid_f ? L.grid_c : L.grid_f;
-        if (small) brx_mx::km_bed<4><<<grid, 128, 0, st>>>(L.mesh, L.state, L.mx);
+        if (L.maxdeg <= 3) brx_mx::km_bed<3><<<grid, 128, 0, st>>>(L.mesh, L.state, L.mx);
+        else if (small) brx_mx::km_bed<4><<<grid, 128, 0, st>>>(L.mesh, L.state, L.mx);
         else brx_mx::km_bed<MAX_CELL_FACES><<<grid, 128, 0, st>>>(L.mesh, L.state, L.mx);
         return 1;
     }

@@ -66,3 +66,20 @@ def test_wall_reflection_matches_fp64(froude):
     a, b = rates
     scale = np.abs(a[1:]).max()
     assert scale > 0 and np.abs(b[1:] - a[1:]).max() <= 1e-4 * scale
+
+
+def test_method_switch_forms_its_bed_tables():
+    """Each method forms its own bed tables: a solver switched between the methods
+    with the bed changed in between gives the bits of one made for the method."""
+    from braids_hkt_gb300.solver import METHODS, RiverSolver, check
+    case = S.small_channel()
+    q = S.perturbed_state(case, 3)
+    s = RiverSolver(case, precision="mixed", method="hllc")
+    for k, method in enumerate(["hllc", "fwave", "hllc", "fwave"]):
+        check(s.lib.brx_method_set(s.h, METHODS[method]))
+        alone = RiverSolver(case, precision="mixed", method=method)
+        for t in (s, alone):
+            t.set_state(q)
+            t.z.copy_(t.torch.from_numpy(case["z"] * (1. + .1 * k)))
+            t.substep(0.02, 0.0)
+        np.testing.assert_array_equal(s.state(), alone.state())
