@@ -32,20 +32,17 @@ sys.path.insert(0, os.path.join(ROOT, "oracle"))
 METRIC = "cell-updates/s"
 BYTES_PER_CELL_UPDATE = {"fp64": 680.0, "mixed": 384.0}   # algorithmic bytes, two-sweep design
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one
-# launch of each mixed-form sweep, each kernel captured alone (ncu --set full,
-# one launch) on the 24-scenario subset with rotors (scenarios 20..43 sorted
-# by size, 1,967,962 cells, inputs larger than L2): a launch of the full batch
-# is scaled by its cells
-TRAFFIC_BYTES_PER_CELL = {"mixed": {"cells": 244.21, "faces": 213.25, "gather": 145.97, "update": 190.15,
-                                    "drag": 63.07}}
-KERNEL_NAMES = ["drag", "boundary", "cells", "faces", "gather", "update", "control"]
+# launch of each mixed-form sweep, each kernel captured alone (ncu, one launch)
+# on a channel of 899,304 triangles without rotors (inputs larger than L2): a
+# launch of the full batch is scaled by its cells
+TRAFFIC_BYTES_PER_CELL = {"mixed": {"cells": 186.4, "faces": 152.9, "update": 225.9, "drag": 38.2}}
+KERNEL_NAMES = ["drag", "boundary", "cells", "faces", "update", "control"]
 # FP64 flops (2 DFMA + DMUL + DADD thread instructions) per cell (per face for
-# the face sweep) of one launch of each FP64-form sweep, each kernel captured
-# alone on config 1 (ncu, one launch from the initial state), and their sum
-# over one substep per cell-update
-FP64_FLOPS = {"cells": ("cell", 995.0), "faces": ("face", 1190.0), "gather": ("cell", 97.0),
-              "update": ("cell", 89.0), "drag": ("cell", 259.0)}
-FP64_FLOPS_PER_CELL_UPDATE = 6220.0
+# the face sweep) of one launch of each FP64-form sweep (the update: the mean of
+# the two stages), each kernel captured alone on a 50k-cell channel (ncu, one
+# trial), and their sum over one substep per cell-update
+FP64_FLOPS = {"cells": ("cell", 169.0), "faces": ("face", 379.0), "update": ("cell", 137.0), "drag": ("cell", 143.0)}
+FP64_FLOPS_PER_CELL_UPDATE = 1900.0
 
 
 def peaks():
@@ -186,11 +183,9 @@ def algorithmic_bytes(kernel, nc, nf, nadj, nslot, precision="fp64", rotor_cells
             # in the cell sweep above: triangles)
             return (nc * 64 + nf * (2 * i4 + i4 + i4 + 8 + 16 + 8) + nf * (8 + 16) +
                     rotor_cells * (2 * 4 + 1) + rotor_faces * (16 + 8))
-        if kernel == "gather":   # id, CSR, record flags, stock, rate/theta out; per entry weight; face fluxes
-            return nc * (i4 + i4 + 4 + d8 + 3 * d8 + d8 + i4) + nadj * (i4 + d8) + nf * (8 + 16)
-        if kernel == "update":    # id, CSR, rate, stage states in/out, primitives out, donor factors; per
-            # entry face id, FP64 and FP32 weights, other cell + flags; per face the FP32 water
-            return nc * (i4 + i4 + 2 * 4 + 3 * d8 + 3 * d8 + d8 + 32 + 4) + nadj * (i4 + d8 + 4 + 8) + nf * 8
+        if kernel == "update":    # id, CSR, record depth and flags, open-face flag, stage states in/out, bed, primitives
+            # out, donor factor; per entry face id, FP64 and FP32 weights; per face water, speed and momentum fluxes
+            return nc * (i4 + i4 + 8 + i4 + 3 * d8 + 3 * d8 + d8 + 32 + 4) + nadj * (i4 + d8 + 4) + nf * (8 + 16)
         if kernel == "drag":
             return nc * (i4 + 6 * d8)
         return 0
@@ -199,12 +194,10 @@ def algorithmic_bytes(kernel, nc, nf, nadj, nslot, precision="fp64", rotor_cells
     if kernel == "cells":
         return (nc * (3 * d8 + d8 + i4 + i4 + 4 * d8 + 128) + nadj * (2 * i4 + 3 * d8) +
                 nf * (3 * i4 + 2 * d8 + 2 * 2 * d8 + 2 * 2 * d8 + 2 * d8) + 3 * nc * d8)
-    if kernel == "gather":
-        return nc * (i4 + d8 + 128 // 8 + 3 * d8 + d8 + i4 + i4) + nadj * 2 * i4 + nf * (d8 + 16 + 32) + nc * 3 * d8
     if kernel == "limit":
         return nf * (16 + 2 * i4 + i4 + i4 + 32) + nc * (d8 + 3 * d8)
-    if kernel == "update":
-        return nc * (i4 + d8 + 3 * d8 + 3 * d8 + 3 * d8 + 3 * d8 + i4) + nadj * 2 * i4 + nf * (d8 + 32)
+    if kernel == "update":        # as the mixed form's, in FP64
+        return nc * (2 * i4 + 32 + i4 + 3 * d8 + 3 * d8 + d8 + 32 + d8) + nadj * (i4 + d8) + nf * (16 + 32)
     if kernel == "drag":
         return nc * (i4 + 6 * d8)
     return 0
@@ -305,7 +298,7 @@ def fp64_roofline(per_kind, nc, nf, value, peak_tflops):
     step = value * FP64_FLOPS_PER_CELL_UPDATE / 1e12
     return {"bound": "fp64", "kernel": f"k_{dom}", "achieved": achieved, "peak": peak_tflops, "unit": "TFLOP/s",
             "frac": achieved / peak_tflops, "kernel_ms": ms, "flops_per_launch": flops,
-            "flops_source": f"ncu FP64 thread-instruction counts per {unit} of a config-1 capture, scaled",
+            "flops_source": f"ncu FP64 thread-instruction counts per {unit} of a 50k-cell channel capture, scaled",
             "peak_source": "brx_fma_rate (measured FP64 FMA rate of this GPU)",
             "step_flops_per_cell_update": FP64_FLOPS_PER_CELL_UPDATE, "step_achieved_tflops": step,
             "step_frac": step / peak_tflops}
@@ -603,7 +596,7 @@ def main():
     total_ms = sum(sum(v) for v in per_kind.values())
     roofline = {"bound": "hbm", "kernel": f"k_{dom}", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic,
-                "traffic_source": ("ncu DRAM bytes per cell of a 24-scenario subset capture, scaled by cells"
+                "traffic_source": ("ncu DRAM bytes per cell of a 900k-cell channel capture, scaled by cells"
                                    if traffic is not None else None),
                 "peak_source": peak_kind,
                 "kernel_ms": dom_ms, "kernel_share_of_substep": sum(per_kind[dom]) / total_ms,
@@ -778,7 +771,7 @@ def main():
                                   "unit": "TFLOP/s",
                                   "frac": plain["value"] * FP64_FLOPS_PER_CELL_UPDATE / 1e12 / fp64_peak,
                                   "step_flops_per_cell_update": FP64_FLOPS_PER_CELL_UPDATE,
-                                  "flops_source": "ncu FP64 thread-instruction counts per cell-update of config 1"}
+                                  "flops_source": "ncu FP64 thread-instruction counts per cell-update of a 50k-cell channel"}
         line["roofline_fp64"] = dict(plain["roofline_fp64"], leg="plain_fp64")
     if chained is not None:
         line["chained"] = chained

@@ -40,7 +40,8 @@ import numpy as np
 from .build import BUILD
 
 # tunable kernel kinds (brx_profile_substep kinds) per method; the rotor
-# gradient / face kernels (12, 13) are timed inside the rotor group (11)
+# gradient / face kernels (12, 13) are timed inside the rotor group (11); the
+# gather (4) runs inside the update and is skipped as a kind that did not run
 KINDS = {
     "fwave": {0: "drag", 2: "cells", 3: "faces", 4: "gather", 6: "update", 11: "rotors"},
     "hllc": {0: "drag", 20: "hllc_cells", 21: "hllc_predict", 23: "hllc_faces", 24: "hllc_budget",

@@ -1,7 +1,7 @@
 // Types and device helpers shared by both arithmetic forms of the river step.
 //
-// One substep = drag(dt/2) -> 2 x [boundary -> cells -> faces -> gather ->
-// limit -> update] -> control. Every kernel is batch-aware: cells and faces
+// One substep = drag(dt/2) -> 2 x [boundary -> cells -> faces -> update with the
+// gather -> the limited cells again] -> control. Every kernel is batch-aware: cells and faces
 // of many scenarios are packed into one index space, each element carries
 // its scenario id, and each scenario owns a Ctrl block on the device that
 // holds its clock (trial dt, elapsed time, hint) and its rejection status.

@@ -394,8 +394,8 @@ int brx_hint_set(brx_solver *s, const double *hint);
 int brx_graph_chunk_set(brx_solver *s, int substeps);
 
 /* Launch shape of one kernel kind (the kinds of brx_profile_substep: 0 drag,
- * 2 cells, 3 faces, 4 gather, 5 limit, 6 update, 12 / 13 rotor gradients /
- * face terms, 15 the mixed tile sweep (block fixed at 256, one tile per block
+ * 2 cells, 3 faces, 5 limit, 6 update, 12 / 13 rotor gradients / ambient
+ * stress, 15 the mixed tile sweep (block fixed at 256, one tile per block
  * and grid-stride step); HLLC 20 cells, 21 predictor, 23 faces, 24 budget,
  * 26 update):
  * threads per block (a multiple of 32 up to the kernel's limit) and the grid
@@ -408,8 +408,8 @@ int brx_launch_shape_get(brx_solver *s, int kind, int *block, int *blocks_per_sm
 /* Time one SSPRK(2,2) trial of exactly dt kernel by kernel with CUDA events
  * on the solver stream (no graph). ms (cap entries) gets each launch's
  * duration and kind (cap entries) its kernel: 0 drag, 1 boundary, 2 cells,
- * 3 faces, 4 gather, 5 limit, 6 update, 7 control, 11 rotor terms (four
- * kernels timed together); for BRX_METHOD_HLLC 20 cells, 21 predictor
+ * 3 faces, 6 update (gather, update and the limited cells again, timed
+ * together), 7 control, 11 rotor terms (timed together); for BRX_METHOD_HLLC 20 cells, 21 predictor
  * source, 22 boundary, 23 faces, 24 budget, 25 rotor terms at the predicted
  * state, 26 update, 27 rotor terms at the start state. *count gets the number
  * of launches. The bound state is advanced as by brx_substep. */
