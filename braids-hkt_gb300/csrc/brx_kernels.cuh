@@ -30,6 +30,14 @@ __device__ __forceinline__ F chezy(int method, F depth, F value)
     return F(18.) * log10(F(12.) * fmax(F(.5), depth / value));
 }
 
+// The drag factor by plain divisions, for a momentum whose square is infinite
+// (factor 0: the cell stops) or not a number: quotient() of those is not one.
+static __device__ __noinline__ double drag_factor_far(double square, double h, double dt, double g, double stiff)
+{
+    const double speed = sqrt(square) / h;
+    return 1. / (1. + dt * g * speed / stiff);
+}
+
 // The depth's sixth root of Manning's law is cbrt(sqrt(h)) (25 FP64
 // instructions, good to about one ulp) instead of pow (88, two ulp), and the
 // quotients go through quotient(), correctly rounded as the divisions they
@@ -42,9 +50,13 @@ __device__ __forceinline__ void drag_cell(const Ctrl &ct, double dt, double &h, 
     if (!greater(h, ct.dry)) { hu = 0.; hv = 0.; return; }
     const double c = ct.roughness_mode == 2 ? quotient(cbrt(sqrt(h)), ct.roughness_value, ct.rrough)
                                             : chezy<double>(ct.roughness_mode, h, ct.roughness_value);
-    const double speed = quotient(sqrt(hu * hu + hv * hv), h, reciprocal(h)), stiff = c * c * h;
-    const double y = 1. + quotient(dt * ct.grav * speed, stiff, reciprocal(stiff));
-    const double factor = quotient(1., y, reciprocal(y));
+    const double square = hu * hu + hv * hv, stiff = c * c * h;
+    double factor;
+    if (finite_bits(square)) {
+        const double speed = quotient(sqrt(square), h, reciprocal(h));
+        const double y = 1. + quotient(dt * ct.grav * speed, stiff, reciprocal(stiff));
+        factor = quotient(1., y, reciprocal(y));
+    } else factor = drag_factor_far(square, h, dt, ct.grav, stiff);
     hu *= factor;
     hv *= factor;
 }

@@ -67,3 +67,23 @@ def test_residual_equals_the_general_sweep_bit_for_bit(name):
         assert (status, freq) == (st.value, fr.value)
         np.testing.assert_array_equal(rate.cpu().numpy(), rate2.cpu().numpy())
         np.testing.assert_array_equal(water.cpu().numpy(), water2.cpu().numpy())
+
+
+@pytest.mark.parametrize("momentum", [1e140, 1e160, 1e200, 1e300])
+def test_drag_of_a_momentum_whose_square_overflows(momentum):
+    """A wet cell's momentum whose square is infinite: the drag's factor is zero
+    and the trial accepted, as in the oracle; one below that is refused by both.
+    The same steps of FP64 arithmetic: 1e-12 of each row's largest value."""
+    from braids_hkt_gb300.solver import RiverSolver
+    from oracle import Oracle
+    case = S.small_channel()
+    q = case["q"].copy()
+    q[1, case["mesh"].nc // 2] = momentum
+    s = RiverSolver(case, precision="fp64")
+    s.set_state(q)
+    status, _ = s.substep(0.004, 0.0)
+    code, _, _ = Oracle(case, threads=4).advance(q, 0.004, 0.0)
+    assert (status == 0) == (code == 0) == (momentum > 1e154)
+    if code == 0:
+        scale = np.abs(q).max(axis=1, keepdims=True)
+        assert (np.abs(s.state() - q) / scale).max() <= 1e-12
