@@ -54,6 +54,20 @@ static_assert(sizeof(HCell) == 96, "HLLC cell record is three 32-byte sectors");
 
 __device__ __forceinline__ int hent_face(int x) { return x >= 0 ? x : ~x; }
 
+// Signal speed of a face with a nonfinite state: extrema that pass over a NaN,
+// as the integer ones do not. The state fails its trial by the cell sweep's
+// infinite peak; a NaN frequency would be halved away step by step instead.
+static __device__ __noinline__ double nonfinite_speed(double etal, double bl, double ul, double etar, double br,
+                                                      double ur, double g, double dry)
+{
+    const double top = fmax(bl, br), hl = fmax(0., etal - top), hr = fmax(0., etar - top);
+    const double cl = sqrt(g * hl), cr = sqrt(g * hr);
+    double sl = fmin(ul - cl, ur - cr), sr = fmax(ul + cl, ur + cr);
+    if (hl <= dry) sl = ur - 2. * cr;
+    if (hr <= dry) sr = ul + 2. * cl;
+    return hl <= dry && hr <= dry ? 0. : fmax(fabs(sl), fabs(sr));
+}
+
 // hllc.h:52-72: HLLC flux of one rotated face; HLLE where a side is dry or
 // the contact state is inadmissible.
 __device__ __forceinline__ void hllc_riemann(double hl, double ul, double vl, double hr, double ur, double vr,
@@ -184,11 +198,11 @@ __global__ void __launch_bounds__(128) k_hllc_cells(MeshDev m, StateDev s, HllcD
         double eta = cv[0] - .5 * dt * (u * (r.g[0] - r.g[6]) + w * (r.g[1] - r.g[7]) + hc * (r.g[2] + r.g[5]));
         double uh = u - .5 * dt * (u * r.g[2] + w * r.g[3] + g * r.g[0]);
         double wh = w - .5 * dt * (u * r.g[4] + w * r.g[5] + g * r.g[1]);
-        if (greater(cv[3], eta)) { eta = cv[0]; uh = u; wh = w; }
+        if (eta < cv[3]) { eta = cv[0]; uh = u; wh = w; }          // false for a NaN, of either sign
         if (shallow) { eta = cv[0]; uh = 0.; wh = 0.; }
         r.p[0] = eta; r.p[1] = uh; r.p[2] = wh; r.p[3] = cv[3];
         rec[c] = r;
-        const double rise = eta - cv[3], hh = greater(rise, 0.) ? rise : 0.;
+        const double rise = eta - cv[3], hh = rise > 0. ? rise : 0.;
         s.q1[c] = hh; s.q1[nc + c] = hh * uh; s.q1[2 * nc + c] = hh * wh;
         if (!finite_bits(eta) || !finite_bits(uh) || !finite_bits(wh)) atomic_max_nonneg(&ct.peak1, INFINITY);
     }
@@ -291,6 +305,8 @@ __global__ void __launch_bounds__(128) k_hllc_faces(MeshDev m, BoundaryDev b, co
         double out[3], speed;
         hllc_riemann(hls, L[1] * nx + L[2] * ny, -L[1] * ny + L[2] * nx, hrs, R[1] * nx + R[2] * ny,
                      -R[1] * ny + R[2] * nx, g, dry, out, speed);
+        if (!finite_bits(speed))
+            speed = nonfinite_speed(L[0], L[3], L[1] * nx + L[2] * ny, R[0], R[3], R[1] * nx + R[2] * ny, g, dry);
         const double el = positive(rl.p[0] - L[3]), er = r < 0 ? el : positive(rr.p[0] - R[3]);
         const double pl = .5 * g * (hl * hl - hls * hls - el * el), pr = .5 * g * (hr * hr - hrs * hrs - er * er);
         double l1 = (out[1] + pl) * nx - out[2] * ny, l2 = (out[1] + pl) * ny + out[2] * nx;

@@ -87,3 +87,20 @@ def test_drag_of_a_momentum_whose_square_overflows(momentum):
     if code == 0:
         scale = np.abs(q).max(axis=1, keepdims=True)
         assert (np.abs(s.state() - q) / scale).max() <= 1e-12
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("row", [0, 1])
+def test_hllc_ends_a_nonfinite_state_at_its_first_trial(row, value):
+    """A nonfinite state gives an infinite CFL peak: the trial is rejected with a
+    zero hint and the interval fails, not after halving down to the floor."""
+    from braids_hkt_gb300.solver import RiverSolver
+    if row == 0 and value == -np.inf:
+        pytest.skip("a negative depth is refused by its own status")
+    case = S.small_channel()
+    q = case["q"].copy()
+    q[row, case["mesh"].nc // 2] = value
+    s = RiverSolver(case, precision="fp64", method="hllc")
+    s.set_state(q)
+    d = s.advance(0.05, 0.0, raise_on_failure=False)
+    assert (d["failed"], d["hydraulic_substeps"], d["hydraulic_rejections"]) == (1, 0, 1)
