@@ -43,7 +43,13 @@ def _f64(a):
 
 
 def _ptr(a):
-    return C.c_void_p(a.ctypes.data) if a is not None else None
+    """Address of an array for a library call; holds the array, so that a
+    temporary outlives the call it is passed to."""
+    if a is None:
+        return None
+    p = C.c_void_p(a.ctypes.data)
+    p.array = a
+    return p
 
 
 def rating_tables(cases):
