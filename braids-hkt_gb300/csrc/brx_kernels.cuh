@@ -495,11 +495,24 @@ __device__ __forceinline__ void lane_sums(SectionWork &w, int n, double (&sum)[R
     for (int r = 0; r < ROWS; ++r) sum[r] = w.sum[r];
 }
 
-// Shrink [lo, hi], f(lo) >= 0 >= f(hi) and f decreasing, to neighbouring
-// numbers, where bisection ends. Each round evaluates the secant point and then
-// twice the distance it is still off, which as a rule is just across the root:
-// the width falls with the square, some twelve evaluations instead of
-// bisection's fifty-odd. A round that does not halve the interval bisects.
+// Bisect [lo, hi], f(lo) >= 0 >= f(hi), to neighbouring numbers. Where f has
+// several roots the one found depends on the points tried: these are the
+// reference's.
+template <class Fn>
+__device__ __forceinline__ void bisect_bracket(double &lo, double &hi, const Fn &f)
+{
+    for (int j = 0; j < 90; ++j) {
+        const double mid = lo + .5 * (hi - lo);
+        if (mid == lo || mid == hi) return;
+        if (f(mid) > 0.) lo = mid; else hi = mid;
+    }
+}
+
+// The same end for an f that decreases throughout, and so has one root. Each
+// round evaluates the secant point and then twice the distance it is still
+// off, which as a rule is just across the root: the width falls with the
+// square, some twelve evaluations instead of bisection's fifty-odd. A round
+// that does not halve the interval bisects.
 template <class Fn>
 __device__ __forceinline__ void shrink_bracket(double &lo, double &hi, double flo, double fhi, const Fn &f)
 {
@@ -570,6 +583,7 @@ __device__ __noinline__ int weir_section(SectionWork &w, const MeshDev &m, const
     // wet faces, each with its incoming normal speed; the bracket of the stage
     // from their sonic depths and their own levels (maxima: in any order)
     double lo = -INFINITY, hi = -INFINITY;
+    double highest = -INFINITY;              // bed of the wet faces
     bool some = false;
     for (int k = k0 + threadIdx.x; k < k1; k += blockDim.x) {
         const int f = b.slot_face[k], c = m.owner[f];
@@ -585,6 +599,7 @@ __device__ __noinline__ int weir_section(SectionWork &w, const MeshDev &m, const
         shrink_bracket(left, right, f_sonic(left), f_sonic(right), f_sonic);
         lo = fmax(lo, b.ext_bed[k] + right);
         hi = fmax(hi, hc + z[c]);
+        highest = fmax(highest, b.ext_bed[k]);
     }
     double eta = 0.;
     if (__syncthreads_or(some)) {
@@ -610,7 +625,13 @@ __device__ __noinline__ int weir_section(SectionWork &w, const MeshDev &m, const
             if (rhi > 0. || !isfinite(rhi)) error = 1;
         }
         if (!error) {
-            shrink_bracket(lo, hi, rlo, rhi, residual);
+            // Above every face's sonic stage its discharge falls with the stage,
+            // unless the face is not deeper than the dry depth there: its
+            // discharge then sets in at a jump within the bracket, and there may
+            // be a root on either side.
+            if (__syncthreads_or(some && highest + dry * (1. + 1.e-9) + 4. * EPS * fabs(highest) >= lo))
+                bisect_bracket(lo, hi, residual);
+            else shrink_bracket(lo, hi, rlo, rhi, residual);
             eta = lo + .5 * (hi - lo);
             const double r = residual(eta), head = fmax(eta - crest, 0.), requested = factor * head * sqrt(head);
             if (!isfinite(r) || fabs(r) > 1e-10 * fmax(requested, 1.)) error = 2;
@@ -770,7 +791,9 @@ __device__ int crit_group(SectionWork &w, const MeshDev &m, const BoundaryDev &b
         double rhi = residual(hi);
         for (int j = 0; j < 60 && rhi > 0.; ++j) { hi = lo + 2. * (hi - lo); rhi = residual(hi); }
         if (rhi > 0. || !isfinite(rhi)) { error = 1; break; }
-        shrink_bracket(lo, hi, rlo, rhi, residual);
+        // several roots on an uneven bed: a face's discharge rises with the stage
+        // before it falls, and the critical discharge drops where a face wets
+        bisect_bracket(lo, hi, residual);
         eta = lo + .5 * (hi - lo);
         bool changed = false;
         for (int i = threadIdx.x; i < n; i += blockDim.x) {
