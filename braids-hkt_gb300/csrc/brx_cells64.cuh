@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(128, 4) k64_cells(MeshDev m, StateDev s, Ctrl 
         for (int j = 0; j < D; ++j) id[j] = j < deg ? g.cidx[k0 + j] : make_int2(-1, 0);
         const Prim64 p = P[c];
         const double dry = ct.dry, zc = s.z[c];
-        if (__double_as_longlong(p.h) < 0 ? p.h != 0. : false) raise_status(ct, stage, ST_SPATIAL);
+        if (negative(p.h)) raise_status(ct, stage, ST_SPATIAL);
         if (!finite_bits(p.h) || !finite_bits(p.eta) || !finite_bits(p.u) || !finite_bits(p.v))
             raise_status(ct, stage, ST_SPATIAL);
         const bool wet = greater(p.h, dry), outlet = g.ccls[c] & 1;

@@ -409,7 +409,7 @@ __global__ void __launch_bounds__(256) k_hllc_update(MeshDev m, StateDev s, Hllc
             v2 -= a * (sign > 0 ? l2 : r2);
         }
         if (!greater(v0, dry)) { v1 = 0.; v2 = 0.; }
-        bad = bad || !finite_bits(v0) || !finite_bits(v1) || !finite_bits(v2) || greater(0., v0);
+        bad = bad || !finite_bits(v0) || !finite_bits(v1) || !finite_bits(v2) || negative(v0);
         if (turb && t.hkt[sid]) {
             double r1 = 0., r2 = 0.;
             add_rotor_momentum(m, t, sid, c, area, r1, r2, false, rarea);

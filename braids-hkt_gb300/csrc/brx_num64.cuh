@@ -22,6 +22,12 @@ __device__ __forceinline__ double unordered(long long k)
 // |x| as an integer that orders like |x|
 __device__ __forceinline__ long long magnitude(double x) { return __double_as_longlong(x) & 0x7fffffffffffffffLL; }
 __device__ __forceinline__ bool greater(double a, double b) { return ordered(a) > ordered(b); }
+// x < 0, false for -0 (which greater() orders below 0) and for a NaN
+__device__ __forceinline__ bool negative(double x)
+{
+    const unsigned long long b = __double_as_longlong(x);
+    return b > 0x8000000000000000ull && b <= 0xfff0000000000000ull;
+}
 __device__ __forceinline__ bool finite_bits(double x)
 {
     return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;

@@ -56,7 +56,7 @@ __device__ __forceinline__ void finish_cell(const MeshDev &m, const StateDev &s,
     if (stage == 1) {
         const double h = s.work[c] + dt * r0;
         double hu = s.work[nc + c] + dt * r1, hv = s.work[2 * nc + c] + dt * r2;
-        if (!quiet && greater(0., h)) raise_status(ct, 1, ST_ENDPOINT);
+        if (!quiet && negative(h)) raise_status(ct, 1, ST_ENDPOINT);
         if (!greater(h, dry)) { hu = 0.; hv = 0.; }
         s.q1[c] = h; s.q1[nc + c] = hu; s.q1[2 * nc + c] = hv;
         if (prim) put_prim64(prim, c, h, hu, hv, s.z[c], dry);       // the second stage's
@@ -64,7 +64,7 @@ __device__ __forceinline__ void finish_cell(const MeshDev &m, const StateDev &s,
         double h = .5 * s.work[c] + .5 * (s.q1[c] + dt * r0);
         double hu = .5 * s.work[nc + c] + .5 * (s.q1[nc + c] + dt * r1);
         double hv = .5 * s.work[2 * nc + c] + .5 * (s.q1[2 * nc + c] + dt * r2);
-        if (!quiet && (!finite_bits(h) || !finite_bits(hu) || !finite_bits(hv) || greater(0., h)))
+        if (!quiet && (!finite_bits(h) || !finite_bits(hu) || !finite_bits(hv) || negative(h)))
             raise_status(ct, 2, ST_ENDPOINT);
         if (!greater(h, dry)) { hu = 0.; hv = 0.; }
         drag_cell(ct, .5 * dt, h, hu, hv);
@@ -123,8 +123,9 @@ __global__ void __launch_bounds__(256) k64_update(MeshDev m, StateDev s, Ctrl *c
                 if (isnan(fr)) raise_status(ct, stage, ST_FREQ);
                 else have = true;
                 const bool active = w.rec[c].flags & 2;
-                finish_cell(m, s, ct, w, stage, sid, c, -sum0, active ? -sum1 : 0., active ? -sum2 : 0., rate_out, t, turb,
-                            prim, limits);
+                // (0 - 0 is 0: the rate of a cell at rest has no sign)
+                finish_cell(m, s, ct, w, stage, sid, c, 0. - sum0, active ? -sum1 : 0., active ? -sum2 : 0., rate_out, t,
+                            turb, prim, limits);
             }
         }
         unsigned long long *peak0 = stage == 1 ? &ctrl[0].peak1 : &ctrl[0].peak2;
