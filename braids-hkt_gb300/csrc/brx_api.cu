@@ -104,15 +104,15 @@ struct brx_solver {
     double *d_tdiag_out = nullptr;   // (nrotor, 16) diagnostics of brx_turbines_diagnose
     ExnerDev exner{};                // bed model (valid when has_exner)
     bool has_exner = false;
-    int exner_widest = 0;            // most chunks of one scenario
+    int exner_chunks = 0;            // of all scenarios
     int *d_cell_off = nullptr, *d_face_off = nullptr;
     double *d_exdt = nullptr;
     double *d_totals = nullptr;      // (nscen, 3) sums, (nscen, 2) gravity and dry depth
     double *h_totals = nullptr;      // (nscen, 3) pinned
-    int *d_totals_first = nullptr;   // (nscen+1) first block of each scenario
+    int *d_totals_first = nullptr, *d_totals_sid = nullptr;   // (nscen+1) first block of each scenario, (blocks) its scenario
     Pair *d_totals_part = nullptr;   // (blocks, 3) partial sums
     unsigned *d_totals_tickets = nullptr;
-    int totals_widest = 0;           // most blocks of one scenario
+    int totals_blocks = 0;           // of all scenarios
     int tile_cells = 0;              // mixed f-wave: cells per tile of the tile sweep (0: separate sweeps)
     TileDev tiles{};                 // tile tables (valid when tile_smem > 0)
     int tile_smem = 0;
@@ -1348,6 +1348,19 @@ extern "C" int brx_tile_get(const brx_solver *s, int *cells, int *smem_bytes)
 // ---------------------------------------------------------------------------
 // Exner bed update
 // ---------------------------------------------------------------------------
+// Blocks of a sweep that gives every scenario blocks of its own: the first of
+// each scenario (nscen + 1) and the scenario of each; returns their number.
+static int split_scenarios(const brx_solver *s, int (*blocks)(int), std::vector<int> &first, std::vector<int> &sid)
+{
+    first.assign(1, 0);
+    sid.clear();
+    for (int i = 0; i < s->nscen; ++i) {
+        sid.insert(sid.end(), blocks(s->cell_offset[i + 1] - s->cell_offset[i]), i);
+        first.push_back((int)sid.size());
+    }
+    return first.back();
+}
+
 extern "C" int brx_exner_set(brx_solver *s, const int *enabled, const double *param, const int *bedbc,
                              const double *feed, const double *rock, const double *dxdy, const double *inverse,
                              const double *xy)
@@ -1395,16 +1408,12 @@ extern "C" int brx_exner_set(brx_solver *s, const int *enabled, const double *pa
     CK(cudaGetLastError());
     e.enabled = p_en; e.param = p_par; e.bedbc = p_bc; e.feed = p_feed; e.rock = p_rock;
     e.wdxdy = p_dxdy; e.inverse = p_inv; e.xy = p_xy;
-    std::vector<int> first(ns + 1, 0);
-    s->exner_widest = 1;
-    for (int i = 0; i < ns; ++i) {
-        const int blocks = exner_blocks(s->cell_offset[i + 1] - s->cell_offset[i]);
-        first[i + 1] = first[i] + blocks;
-        s->exner_widest = std::max(s->exner_widest, blocks);
-    }
-    int *p_first;
+    std::vector<int> first, chunk_sid;
+    s->exner_chunks = split_scenarios(s, exner_blocks, first, chunk_sid);
+    int *p_first, *p_csid;
     TRY(s->upload(&p_first, first.data(), first.size()));
-    e.first = p_first;
+    TRY(s->upload(&p_csid, chunk_sid.data(), chunk_sid.size()));
+    e.first = p_first; e.chunk_sid = p_csid;
     TRY(s->alloc(&e.part, 3 * (size_t)first[ns])); TRY(s->alloc(&e.tickets, ns)); TRY(s->alloc(&e.out_of_range, ns));
     CK(cudaMemset(e.tickets, 0, sizeof(unsigned) * ns));
     CK(cudaStreamSynchronize(nullptr));
@@ -1441,7 +1450,7 @@ extern "C" int brx_exner(brx_solver *s, const double *dt, double *stats)
     k_ex_cells<<<s->grid_c256, 256, 0, st>>>(s->mesh, e, q, z);
     k_ex_faces<<<s->grid_f, 128, 0, st>>>(s->mesh, e, z);
     k_ex_donor<<<s->grid_c256, 256, 0, st>>>(s->mesh, e, z);
-    k_ex_trial<<<dim3(s->exner_widest, s->nscen), 256, 0, st>>>(s->mesh, e, s->bnd, q, z);
+    k_ex_trial<<<s->exner_chunks, 256, 0, st>>>(s->mesh, e, s->bnd, q, z);
     k_ex_commit<<<s->grid_c256, 256, 0, st>>>(s->mesh, e, z);
     s->launches += 5;
     CK(cudaGetLastError());
@@ -1912,14 +1921,10 @@ extern "C" int brx_advance_poll(brx_solver *s, int *done, brx_advance_stats *sta
 static int ensure_totals(brx_solver *s)
 {
     if (s->d_totals) return BRX_OK;
-    std::vector<int> first(s->nscen + 1, 0);
-    s->totals_widest = 1;
-    for (int i = 0; i < s->nscen; ++i) {
-        const int blocks = totals_blocks(s->cell_offset[i + 1] - s->cell_offset[i]);
-        first[i + 1] = first[i] + blocks;
-        s->totals_widest = std::max(s->totals_widest, blocks);
-    }
+    std::vector<int> first, block_sid;
+    s->totals_blocks = split_scenarios(s, totals_blocks, first, block_sid);
     TRY(s->upload(&s->d_totals_first, first.data(), first.size()));
+    TRY(s->upload(&s->d_totals_sid, block_sid.data(), block_sid.size()));
     TRY(s->alloc(&s->d_totals_part, 3 * (size_t)first[s->nscen]));
     TRY(s->alloc(&s->d_totals_tickets, s->nscen));
     CK(cudaMemset(s->d_totals_tickets, 0, sizeof(unsigned) * s->nscen));
@@ -1937,8 +1942,9 @@ extern "C" int brx_totals(brx_solver *s, double *out)
     double *d = s->d_totals, *gd = s->d_totals + 3 * (size_t)s->nscen;
     for (int i = 0; i < s->nscen; ++i) { s->h_totals[2 * i] = s->h_ctrl[i].grav; s->h_totals[2 * i + 1] = s->h_ctrl[i].dry; }
     CK(cudaMemcpyAsync(gd, s->h_totals, sizeof(double) * 2 * s->nscen, cudaMemcpyHostToDevice, s->stream));
-    k_totals<false><<<dim3(s->totals_widest, s->nscen), 256, 0, s->stream>>>(
-        s->mesh, s->state.q[0], nullptr, s->state.z, gd, s->d_totals_first, s->d_totals_part, s->d_totals_tickets, d);
+    k_totals<false><<<s->totals_blocks, 256, 0, s->stream>>>(s->mesh, s->state.q[0], nullptr, s->state.z, gd,
+                                                             s->d_totals_first, s->d_totals_sid, s->d_totals_part,
+                                                             s->d_totals_tickets, d);
     s->launches++;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(s->h_totals, d, sizeof(double) * 2 * s->nscen, cudaMemcpyDeviceToHost, s->stream));
@@ -1953,9 +1959,9 @@ extern "C" int brx_step_budget(brx_solver *s, const double *start_device, double
     if (!start_device || !out) return fail(BRX_ERR_ARGUMENT, "null argument");
     if (s->pending) return fail(BRX_ERR_STATE, "an asynchronous interval is in flight");
     TRY(ensure_totals(s));
-    k_totals<true><<<dim3(s->totals_widest, s->nscen), 256, 0, s->stream>>>(
-        s->mesh, s->state.q[0], start_device, s->state.z, nullptr, s->d_totals_first, s->d_totals_part,
-        s->d_totals_tickets, s->d_totals);
+    k_totals<true><<<s->totals_blocks, 256, 0, s->stream>>>(s->mesh, s->state.q[0], start_device, s->state.z, nullptr,
+                                                            s->d_totals_first, s->d_totals_sid, s->d_totals_part,
+                                                            s->d_totals_tickets, s->d_totals);
     s->launches++;
     CK(cudaGetLastError());
     CK(cudaMemcpyAsync(s->h_totals, s->d_totals, sizeof(double) * 3 * s->nscen, cudaMemcpyDeviceToHost, s->stream));

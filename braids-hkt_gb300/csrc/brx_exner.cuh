@@ -43,7 +43,7 @@ struct ExnerDev {
     double *ztrial;              // (nc)
     double *stats;               // (nscen, 8)
     double *part;                // (blocks, 3) residual sum, donor minimum, change maximum of a chunk of cells
-    const int *first;            // (nscen+1) first chunk of each scenario
+    const int *first, *chunk_sid;   // (nscen+1) first chunk of each scenario; (chunks) scenario of each
     unsigned *tickets;           // (nscen) zero between calls
     int *wet;                    // (nc)
     int *bad;                    // (nscen) slope operator status
@@ -193,15 +193,14 @@ __global__ void __launch_bounds__(256) k_ex_trial(MeshDev m, ExnerDev e, Boundar
 {
     __shared__ double red[3][256];
     __shared__ bool last;
-    const int sid = blockIdx.y, tid = threadIdx.x;
+    const int sid = e.chunk_sid[blockIdx.x], tid = threadIdx.x;
     if (!e.enabled[sid]) return;
     const int c0 = m.act.cell_off[sid], c1 = m.act.cell_off[sid + 1], blocks = exner_blocks(c1 - c0);
-    if ((int)blockIdx.x >= blocks) return;
     const double *p = e.param + (size_t)sid * EP_N;
     const double dtm = e.dt[sid] * p[EP_MORFAC], phi = 1.0 - p[EP_POROSITY], sd = p[EP_SEDDEPTH], scale = dtm / phi;
     double res = 0., donor = 1., change = 0.;
     bool wrong = false;
-    const int from = c0 + blockIdx.x * EX_CHUNK, to = min(c1, from + EX_CHUNK);
+    const int from = c0 + ((int)blockIdx.x - e.first[sid]) * EX_CHUNK, to = min(c1, from + EX_CHUNK);
     for (int i = from + tid; i < to; i += blockDim.x) {
         double r = 0.;
         for (int k = m.offset[i]; k < m.offset[i + 1]; ++k) {
@@ -227,7 +226,7 @@ __global__ void __launch_bounds__(256) k_ex_trial(MeshDev m, ExnerDev e, Boundar
         __syncthreads();
     }
     if (tid == 0) {
-        double *o = e.part + 3 * (size_t)(e.first[sid] + blockIdx.x);
+        double *o = e.part + 3 * (size_t)blockIdx.x;
         o[0] = red[0][0]; o[1] = red[1][0]; o[2] = red[2][0];
         if (any_wrong) atomicOr(&e.out_of_range[sid], 1);
         __threadfence();

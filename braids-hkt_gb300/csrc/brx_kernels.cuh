@@ -2275,20 +2275,21 @@ __host__ __device__ __forceinline__ int totals_blocks(int cells) { return (cells
 // BUDGET false: water volume sum(A h) and mechanical energy per unit density
 // sum(A (|hu|^2 / (2h) + g h^2 / 2 + g h z)) (kinetic only where h > dry; gd: the
 // scenarios' gravity and dry depth). BUDGET true: volume of the start state q0,
-// volume of q, and the inventory sum(A max(h0, h)). part: (blocks, 3) scratch,
-// blocks of scenario i from first[i]; tickets (nscen) zero, left zero.
+// volume of q, and the inventory sum(A max(h0, h)). One grid dimension over the
+// blocks of all scenarios (a grid's second holds 65,535): block i works for
+// scenario block_sid[i], whose blocks begin at first[]. part: (blocks, 3)
+// scratch; tickets (nscen) zero, left zero.
 template <bool BUDGET>
 __global__ void __launch_bounds__(256) k_totals(MeshDev m, const double *q, const double *q0, const double *z,
-                                                const double *gd, const int *first, Pair *part, unsigned *tickets,
-                                                double *out)
+                                                const double *gd, const int *first, const int *block_sid, Pair *part,
+                                                unsigned *tickets, double *out)
 {
     constexpr int N = BUDGET ? 3 : 2;
     __shared__ Pair warps[N][8];
     __shared__ bool last;
-    const int sid = blockIdx.y, nc = m.nc, c0 = m.act.cell_off[sid], c1 = m.act.cell_off[sid + 1];
-    const int blocks = totals_blocks(c1 - c0);
-    if ((int)blockIdx.x >= blocks) return;
-    const int from = c0 + blockIdx.x * TOTALS_CHUNK, to = min(c1, from + TOTALS_CHUNK);
+    const int sid = block_sid[blockIdx.x], nc = m.nc, c0 = m.act.cell_off[sid], c1 = m.act.cell_off[sid + 1];
+    const int blocks = totals_blocks(c1 - c0), block = blockIdx.x - first[sid];
+    const int from = c0 + block * TOTALS_CHUNK, to = min(c1, from + TOTALS_CHUNK);
     const double g = BUDGET ? 0. : gd[2 * sid], dry = BUDGET ? 0. : gd[2 * sid + 1];
     Pair p[N] = {};
     for (int c = from + threadIdx.x; c < to; c += blockDim.x) {
@@ -2315,7 +2316,7 @@ __global__ void __launch_bounds__(256) k_totals(MeshDev m, const double *q, cons
     if (warp < N) {
         Pair v = lane < 8 ? warps[warp][lane] : Pair{0., 0.};
         merge_warp(v);
-        if (lane == 0) { part[3 * (size_t)(first[sid] + blockIdx.x) + warp] = v; __threadfence(); }
+        if (lane == 0) { part[3 * (size_t)blockIdx.x + warp] = v; __threadfence(); }
     }
     __syncthreads();
     if (threadIdx.x == 0) last = atomicInc(&tickets[sid], blocks - 1) == (unsigned)(blocks - 1);
