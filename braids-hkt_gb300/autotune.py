@@ -22,14 +22,16 @@ restored after every trial, so tuning changes nothing but speed. The chunk is
 then chosen by timing a short fixed interval per candidate, and so is the
 cell tile (the tile sweep waits for the boundary and rotor kernels that the
 separate cell sweep overlaps, so only whole intervals compare them). Choices are cached
-per (device, form, method, cells, faces, scenarios) in a JSON file beside the
-built library, so a solver of the same shape is tuned once.
+per (device, library, form, method, cells, faces, scenarios) in a JSON file
+beside the built library, so a solver of the same shape is tuned once; another
+build of the library has other kernels and is tuned anew.
 
 The reference has no counterpart: its kernels launch with fixed 128-thread
 blocks (src/braids_support/gpu_fwave/reconstruction.py, resident_update.py).
 """
 from __future__ import annotations
 
+import hashlib
 import json
 import os
 import time
@@ -37,11 +39,12 @@ from pathlib import Path
 
 import numpy as np
 
-from .build import BUILD
+from .build import BUILD, LIBRARY
 
 # tunable kernel kinds (brx_profile_substep kinds) per method; the rotor
 # gradient / face kernels (12, 13) are timed inside the rotor group (11); the
 # gather (4) runs inside the update and is skipped as a kind that did not run
+# (its slot is accepted and has no effect)
 KINDS = {
     "fwave": {0: "drag", 2: "cells", 3: "faces", 4: "gather", 6: "update", 11: "rotors"},
     "hllc": {0: "drag", 20: "hllc_cells", 21: "hllc_predict", 23: "hllc_faces", 24: "hllc_budget",
@@ -57,10 +60,15 @@ K_TILE = 15
 CACHE = BUILD / "autotune.json"
 
 
+def _library():
+    """Digest of the built library."""
+    return hashlib.sha256(LIBRARY.read_bytes()).hexdigest()[:16]
+
+
 def _key(solver):
     import torch
     dev = torch.cuda.get_device_name(torch.cuda.current_device())
-    return f"{dev}|{solver.precision}|{solver.method}|{solver.nc}|{solver.nf}|{solver.nscen}"
+    return f"{dev}|{_library()}|{solver.precision}|{solver.method}|{solver.nc}|{solver.nf}|{solver.nscen}"
 
 
 def _members(solver, kind):

@@ -1157,6 +1157,7 @@ static int max_block(const brx_solver *s, int kind)
         break;
     case K_FACES: fn = s->has_turb ? (const void *)k64_faces<true> : (const void *)k64_faces<false>; break;
     case K_LIMIT: fn = (const void *)k_limit; break;
+    case K_GATHER:               // part of the update: the slot is kept, its shape has no effect
     case K_UPDATE: fn = (const void *)k64_update; break;
     case K_HKT_GRAD: fn = (const void *)k_hkt_gradients; break;
     case K_HKT_FACES: fn = (const void *)k_hkt_stress; break;

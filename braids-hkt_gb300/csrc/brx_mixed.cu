@@ -1505,6 +1505,7 @@ int mixed_max_block(int kind, int maxdeg)
         break;
     case K_FACES: fn = (const void *)brx_mx::km_faces; break;
     case K_LIMIT: fn = (const void *)brx_mx::km_limit; break;
+    case K_GATHER:               // part of the update: the slot is kept, its shape has no effect
     case K_UPDATE: fn = (const void *)brx_mx::km_update; break;
     case KH_CELLS: fn = (const void *)brx_mx::km_hllc_cells; break;
     case KH_PREDICT: fn = (const void *)brx_mx::km_hllc_predict; break;

@@ -394,7 +394,8 @@ int brx_hint_set(brx_solver *s, const double *hint);
 int brx_graph_chunk_set(brx_solver *s, int substeps);
 
 /* Launch shape of one kernel kind (the kinds of brx_profile_substep: 0 drag,
- * 2 cells, 3 faces, 5 limit, 6 update, 12 / 13 rotor gradients / ambient
+ * 2 cells, 3 faces, 4 gather (part of the update: accepted, without effect),
+ * 5 limit, 6 update, 12 / 13 rotor gradients / ambient
  * stress, 15 the mixed tile sweep (block fixed at 256, one tile per block
  * and grid-stride step); HLLC 20 cells, 21 predictor, 23 faces, 24 budget,
  * 26 update):
