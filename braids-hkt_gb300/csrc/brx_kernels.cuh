@@ -30,12 +30,15 @@ __device__ __forceinline__ F chezy(int method, F depth, F value)
     return F(18.) * log10(F(12.) * fmax(F(.5), depth / value));
 }
 
-// The drag factor by plain divisions, for a momentum whose square is infinite
-// (factor 0: the cell stops) or not a number: quotient() of those is not one.
-static __device__ __noinline__ double drag_factor_far(double square, double h, double dt, double g, double stiff)
+// The drag factor by plain divisions, where quotient() leaves its domain: a
+// momentum whose square is infinite (factor 0: the cell stops), a roughness whose
+// squared Chezy coefficient is (factor 1: no friction) or vanishes (factor 0).
+static __device__ __noinline__ double drag_factor_far(const Ctrl &ct, double square, double h, double dt)
 {
+    const double c = ct.roughness_mode == 2 ? cbrt(sqrt(h)) / ct.roughness_value
+                                            : chezy<double>(ct.roughness_mode, h, ct.roughness_value);
     const double speed = sqrt(square) / h;
-    return 1. / (1. + dt * g * speed / stiff);
+    return 1. / (1. + dt * ct.grav * speed / (c * c * h));
 }
 
 // The depth's sixth root of Manning's law is cbrt(sqrt(h)) (25 FP64
@@ -51,12 +54,10 @@ __device__ __forceinline__ void drag_cell(const Ctrl &ct, double dt, double &h, 
     const double c = ct.roughness_mode == 2 ? quotient(cbrt(sqrt(h)), ct.roughness_value, ct.rrough)
                                             : chezy<double>(ct.roughness_mode, h, ct.roughness_value);
     const double square = hu * hu + hv * hv, stiff = c * c * h;
-    double factor;
-    if (finite_bits(square)) {
-        const double speed = quotient(sqrt(square), h, reciprocal(h));
-        const double y = 1. + quotient(dt * ct.grav * speed, stiff, reciprocal(stiff));
-        factor = quotient(1., y, reciprocal(y));
-    } else factor = drag_factor_far(square, h, dt, ct.grav, stiff);
+    const double speed = quotient(sqrt(square), h, reciprocal(h));
+    const double y = 1. + quotient(dt * ct.grav * speed, stiff, reciprocal(stiff));
+    double factor = quotient(1., y, reciprocal(y));
+    if (!finite_bits(factor)) factor = drag_factor_far(ct, square, h, dt);
     hu *= factor;
     hv *= factor;
 }
