@@ -1553,9 +1553,10 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary_plain(MeshDev m, 
     double Q = 0., level = 0.;
     if (b.table_len > 0) {
         const double t = ct.time0 + ct.elapsed + (stage == 2 ? trial : hancock ? .5 * trial : 0.0);
-        const bool first = n > 0 && tile.first == b.seg_off[tile.sg] && at == 0;     // writes the sampled rows
-        if (n > 0 && (mode == 6 || first)) Q = table_forcing(b, 0, tile.sg, t);
-        if (n > 0 && (mode == 2 || first)) level = table_forcing(b, 1, tile.sg, t);
+        // writes the sampled rows, those of a segment without faces too
+        const bool first = i < ntile && tile.first == b.seg_off[tile.sg] && at == 0;
+        if (mode == 6 || first) Q = table_forcing(b, 0, tile.sg, t);
+        if (mode == 2 || first) level = table_forcing(b, 1, tile.sg, t);
         if (first) { b.forcing[tile.sg] = Q; b.forcing[nseg + tile.sg] = level; }
     } else if (n > 0) { Q = b.forcing[tile.sg]; level = b.forcing[nseg + tile.sg]; }
     // wetted stage sum and wetted width of the conveyance inlets' tiles: a row
