@@ -90,7 +90,8 @@ struct brx_solver {
     int launches_per_substep = 0;
     MixedGeo mx{};                   // FP32 geometry of the mixed form
     Cells64 c64{};                   // FP64 form, cells of at most four faces: tables of the cell sweep
-    bool small64 = false;            // c64 is in use
+    bool small64 = false;            // the f-wave method uses c64
+    bool tables64_dirty = true;      // c64 is to be formed (again)
     std::vector<int2> h_cidx;        // host copy: stage-outlet flags follow brx_boundary_set
     int2 *d_cidx = nullptr;
     std::vector<int> h_faces_csr;
@@ -386,29 +387,7 @@ extern "C" int brx_solver_create(int nscen, const int *cell_offset, const int *f
         CK(cudaMemset(a.count, 0, sizeof(int) * 5));
         a.cell_off = s->d_cell_off; a.face_off = s->d_face_off;
         TRY(s->alloc(&s->work.limited, nc));
-        if (precision == BRX_FP64) {
-            double2 *p_cw;
-            double *p_rarea;
-            TRY(s->alloc(&p_cw, nadj)); TRY(s->alloc(&p_rarea, nc));
-            // on the default stream, which follows the uploads
-            k64_weights<<<std::max(1, std::min((nc + 255) / 256, s->sms * 32)), 256>>>(m, p_cw, p_rarea);
-            CK(cudaGetLastError());
-            CK(cudaStreamSynchronize(nullptr));
-            s->work.cw = p_cw; s->work.rarea = p_rarea;
-            TRY(s->alloc(&s->c64.prim[0], nc));
-        }
         s->small64 = precision == BRX_FP64 && s->maxdeg <= 4;
-        if (s->small64) {
-            // the cell sweep's tables, formed on the device from the uploaded
-            // geometry: the default stream follows the uploads
-            Cells64 &g = s->c64;
-            TRY(s->alloc(&g.ls, nc)); TRY(s->alloc(&g.lsr, nc)); TRY(s->alloc(&g.par, nc)); TRY(s->alloc(&g.ccls, nc));
-            TRY(s->alloc(&g.cidx, nadj)); TRY(s->alloc(&g.ent, nadj)); TRY(s->alloc(&g.unit, nadj));
-            TRY(s->alloc(&g.gbed, nc)); TRY(s->alloc(&g.prim[1], nc));
-            k64_tables<<<std::max(1, std::min((nc + 255) / 256, s->sms * 32)), 256>>>(m, g);
-            CK(cudaGetLastError());
-            CK(cudaStreamSynchronize(nullptr));
-        }
         if (precision == BRX_MIXED) {
             // FP32 geometry packed per cell, per CSR entry and per face; the LS
             // inverse is formed in FP64 here so the sweep only multiplies.
@@ -604,12 +583,7 @@ extern "C" int brx_boundary_set(brx_solver *s, const int *seg_mode, const int *s
     CK(cudaMemcpy(s->d_stage_policy_rw, stage_policy, sizeof(int) * nseg, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(s->d_ext_bed_rw, ext.data(), sizeof(double) * s->nslot, cudaMemcpyHostToDevice));
     CK(cudaMemcpy(s->bnd.forcing, forcing, sizeof(double) * 2 * nseg, cudaMemcpyHostToDevice));
-    if (s->small64) {
-        // the modes changed: the entries' stage-outlet flags with them
-        k64_tables<<<std::max(1, std::min((s->nc + 255) / 256, s->sms * 32)), 256>>>(s->mesh, s->c64);
-        CK(cudaGetLastError());
-        CK(cudaStreamSynchronize(nullptr));
-    }
+    s->tables64_dirty = true;        // the entries' stage-outlet flags
     if (s->precision == BRX_MIXED) {
         // entries on a stage outlet face (flag bit1) for the mixed cell sweep
         std::fill(s->h_ccls.begin(), s->h_ccls.end(), 0);
@@ -831,6 +805,46 @@ extern "C" int brx_forcing_table_set(brx_solver *s, int len, const double *time,
     return BRX_OK;
 }
 
+// Mesh tables of the FP64 form that the selected method reads, formed on the
+// device from the uploaded geometry: where the state is bound (the last step of
+// a set-up), and again where the method or the boundary modes changed since.
+// The default stream follows the uploads.
+static int ensure_tables64(brx_solver *s)
+{
+    if (s->precision != BRX_FP64 || s->pending) return BRX_OK;     // an interval in flight reads them
+    const bool fwave = s->method == BRX_METHOD_FWAVE;
+    const int grid = std::max(1, std::min((s->nc + 255) / 256, s->sms * 32));
+    bool formed = false;
+    if (!s->work.rarea || (fwave && !s->work.cw)) {
+        double2 *cw = nullptr;
+        double *rarea = const_cast<double *>(s->work.rarea);
+        if (fwave) TRY(s->alloc(&cw, s->nadj));
+        if (!rarea) TRY(s->alloc(&rarea, s->nc));
+        k64_weights<<<grid, 256>>>(s->mesh, cw, rarea);
+        s->work.cw = cw; s->work.rarea = rarea;
+        formed = true;
+    }
+    Cells64 &g = s->c64;
+    if (!g.prim[0] && (!fwave || s->small64)) {
+        TRY(s->alloc(&g.prim[0], s->nc));
+        s->hllc.prim = g.prim[0];
+    }
+    if (fwave && s->small64 && s->tables64_dirty) {
+        if (!g.prim[1]) {
+            TRY(s->alloc(&g.ls, s->nc)); TRY(s->alloc(&g.lsr, s->nc)); TRY(s->alloc(&g.par, s->nc));
+            TRY(s->alloc(&g.ccls, s->nc)); TRY(s->alloc(&g.cidx, s->nadj)); TRY(s->alloc(&g.ent, s->nadj));
+            TRY(s->alloc(&g.unit, s->nadj)); TRY(s->alloc(&g.gbed, s->nc)); TRY(s->alloc(&g.prim[1], s->nc));
+        }
+        k64_tables<<<grid, 256>>>(s->mesh, g);
+        formed = true;
+    }
+    if (!formed) return BRX_OK;
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(nullptr));
+    if (fwave) s->tables64_dirty = false;
+    return BRX_OK;
+}
+
 extern "C" int brx_state_bind(brx_solver *s, double *q_device, double *z_device)
 {
     if (!s || !q_device || !z_device) return fail(BRX_ERR_ARGUMENT, "null state pointer");
@@ -838,7 +852,7 @@ extern "C" int brx_state_bind(brx_solver *s, double *q_device, double *z_device)
     s->state.z = z_device;
     s->bound = true;
     s->graph_dirty = true;
-    return BRX_OK;
+    return s->boundary_ready || !s->nseg ? ensure_tables64(s) : BRX_OK;
 }
 
 extern "C" int brx_scenarios_activate(brx_solver *s, const int *active)
@@ -1056,7 +1070,7 @@ extern "C" int brx_hllc_set(brx_solver *s, const int *entry_face, const int *ent
         k_hllc_squares<<<std::max(1, std::min((nadj + 255) / 256, s->sms * 32)), 256>>>(nadj, p_geo, p_square);
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(nullptr));
-        s->hllc.square = p_square; s->hllc.prim = s->c64.prim[0];
+        s->hllc.square = p_square;
     }
     if (s->precision == BRX_MIXED) {
         // FP32 stencil of the mixed form: LS offset over its squared length
@@ -1838,7 +1852,7 @@ static int ensure_ready(brx_solver *s)
     if (!s) return fail(BRX_ERR_ARGUMENT, "null solver");
     if (!s->bound) return fail(BRX_ERR_STATE, "no state bound (brx_state_bind)");
     if (!s->boundary_ready && s->nseg) return fail(BRX_ERR_STATE, "open boundaries not configured (brx_boundary_set)");
-    return BRX_OK;
+    return ensure_tables64(s);
 }
 
 static int build_graph(brx_solver *s)

@@ -41,7 +41,7 @@ struct Cells64 {
     Prim64 *prim[2];          // (nc) primitives of the two stage inputs
 };
 
-// The mesh tables of Cells64 (at creation, and when the boundary modes change).
+// The mesh tables of Cells64 (at set-up, and when the boundary modes change).
 __global__ void __launch_bounds__(256) k64_tables(MeshDev m, Cells64 g)
 {
     const int nc = m.nc, nf = m.nf;

@@ -21,12 +21,13 @@
 
 namespace brx {
 
-// Entry tables (at creation).
+// Entry and cell tables; cw may be null (the HLLC method reads the cells' alone).
 __global__ void __launch_bounds__(256) k64_weights(MeshDev m, double2 *cw, double *rarea)
 {
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < m.nc; c += gridDim.x * blockDim.x) {
         const double area = m.area[c];
         rarea[c] = 1. / area;
+        if (!cw) continue;
         for (int k = m.offset[c]; k < m.offset[c + 1]; ++k) {
             const double len = m.length[m.faces[k]];
             cw[k] = make_double2(m.signs[k] * len / area, len);

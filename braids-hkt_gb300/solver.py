@@ -314,7 +314,6 @@ class RiverSolver:
         dev = torch.device("cuda", torch.cuda.current_device())
         self.q = torch.from_numpy(p["q"]).to(dev).contiguous()
         self.z = torch.from_numpy(p["z"]).to(dev).contiguous()
-        check(self.lib.brx_state_bind(self.h, C.c_void_p(self.q.data_ptr()), C.c_void_p(self.z.data_ptr())))
         check(self.lib.brx_graph_chunk_set(self.h, int(graph_chunk)))
         self.graph_chunk = int(graph_chunk)
         self.rotors = None
@@ -350,6 +349,8 @@ class RiverSolver:
         self.bed_model = None
         if any(c.get("exner") for c in self.cases):
             self._set_exner()
+        # last: it forms the tables that the chosen method reads
+        check(self.lib.brx_state_bind(self.h, C.c_void_p(self.q.data_ptr()), C.c_void_p(self.z.data_ptr())))
         self.time = np.zeros(self.nscen)
         self.steps = 0
 
