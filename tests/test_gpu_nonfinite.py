@@ -1,0 +1,29 @@
+"""A state that is not finite is refused by the f-wave method in both forms: the
+trial reports a status and the interval fails as the oracle's does, with the
+bound state as it was."""
+import numpy as np
+import pytest
+
+import braids_hkt_gb300.scenarios as S
+from oracle import Oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("make", [S.small_channel, S.cartesian_channel])
+@pytest.mark.parametrize("row,value", [(0, np.nan), (0, np.inf), (0, -1.0), (0, -np.inf), (1, np.nan), (1, np.inf),
+                                       (2, -np.inf), (2, np.nan)])
+def test_nonfinite_or_negative_cell(make, row, value, precision):
+    from braids_hkt_gb300.solver import RiverSolver
+    case = make()
+    q = case["q"].copy()
+    q[row, case["mesh"].nc // 2] = value
+    s = RiverSolver(case, precision=precision)
+    s.set_state(q)
+    assert int(s.substep(0.004)[0]) != 0
+    np.testing.assert_array_equal(s.state(), q)
+    d = s.advance(0.05, 0.0, raise_on_failure=False)
+    code, _, stats = Oracle(case).advance(q.copy(), 0.05, 0.0)
+    assert code != 0 and d["failed"] != 0 and d["hydraulic_substeps"] == stats["substeps"] == 0
+    np.testing.assert_array_equal(s.state(), q)
