@@ -152,6 +152,11 @@ __device__ __forceinline__ SlotTile slot_tile(const BoundaryDev &b, int s0, int 
 }
 
 constexpr int BOUNDARY_THREADS = 128;      // one warp per sub-partition: FP64 work does not overlap within one
+// openings beyond a cluster, which keep one block: its loads and FP32 powers want
+// more warps. Openings of 1,030 / 2,000 / 4,000 faces, 128 -> 512 threads, us a
+// stage: FP64 193 / 359 / 711 -> 147 / 264 / 522, mixed 176 / 329 / 652 -> 129 / 231 / 464
+// (256: 155 / 283 / 555 and 138 / 252 / 498)
+constexpr int BOUNDARY_WIDE = 512;
 
 // The sum of a tile's terms in slot order, formed by one warp: lane l's terms
 // are those of slots first + l and first + 32 + l; rows are summed by as many
@@ -1618,11 +1623,13 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary_plain(MeshDev m, 
     if (rank == 0) scenario_water(b, ct, stage, s0, ntile);
 }
 
-// The open boundary of one scenario in one block: any modes, any width.
-template <class F>
-__global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int stage_in)
+// The open boundary of one scenario in one block: any width, and any modes with
+// BOUNDARY_THREADS (a section solve's lanes); with more, no section solves.
+template <class F, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_boundary(MeshDev m, StateDev s, BoundaryDev b, Ctrl *ctrl, int stage_in)
 {
-    __shared__ double tile_buf[2][BOUNDARY_TILES], warp_buf[BOUNDARY_THREADS / 32][2][64];
+    const bool sections = THREADS == BOUNDARY_THREADS && b.sections;
+    __shared__ double tile_buf[2][BOUNDARY_TILES], warp_buf[THREADS / 32][2][64];
     const int sid = blockIdx.x, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     Ctrl &ct = ctrl[sid];
     const bool hancock = stage_in == STAGE_HANCOCK;
@@ -1647,7 +1654,7 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
     // (river_exterior_bed.py:199-200); a section without a root rejects the trial
     __shared__ SectionWork section;
     bool line_failed = false;
-    if (b.sections && b.line_kind) {
+    if (sections && b.line_kind) {
         for (int pass = 1; pass <= 2; ++pass)
             for (int sg = s0; sg < s1; ++sg)          // block-uniform
                 if (b.seg_mode[sg] == 9 && b.line_kind[sg] == pass &&
@@ -1658,7 +1665,7 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
     int ntile = 0;
     for (int sg = s0; sg < s1; ++sg) ntile += tile_count(b, sg);
     // wetted stage sum and wetted width of the conveyance inlets' segments
-    for (int i = warp; i < ntile; i += BOUNDARY_THREADS / 32) {
+    for (int i = warp; i < ntile; i += THREADS / 32) {
         const SlotTile tile = slot_tile(b, s0, i);
         if (b.seg_mode[tile.sg] != 6) continue;
         double lo[2] = {0., 0.}, hi[2] = {0., 0.};
@@ -1685,7 +1692,7 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
     }
     __syncthreads();
     // conveyance weights
-    for (int i = warp; i < ntile; i += BOUNDARY_THREADS / 32) {
+    for (int i = warp; i < ntile; i += THREADS / 32) {
         const SlotTile tile = slot_tile(b, s0, i);
         if (b.seg_mode[tile.sg] != 6) continue;
         double lo[1] = {0.}, hi[1] = {0.};
@@ -1711,7 +1718,7 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
     }
     __syncthreads();
     unsigned bad = 0;
-    for (int i = threadIdx.x >> 6; i < ntile; i += BOUNDARY_THREADS / 64) {
+    for (int i = threadIdx.x >> 6; i < ntile; i += THREADS / 64) {
         const SlotTile tile = slot_tile(b, s0, i);
         const int k = tile.first + (threadIdx.x & 63), mode = b.seg_mode[tile.sg];
         if (k >= tile.end) continue;
@@ -1725,8 +1732,8 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
         for (int r = 0; r < 3; ++r) { b.trace[r * ns + k] = tr[r]; b.flux[r * ns + k] = fl[r]; }
     }
     __syncthreads();
-    if (b.sections) {
-    // section owners of the remaining outlet modes, after the face loop, in
+    if (sections) {
+        // section owners of the remaining outlet modes, after the face loop, in
         // the reference's order (river_exterior_bed.py:213-217): a normal-depth
         // chain without a root rejects the trial before the rating owner runs; a
         // rating section without a solution fails the scenario
@@ -1788,10 +1795,10 @@ __global__ void __launch_bounds__(BOUNDARY_THREADS) k_boundary(MeshDev m, StateD
     if (bad) raise_status(ct, stage, ST_SPATIAL);
     // outlet stock cap, one thread per unique owner, its faces in boundary order
     const int u0 = b.scen_own[sid], u1 = b.scen_own[sid + 1];
-    cap_owners(m, b, base, ct.trial, u0 + (int)threadIdx.x, u1, BOUNDARY_THREADS, false);
+    cap_owners(m, b, base, ct.trial, u0 + (int)threadIdx.x, u1, THREADS, false);
     if (b.inlet) inlet_allocation(m, b, ct, base, s0, s1, u0, u1);
     __syncthreads();
-    for (int i = warp; i < 2 * ntile; i += BOUNDARY_THREADS / 32) {
+    for (int i = warp; i < 2 * ntile; i += THREADS / 32) {
         const SlotTile tile = slot_tile(b, s0, i >> 1);
         const int first = tile.first + 32 * (i & 1), k = first + lane;
         const double2 sum = warp_water(k < tile.end ? double(F(b.flux[k])) * m.length[b.slot_face[k]] : 0.);
@@ -1808,7 +1815,8 @@ inline void launch_boundary(const MeshDev &m, const StateDev &s, const BoundaryD
                             cudaStream_t st)
 {
     if (b.cluster == 0) {
-        k_boundary<F><<<nscen, BOUNDARY_THREADS, 0, st>>>(m, s, b, ctrl, stage);
+        if (b.sections) k_boundary<F, BOUNDARY_THREADS><<<nscen, BOUNDARY_THREADS, 0, st>>>(m, s, b, ctrl, stage);
+        else k_boundary<F, BOUNDARY_WIDE><<<nscen, BOUNDARY_WIDE, 0, st>>>(m, s, b, ctrl, stage);
         return;
     }
     cudaLaunchAttribute attr{};
