@@ -1403,17 +1403,23 @@ __global__ void __launch_bounds__(64) km_limited(MeshDev m, StateDev s, Ctrl *ct
         }
     const float2 *ws = reinterpret_cast<const float2 *>(w.ws);
     const float *theta32 = reinterpret_cast<const float *>(w.theta);
-    // four threads per listed cell: itself, then its entries in turn; a
-    // neighbour that is listed too is left to its own entry
-    const int n = 4 * m.act.count[2 + stage];
+    // a thread per listed cell and entry (D > 0; else four that take them in
+    // turn): the cell itself, then the neighbours; one that is listed too is left to
+    // its own entry. One call for both: a warp's cells and neighbours then wait on
+    // one chain of loads together, not on one after the other (update and redo of a
+    // substep, wet/dry lake of 40,000 triangles 41.6 -> 35.3 us, 1,600 37.4 -> 33.2)
+    constexpr int PARTS = D > 0 ? D + 1 : 4;
+    const int n = PARTS * m.act.count[2 + stage];
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const int c = w.limited[i >> 2], part = i & 3;
-        if (part == 0) mx_limited_cell<D>(m, s, ctrl, w, g, stage, c, rate_out, t, turb);
-        for (int k = m.offset[c] + (part + 3) % 4; k < m.offset[c + 1]; k += 4) {
-            const int2 id = g.cidx[k];
-            const float wf = ws[m.faces[k]].x;
-            if (id.x >= 0 && wf != 0.f && (wf > 0.f) == ((id.y & 16) != 0) && theta32[id.x] == 1.f)
-                mx_limited_cell<D>(m, s, ctrl, w, g, stage, id.x, rate_out, t, turb);
+        const int c = w.limited[i / PARTS], k0 = m.offset[c], deg = m.offset[c + 1] - k0;
+        for (int part = i % PARTS; part <= deg; part += PARTS) {
+            int target = c;
+            if (part > 0) {
+                const int2 id = g.cidx[k0 + part - 1];
+                const float wf = ws[m.faces[k0 + part - 1]].x, th = id.x >= 0 ? theta32[id.x] : 0.f;
+                target = wf != 0.f && (wf > 0.f) == ((id.y & 16) != 0) && th == 1.f ? id.x : -1;
+            }
+            if (target >= 0) mx_limited_cell<D>(m, s, ctrl, w, g, stage, target, rate_out, t, turb);
         }
     }
 }
