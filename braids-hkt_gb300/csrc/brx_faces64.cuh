@@ -20,8 +20,9 @@
 //     shock's two terms one is zero.
 // About 300 FP64 instructions per wet face instead of 970. Per launch, before
 // -> after: 302k cells 831 -> 306 us, 50k 158 -> 70 us, 360 cells 53 -> 29 us.
-// A face with a dry side takes the general solver (dry_face64), which keeps the
-// reference's whole sequence.
+// A face with a dry side, or with a state whose solution is not finite, takes the
+// general solver (dry_face64), which keeps the reference's whole sequence: its
+// extrema pass over a NaN, so such a face has the reference's status and speed.
 #pragma once
 #include "brx_num64.cuh"
 #include "brx_turbine.cuh"
@@ -166,8 +167,8 @@ __device__ __forceinline__ bool wet_face64(double hL, double huL, double hvL, do
     return bad;
 }
 
-// A face with a dry state: whether it is closed, the general augmented solver
-// with its reflecting wall at a dry side, and the closed face's speed.
+// A face with a dry or nonfinite state: whether it is closed, the general augmented
+// solver with its reflecting wall at a dry side, and the closed face's speed.
 // loc: h, un, ut, b of both reconstructed states (brx_fwave.cuh's order).
 __device__ __noinline__ bool dry_face64(const double *loc, double hc, double zc, double hn, double zn, int kind,
                                         double hL, double bL, double unL, double hR, double bR, double unR, double dc,
@@ -277,12 +278,12 @@ __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, Bound
             const double kr = greater(hR, dry) ? quotient(hr, hR, reciprocal(hR)) : 0.;
             const double loc[8] = {inner ? hl : hL, inner ? unL * kl : unL, inner ? utL * kl : utL, inner ? top : bL,
                                    inner ? hr : hR, inner ? unR * kr : unR, inner ? utR * kr : utR, inner ? top : bR};
-            Solve64 o;
+            Solve64 o{};
             bool closed = false;
             const bool wet = greater(loc[0], dry) && greater(loc[4], dry);
-            if (wet) {
-                if (wet_face64(loc[0], loc[1], loc[2], loc[4], loc[5], loc[6], grav, ct.g16r, o)) bad = 1;
-            } else {
+            bool general = !wet;
+            if (wet) general = wet_face64(loc[0], loc[1], loc[2], loc[4], loc[5], loc[6], grav, ct.g16r, o);
+            if (general) {
                 double in[8];
 #pragma unroll
                 for (int j = 0; j < 8; ++j) in[j] = loc[j];
@@ -290,6 +291,7 @@ __global__ void __launch_bounds__(128, 4) k64_faces(MeshDev m, StateDev s, Bound
                 bool shut;
                 if (dry_face64(in, rc.h, rc.b, rn.h, rn.b, inner ? 1 : 2, hL, bL, unL, hR, bR, unR,
                                m.distance[f], m.distance[nf + f], dry, grav, shut, d)) bad = 1;
+                d.ul = o.ul; d.ur = o.ur;
                 o = d;
                 closed = shut;
             }

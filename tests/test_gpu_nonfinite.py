@@ -27,3 +27,18 @@ def test_nonfinite_or_negative_cell(make, row, value, precision):
     code, _, stats = Oracle(case).advance(q.copy(), 0.05, 0.0)
     assert code != 0 and d["failed"] != 0 and d["hydraulic_substeps"] == stats["substeps"] == 0
     np.testing.assert_array_equal(s.state(), q)
+
+
+@pytest.mark.parametrize("make", [S.small_channel, S.cartesian_channel, S.dam_break])
+@pytest.mark.parametrize("row,value,word", [(0, np.nan, 5), (0, np.inf, 5), (0, -1.0, 1), (1, np.nan, 5), (1, np.inf, 5),
+                                            (2, -np.inf, 5), (1, 1e200, 5)])
+def test_status_word(make, row, value, word):
+    """Spatial (1) and rate (4) failures of the FP64 form. A wave speed that is not a
+    number is passed over, as in the reference's extrema: no frequency failure (16)."""
+    from braids_hkt_gb300.solver import RiverSolver
+    case = make()
+    q = case["q"].copy()
+    q[row, int(np.argmax(q[0]))] = value
+    s = RiverSolver(case)
+    s.set_state(q)
+    assert int(s.rate(0.004)[2]) & ~32 == word
