@@ -297,13 +297,17 @@ __global__ void __launch_bounds__(128) k64_bed(MeshDev m, Cells64 g, const doubl
 }
 
 // First stage's primitives of a state placed in work directly (single residual).
-__global__ void __launch_bounds__(256) k64_prim(MeshDev m, StateDev s, const Ctrl *ctrl, Cells64 g)
+// A nonfinite momentum of a dry cell, which a substep's drag has set to zero,
+// fails the stage; the velocity that its neighbours see is zero.
+__global__ void __launch_bounds__(256) k64_prim(MeshDev m, StateDev s, Ctrl *ctrl, Cells64 g)
 {
     const int nc = m.nc;
     FOR_ACTIVE_CELLS(m.act, c) {
-        const Ctrl &ct = ctrl[m.cell_sid[c]];
+        Ctrl &ct = ctrl[m.cell_sid[c]];
         if (!ct.active || ct.done) continue;
-        put_prim64(g.prim[0], c, s.work[c], s.work[nc + c], s.work[2 * nc + c], s.z[c], ct.dry);
+        const double hu = s.work[nc + c], hv = s.work[2 * nc + c];
+        if (!finite_bits(hu) || !finite_bits(hv)) raise_status(ct, 1, ST_SPATIAL);
+        put_prim64(g.prim[0], c, s.work[c], hu, hv, s.z[c], ct.dry);
     }
 }
 

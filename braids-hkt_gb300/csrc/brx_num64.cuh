@@ -78,10 +78,7 @@ __device__ __forceinline__ void put_prim64(Prim64 *P, int c, double h, double hu
     if (greater(h, dry)) {
         const double r = reciprocal(h);
         p.u = quotient(hu, h, r); p.v = quotient(hv, h, r);
-    } else {
-        // a nonfinite momentum of a dry cell fails the stage as in a wet one
-        p.u = finite_bits(hu) ? 0. : hu; p.v = finite_bits(hv) ? 0. : hv;
-    }
+    } else p.u = p.v = 0.;
     P[c] = p;
 }
 

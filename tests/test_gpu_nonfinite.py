@@ -42,3 +42,23 @@ def test_status_word(make, row, value, word):
     s = RiverSolver(case)
     s.set_state(q)
     assert int(s.rate(0.004)[2]) & ~32 == word
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf])
+def test_residual_beside_a_dry_cell_of_nonfinite_momentum(value):
+    """A dry cell's momentum takes no part: its residual fails (1), and the rates of
+    its neighbours are those beside a dry cell at rest."""
+    from braids_hkt_gb300.solver import RiverSolver
+    case = S.lake_at_rest()
+    q = S.perturbed_state(case, 3, 0.2, 0.5)
+    dry = int(np.flatnonzero(q[0] == 0.0)[0])
+    s = RiverSolver(case)
+    s.set_state(q)
+    rest = s.rate(0.004)
+    q[1, dry] = value
+    s.set_state(q)
+    rate, water, status, freq = s.rate(0.004)
+    assert int(rest[2]) == 0 and int(status) == 1 and freq == rest[3]
+    np.testing.assert_array_equal(rate.cpu().numpy(), rest[0].cpu().numpy())
+    np.testing.assert_array_equal(water.cpu().numpy(), rest[1].cpu().numpy())
+    assert int(s.substep(0.004)[0]) == 0                 # the drag sets it to zero
