@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256) k_ex_cells(MeshDev m, ExnerDev e, const d
         const double r = reciprocal(h), u = quotient(hu, h, r), v = quotient(hv, h, r), speed = hypot(u, v);
         const double unit = c * c * 1.65 * d, theta = quotient(speed * speed, unit, reciprocal(unit));
         double x = 0., y = 0.;
-        if (greater(speed, 0.)) {
+        if (speed > 0.) {                                // false for a NaN, which the slope operator reports
             const double depth = greater(h, .01) ? h : .01, rough = quotient(depth, d90, reciprocal(d90));
             const double grain = 18. * log10(12. * (greater(rough, 1.) ? rough : 1.)), part = quotient(c, grain, reciprocal(grain));
             const double power = part * sqrt(part), mu = greater(power, 1.) ? 1. : power;

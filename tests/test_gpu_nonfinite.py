@@ -62,3 +62,18 @@ def test_residual_beside_a_dry_cell_of_nonfinite_momentum(value):
     np.testing.assert_array_equal(rate.cpu().numpy(), rest[0].cpu().numpy())
     np.testing.assert_array_equal(water.cpu().numpy(), rest[1].cpu().numpy())
     assert int(s.substep(0.004)[0]) == 0                 # the drag sets it to zero
+
+
+def test_bed_update_of_a_state_that_is_not_a_number():
+    """Refused by the slope operator with the bed as it was; the cell carries no
+    transport, so the budget residual is a number."""
+    from braids_hkt_gb300.solver import RiverSolver
+    case = S.cartesian_channel()
+    case["exner"] = S.exner_params(case)
+    q = S.perturbed_state(case, 3, 0.1, 1.0)
+    q[2, case["mesh"].nc // 2] = np.nan
+    s = RiverSolver(case)
+    s.set_state(q)
+    row = s.morphology(1.0)
+    assert not row["ok"] and row["slope_failure"] and np.isfinite(row["residual"])
+    np.testing.assert_array_equal(s.z.cpu().numpy(), case["z"])
