@@ -73,8 +73,8 @@ __global__ void __launch_bounds__(256) k_ex_cells(MeshDev m, ExnerDev e, const d
         }
         e.gz[i] = e.inverse[i] * bx + e.inverse[n + i] * by;
         e.gz[n + i] = e.inverse[n + i] * bx + e.inverse[2 * n + i] * by;
-        const double r = reciprocal(h), u = quotient(hu, h, r), v = quotient(hv, h, r), speed = hypot(u, v);
-        const double unit = c * c * 1.65 * d, theta = quotient(speed * speed, unit, reciprocal(unit));
+        const double r = reciprocal(h), u = any_quotient(hu, h, r), v = any_quotient(hv, h, r), speed = hypot(u, v);
+        const double unit = c * c * 1.65 * d, theta = any_quotient(speed * speed, unit, reciprocal(unit));
         double x = 0., y = 0.;
         if (speed > 0.) {                                // false for a NaN, which the slope operator reports
             const double depth = greater(h, .01) ? h : .01, rough = quotient(depth, d90, reciprocal(d90));
@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) k_ex_cells(MeshDev m, ExnerDev e, const d
             const double excess = mu * theta - .047 * hide;
             if (greater(excess, 0.)) {
                 const double mag = 2650. * 8. * sqrt(9.81 * 1.65 * d * excess) * d * excess, rs = reciprocal(speed);
-                x = quotient(mag * u, speed, rs); y = quotient(mag * v, speed, rs);
+                x = any_quotient(mag * u, speed, rs); y = any_quotient(mag * v, speed, rs);
             }
         }
         e.cell[i] = x; e.cell[n + i] = y; e.cell[2 * n + i] = theta;

@@ -54,6 +54,15 @@ __device__ __forceinline__ double reciprocal(double y)
     return __fma_rn(__fma_rn(-y, r, 1.), r, r);
 }
 
+// x / y as quotient() gives it, or by a division where that is not finite: an
+// infinite operand, a divisor outside reciprocal()'s range, an overflow.
+static __device__ __noinline__ double plain_quotient(double x, double y) { return x / y; }
+__device__ __forceinline__ double any_quotient(double x, double y, double r)
+{
+    const double q = quotient(x, y, r);
+    return finite_bits(q) ? q : plain_quotient(x, y);
+}
+
 // FP32 image of a double by truncation, on the integer pipe (a conversion
 // instruction runs on the FP64 pipe): relative error below 2^-23, values
 // below the FP32 normal range become 0, those above it the largest float.

@@ -77,3 +77,24 @@ def test_bed_update_of_a_state_that_is_not_a_number():
     row = s.morphology(1.0)
     assert not row["ok"] and row["slope_failure"] and np.isfinite(row["residual"])
     np.testing.assert_array_equal(s.z.cpu().numpy(), case["z"])
+
+
+def test_bed_update_beside_an_infinite_depth():
+    """A cell of infinite depth has no speed and no transport: the update of still
+    water is accepted and moves nothing; one of infinite stress is refused."""
+    from braids_hkt_gb300.solver import RiverSolver
+    case = S.cartesian_channel()
+    case["exner"] = S.exner_params(case)
+    q = case["q"].copy()
+    q[0, case["mesh"].nc // 2] = np.inf
+    s = RiverSolver(case)
+    s.set_state(q)
+    row = s.morphology(1.0)
+    assert row["ok"] and not row["slope_failure"] and row["residual"] == 0.0 and row["change"] == 0.0
+    np.testing.assert_array_equal(s.z.cpu().numpy(), case["z"])
+    q = case["q"].copy()
+    q[1, case["mesh"].nc // 2] = 1e200
+    s.set_state(q)
+    row = s.morphology(1.0)
+    assert not row["ok"] and row["slope_failure"]
+    np.testing.assert_array_equal(s.z.cpu().numpy(), case["z"])
