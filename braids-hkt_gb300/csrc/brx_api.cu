@@ -1167,7 +1167,7 @@ static int max_block(const brx_solver *s, int kind)
     case K_DRAG: fn = (const void *)k_open_drag; break;
     case K_CELLS:
         fn = s->maxdeg <= 3 ? (const void *)k64_cells<3> : small ? (const void *)k64_cells<4>
-                            : (const void *)k_cells<double, MAX_CELL_FACES>;
+                            : (const void *)k_cells<MAX_CELL_FACES>;
         break;
     case K_FACES: fn = s->has_turb ? (const void *)k64_faces<true> : (const void *)k64_faces<false>; break;
     case K_LIMIT: fn = (const void *)k_limit; break;
@@ -1649,7 +1649,7 @@ static int launch_kernel(brx_solver *s, int kind, int stage, double *rate_out, c
             k64_cells<3><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, s->c64, stage);
         else if (s->maxdeg <= 4)
             k64_cells<4><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, s->c64, stage);
-        else k_cells<double, MAX_CELL_FACES><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
+        else k_cells<MAX_CELL_FACES><<<SSHAPE(K_CELLS, s->nc), 0, st>>>(s->mesh, s->state, s->d_ctrl, s->work, stage);
         return 1;
     case K_FACES:
         if (s->has_turb)
@@ -2509,7 +2509,7 @@ extern "C" int brx_rate_noalloc(int nc, int nf, int nadj, const int *owner, cons
     k_noalloc_ctrl<<<1, 1, 0, st>>>(ctrl, init, act, nc, nf);
     const int n = nc > nf ? nc : nf;
     k_noalloc_tables<<<(n + 255) / 256, 256, 0, st>>>(m, ctrl, cell_sid, cflags, face_sid, bslot, bmode, disp_unit);
-    k_cells<double, MAX_CELL_FACES><<<(nc + 127) / 128, 128, 0, st>>>(m, sd, ctrl, w, 1);
+    k_cells<MAX_CELL_FACES><<<(nc + 127) / 128, 128, 0, st>>>(m, sd, ctrl, w, 1);
     k64_faces<false><<<(nf + 127) / 128, 128, 0, st>>>(m, sd, b, ctrl, w, 1, TurbDev{});
     k64_update<<<(nc + 255) / 256, 256, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);
     k_limited<<<(nc + 63) / 64, 64, 0, st>>>(m, sd, ctrl, w, 1, rate, TurbDev{}, 0, nullptr);

@@ -3,9 +3,9 @@
 // Included by one translation unit per arithmetic form. Each includer
 // defines BRX_NS (the namespace its kernel copies live in) so the FP64
 // unit (-fmad=false, reference operation order) and the mixed unit (FP32
-// fluxes, FMA on) never share a symbol. Kernels whose arithmetic differs
-// between the forms are templates on the flux type F; with F = double they
-// evaluate exactly the FP64 expressions of the reference.
+// fluxes, FMA on) never share a symbol. The boundary kernels, whose arithmetic
+// differs between the forms, are templates on the flux type F; the others are
+// the FP64 form's and evaluate the FP64 expressions of the reference.
 #pragma once
 #include "brx_common.cuh"
 #include <cooperative_groups.h>
@@ -1830,52 +1830,40 @@ inline void launch_boundary(const MeshDev &m, const StateDev &s, const BoundaryD
 
 // ---------------------------------------------------------------------------
 // Cells: primitive values, limited least-squares gradients, flattening flag.
-// Depth, surface and bed stay FP64 (the stage reconstruction); gradients,
-// limiter factors and the projection run in F.
+// The general FP64 sweep: cells of more than four faces, and the
+// allocation-free residual.
 // ---------------------------------------------------------------------------
-// Roundoff scale of the arithmetic type: the reference's FP64 thresholds
-// (64 eps, 2e-14) are kept verbatim for F = double; in FP32 the same tests
-// are widened to FP32 rounding so that a projection vertex lying on its own
-// constraints is not rejected by rounding noise.
-template <class F> struct Eps { static constexpr double value = 2.2204460492503131e-16; };
-template <> struct Eps<float> { static constexpr double value = 1.1920928955078125e-07; };
-
-template <class F>
-__device__ __forceinline__ bool feasible(F x, F y, int count, const F *ax, const F *ay, const F *bb)
+__device__ __forceinline__ bool feasible(double x, double y, int count, const double *ax, const double *ay, const double *bb)
 {
-    for (int i = 0; i < count; ++i) {
-        F tol = F(2.e-14);
-        if (sizeof(F) != 8) tol += F(16. * Eps<F>::value) * (fabs(ax[i] * x) + fabs(ay[i] * y) + fabs(bb[i]));
-        if (ax[i] * x + ay[i] * y > bb[i] + tol) return false;
-    }
+    for (int i = 0; i < count; ++i)
+        if (ax[i] * x + ay[i] * y > bb[i] + 2.e-14) return false;
     return true;
 }
 
-template <class F>
-__device__ __noinline__ void project_pair(F &x, F &y, int count, const F *ax, const F *ay, const F *bb)
+static __device__ __noinline__ void project_pair(double &x, double &y, int count, const double *ax, const double *ay, const double *bb)
 {
-    const F rx = x, ry = y;
-    if (feasible<F>(rx, ry, count, ax, ay, bb)) return;
-    F bx = F(0.), by = F(0.), best = rx * rx + ry * ry;
+    const double rx = x, ry = y;
+    if (feasible(rx, ry, count, ax, ay, bb)) return;
+    double bx = 0., by = 0., best = rx * rx + ry * ry;
     for (int i = 0; i < count; ++i) {
-        const F dot = ax[i] * rx + ay[i] * ry - bb[i];
-        F cx = rx - dot * ax[i], cy = ry - dot * ay[i];
-        F d = (cx - rx) * (cx - rx) + (cy - ry) * (cy - ry);
-        if (d < best && feasible<F>(cx, cy, count, ax, ay, bb)) { bx = cx; by = cy; best = d; }
+        const double dot = ax[i] * rx + ay[i] * ry - bb[i];
+        double cx = rx - dot * ax[i], cy = ry - dot * ay[i];
+        double d = (cx - rx) * (cx - rx) + (cy - ry) * (cy - ry);
+        if (d < best && feasible(cx, cy, count, ax, ay, bb)) { bx = cx; by = cy; best = d; }
         for (int j = 0; j < i; ++j) {
-            const F det = ax[i] * ay[j] - ay[i] * ax[j];
-            if (fabs(det) < F(1.e-12)) continue;
+            const double det = ax[i] * ay[j] - ay[i] * ax[j];
+            if (fabs(det) < 1.e-12) continue;
             cx = (bb[i] * ay[j] - ay[i] * bb[j]) / det;
             cy = (ax[i] * bb[j] - bb[i] * ax[j]) / det;
             d = (cx - rx) * (cx - rx) + (cy - ry) * (cy - ry);
-            if (d < best && feasible<F>(cx, cy, count, ax, ay, bb)) { bx = cx; by = cy; best = d; }
+            if (d < best && feasible(cx, cy, count, ax, ay, bb)) { bx = cx; by = cy; best = d; }
         }
     }
     x = bx; y = by;
 }
 
-// MAXF bounds the faces of one cell (4 for triangle/quad meshes, 32 in general).
-template <class F, int MAXF>
+// MAXF bounds the faces of one cell.
+template <int MAXF>
 __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl, Work w, int stage)
 {
     const int nc = m.nc, nf = m.nf, nadj = m.nadj;
@@ -1889,15 +1877,15 @@ __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl
         if (h < 0.0 || !isfinite(h) || !isfinite(zc) || !isfinite(hu) || !isfinite(hv))
             raise_status(ct, stage, ST_SPATIAL);
         double centre[4] = {h + zc, 0., 0., zc};
-        if (h > dry) { centre[1] = double(F(hu) / F(h)); centre[2] = double(F(hv) / F(h)); }
+        if (h > dry) { centre[1] = hu / h; centre[2] = hv / h; }
         double lo[4], hi[4];
-        F gx[4] = {F(0.), F(0.), F(0.), F(0.)}, gy[4] = {F(0.), F(0.), F(0.), F(0.)};
+        double gx[4] = {0., 0., 0., 0.}, gy[4] = {0., 0., 0., 0.};
 #pragma unroll
         for (int p = 0; p < 4; ++p) { lo[p] = centre[p]; hi[p] = centre[p]; }
         const int k0 = m.offset[c], k1 = m.offset[c + 1];
         // active: wet, or touching an open face or a wet neighbour
         bool active = h > dry;
-        F bx[4] = {F(0.), F(0.), F(0.), F(0.)}, by[4] = {F(0.), F(0.), F(0.), F(0.)};
+        double bx[4] = {0., 0., 0., 0.}, by[4] = {0., 0., 0., 0.};
         for (int k = k0; k < k1; ++k) {
             const int f = m.faces[k];
             const int n = m.signs[k] < 0 ? m.owner[f] : m.neighbour[f];
@@ -1905,22 +1893,22 @@ __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl
             const double hn = q[n], zn = z[n];
             if (hn > dry) active = true;
             double vn[4] = {hn + zn, 0., 0., zn};
-            if (hn > dry) { vn[1] = double(F(q[nc + n]) / F(hn)); vn[2] = double(F(q[2 * nc + n]) / F(hn)); }
-            const F rx = F(m.ls_delta[k]), ry = F(m.ls_delta[nadj + k]), wt = F(m.ls_weight[k]);
+            if (hn > dry) { vn[1] = q[nc + n] / hn; vn[2] = q[2 * nc + n] / hn; }
+            const double rx = m.ls_delta[k], ry = m.ls_delta[nadj + k], wt = m.ls_weight[k];
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
                 double adj = vn[p];
                 if (p == 0 && centre[0] - centre[3] > dry && vn[0] - vn[3] <= dry && vn[3] >= centre[0]) adj = centre[0];
-                const F d = F(adj - centre[p]);
+                const double d = adj - centre[p];
                 bx[p] += wt * rx * d;
                 by[p] += wt * ry * d;
                 lo[p] = fmin(lo[p], adj); hi[p] = fmax(hi[p], adj);
             }
         }
         if (active) {
-            const F a11 = F(m.ls_matrix[c]), a12 = F(m.ls_matrix[nc + c]), a22 = F(m.ls_matrix[2 * nc + c]),
-                    det = F(m.ls_matrix[3 * nc + c]);
-            if (a11 + a22 > F(0.0)) {
+            const double a11 = m.ls_matrix[c], a12 = m.ls_matrix[nc + c], a22 = m.ls_matrix[2 * nc + c],
+                    det = m.ls_matrix[3 * nc + c];
+            if (a11 + a22 > 0.0) {
                 if (h > dry)
                     for (int k = k0; k < k1; ++k) {
                         const int f = m.faces[k];
@@ -1931,7 +1919,7 @@ __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl
                         lo[1] = fmin(lo[1], mx); hi[1] = fmax(hi[1], mx);
                         lo[2] = fmin(lo[2], my); hi[2] = fmax(hi[2], my);
                     }
-                const bool full = det > F(1.e-12) * ((a11 + a22) * (a11 + a22));
+                const bool full = det > 1.e-12 * ((a11 + a22) * (a11 + a22));
 #pragma unroll
                 for (int p = 0; p < 4; ++p) {
                     if (full) {
@@ -1943,43 +1931,43 @@ __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl
                     }
                 }
                 const double hh = centre[0] - centre[3];
-                const F sq = hh > dry ? sqrt(F(grav) * F(hh)) : F(0.);
-                const F bedtol = F(64.0 * Eps<F>::value) * fmax(F(1.0), F(fabs(centre[3])));
-                F theta1 = F(1.), theta2 = F(1.);
-                F ax0[2 * MAXF], ay0[2 * MAXF], b0[2 * MAXF];
-                F ax3[2 * MAXF], ay3[2 * MAXF], b3[2 * MAXF];
+                const double sq = hh > dry ? sqrt(grav * hh) : 0.;
+                const double bedtol = 64.0 * EPS * fmax(1.0, fabs(centre[3]));
+                double theta1 = 1., theta2 = 1.;
+                double ax0[2 * MAXF], ay0[2 * MAXF], b0[2 * MAXF];
+                double ax3[2 * MAXF], ay3[2 * MAXF], b3[2 * MAXF];
                 int n0 = 0, n3 = 0;
                 for (int k = k0; k < k1; ++k) {
                     const int f = m.faces[k];
                     const int side = m.signs[k] < 0;
-                    const F rx = F(m.disp[side * nf + f]), ry = F(m.disp[(2 + side) * nf + f]);
+                    const double rx = m.disp[side * nf + f], ry = m.disp[(2 + side) * nf + f];
                     // an open stage outlet with a subcritical wet owner keeps its bed slope
                     if (m.bmode[f] == 2 && m.neighbour[f] < 0 && hh > dry &&
-                        fabs(F(centre[1]) * F(m.normal[f]) + F(centre[2]) * F(m.normal[nf + f])) < sq &&
+                        fabs(centre[1] * m.normal[f] + centre[2] * m.normal[nf + f]) < sq &&
                         fabs(gx[3] * rx + gy[3] * ry) > bedtol) continue;
 #pragma unroll
                     for (int p = 1; p < 3; ++p) {
-                        const F d = gx[p] * rx + gy[p] * ry;
-                        if (fabs(d) <= F(64.0 * Eps<F>::value) * fmax(F(1.0), F(fmax(fabs(centre[p]), fmax(fabs(lo[p]), fabs(hi[p]))))))
+                        const double d = gx[p] * rx + gy[p] * ry;
+                        if (fabs(d) <= 64.0 * EPS * fmax(1.0, fmax(fabs(centre[p]), fmax(fabs(lo[p]), fabs(hi[p])))))
                             continue;
-                        F &th = p == 1 ? theta1 : theta2;
-                        if (d > F(0.)) th = fmin(th, F(hi[p] - centre[p]) / d);
-                        if (d < F(0.)) th = fmin(th, F(lo[p] - centre[p]) / d);
+                        double &th = p == 1 ? theta1 : theta2;
+                        if (d > 0.) th = fmin(th, (hi[p] - centre[p]) / d);
+                        if (d < 0.) th = fmin(th, (lo[p] - centre[p]) / d);
                     }
-                    const F len = F(m.disp_len[side * nf + f]);
-                    if (len <= F(0.)) continue;
-                    const F ux = F(m.disp_unit[side * nf + f]), uy = F(m.disp_unit[(2 + side) * nf + f]);
-                    ax0[n0] = ux; ay0[n0] = uy; b0[n0++] = fmax(F(0.), F(hi[0] - centre[0])) / len;
-                    ax0[n0] = -ux; ay0[n0] = -uy; b0[n0++] = fmax(F(0.), F(centre[0] - lo[0])) / len;
+                    const double len = m.disp_len[side * nf + f];
+                    if (len <= 0.) continue;
+                    const double ux = m.disp_unit[side * nf + f], uy = m.disp_unit[(2 + side) * nf + f];
+                    ax0[n0] = ux; ay0[n0] = uy; b0[n0++] = fmax(0., hi[0] - centre[0]) / len;
+                    ax0[n0] = -ux; ay0[n0] = -uy; b0[n0++] = fmax(0., centre[0] - lo[0]) / len;
                     if (m.neighbour[f] < 0 && m.bid[f] < 0) continue;   // walls do not bound the bed
-                    ax3[n3] = ux; ay3[n3] = uy; b3[n3++] = fmax(F(0.), F(hi[3] - centre[3])) / len;
-                    ax3[n3] = -ux; ay3[n3] = -uy; b3[n3++] = fmax(F(0.), F(centre[3] - lo[3])) / len;
+                    ax3[n3] = ux; ay3[n3] = uy; b3[n3++] = fmax(0., hi[3] - centre[3]) / len;
+                    ax3[n3] = -ux; ay3[n3] = -uy; b3[n3++] = fmax(0., centre[3] - lo[3]) / len;
                 }
-                F px0 = gx[0], py0 = gy[0], px3 = gx[3], py3 = gy[3];
-                project_pair<F>(px0, py0, n0, ax0, ay0, b0);
-                project_pair<F>(px3, py3, n3, ax3, ay3, b3);
-                gx[1] *= fmax(F(0.), theta1); gy[1] *= fmax(F(0.), theta1);
-                gx[2] *= fmax(F(0.), theta2); gy[2] *= fmax(F(0.), theta2);
+                double px0 = gx[0], py0 = gy[0], px3 = gx[3], py3 = gy[3];
+                project_pair(px0, py0, n0, ax0, ay0, b0);
+                project_pair(px3, py3, n3, ax3, ay3, b3);
+                gx[1] *= fmax(0., theta1); gy[1] *= fmax(0., theta1);
+                gx[2] *= fmax(0., theta2); gy[2] *= fmax(0., theta2);
                 gx[0] = px0; gy[0] = py0; gx[3] = px3; gy[3] = py3;
             }
         }
@@ -1988,15 +1976,15 @@ __global__ void __launch_bounds__(128) k_cells(MeshDev m, StateDev s, Ctrl *ctrl
             for (int k = k0; k < k1; ++k) {
                 const int f = m.faces[k];
                 const int side = (c == m.owner[f]) ? 0 : 1;
-                const F rx = F(m.disp[side * nf + f]), ry = F(m.disp[(2 + side) * nf + f]);
-                const double eta = (centre[0] + double(gx[0] * rx)) + double(gy[0] * ry);
-                const double zb = (centre[3] + double(gx[3] * rx)) + double(gy[3] * ry);
+                const double rx = m.disp[side * nf + f], ry = m.disp[(2 + side) * nf + f];
+                const double eta = (centre[0] + gx[0] * rx) + gy[0] * ry;
+                const double zb = (centre[3] + gx[3] * rx) + gy[3] * ry;
                 if (eta - zb <= dry || fabs(zb - centre[3]) >= h) { flatten = true; break; }
             }
         CellRec r;
         r.h = h; r.eta = centre[0]; r.u = centre[1]; r.v = centre[2]; r.b = centre[3];
 #pragma unroll
-        for (int p = 0; p < 4; ++p) { r.gx[p] = double(gx[p]); r.gy[p] = double(gy[p]); }
+        for (int p = 0; p < 4; ++p) { r.gx[p] = gx[p]; r.gy[p] = gy[p]; }
         r.flags = (flatten ? 1 : 0) | (active ? 2 : 0);
         r.pad = 0; r.pad2 = 0.;
         w.rec[c] = r;

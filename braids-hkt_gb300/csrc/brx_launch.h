@@ -91,7 +91,8 @@ inline int shape_grid(const Launch &L, int kind, int n)
     return g < 1 ? 1 : (g < cap ? g : cap);
 }
 
-// Kernel kinds of one substep, in launch order within a stage.
+// Kernel kinds of one substep, in launch order within a stage. K_GATHER has no
+// kernel of its own (the update gathers); its launch-shape slot is kept.
 enum KernelKind { K_DRAG = 0, K_BOUNDARY = 1, K_CELLS = 2, K_FACES = 3, K_GATHER = 4, K_LIMIT = 5, K_UPDATE = 6 };
 // Mixed form only: first-stage primitives of a state placed in work, the
 // bed-derived tables, the limited water flux into a caller buffer.
