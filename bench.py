@@ -32,17 +32,22 @@ sys.path.insert(0, os.path.join(ROOT, "oracle"))
 METRIC = "cell-updates/s"
 BYTES_PER_CELL_UPDATE = {"fp64": 680.0, "mixed": 384.0}   # algorithmic bytes, two-sweep design
 # DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per cell of one
-# launch of each mixed-form sweep, each kernel captured alone (ncu, one launch)
-# on a channel of 899,304 triangles without rotors (inputs larger than L2): a
+# launch of each mixed-form sweep (the mean of the two stages), each kernel
+# captured alone (ncu, one launch) on the 24-scenario subset with rotors
+# (scenarios 20..43 sorted by size, 1,967,962 cells, inputs larger than L2): a
 # launch of the full batch is scaled by its cells
-TRAFFIC_BYTES_PER_CELL = {"mixed": {"cells": 186.4, "faces": 152.9, "update": 225.9, "drag": 38.2}}
+TRAFFIC_BYTES_PER_CELL = {"mixed": {"cells": 241.7, "faces": 210.3, "update": 245.8, "drag": 62.9}}
 KERNEL_NAMES = ["drag", "boundary", "cells", "faces", "update", "control"]
 # FP64 flops (2 DFMA + DMUL + DADD thread instructions) per cell (per face for
-# the face sweep) of one launch of each FP64-form sweep (the update: the mean of
-# the two stages), each kernel captured alone on a 50k-cell channel (ncu, one
-# trial), and their sum over one substep per cell-update
-FP64_FLOPS = {"cells": ("cell", 169.0), "faces": ("face", 379.0), "update": ("cell", 137.0), "drag": ("cell", 143.0)}
-FP64_FLOPS_PER_CELL_UPDATE = 1900.0
+# the face sweep) of one launch of the FP64 form's two large sweeps (the mean of the
+# two stages), each kernel captured alone (ncu, one trial), and the sum of all
+# kernels over one substep per cell-update: a 50k-cell channel without rotors,
+# config 2 with three (the face sweep forms their pressure, the wet gradients
+# are a sweep more)
+FP64_FLOPS = {"plain": {"cells": ("cell", 169.0), "faces": ("face", 379.0), "cell_update": 1900.0},
+              "rotors": {"cells": ("cell", 178.3), "faces": ("face", 581.2), "cell_update": 2829.0}}
+FP64_SOURCE = {"plain": "ncu FP64 thread-instruction counts of a 50k-cell channel, scaled",
+               "rotors": "ncu FP64 thread-instruction counts of config 2 (124k cells, 3 rotors), scaled"}
 
 
 def peaks():
@@ -286,21 +291,22 @@ def fp64_comparison(cases, outer, steps, mixed_state, mixed_z, mixed_rotors, tor
     return out
 
 
-def fp64_roofline(per_kind, nc, nf, value, peak_tflops):
+def fp64_roofline(per_kind, nc, nf, value, peak_tflops, rotors):
     """Compute roofline of the FP64 form: the FP64 flops of the slower of the
     two FP64 sweeps over its live duration, and of the whole step at the
     measured throughput, against the measured FP64 FMA rate."""
+    flavour = "rotors" if rotors else "plain"
     dom = max(("cells", "faces"), key=lambda k: sum(per_kind.get(k, [0.0])))
-    unit, per = FP64_FLOPS[dom]
+    unit, per = FP64_FLOPS[flavour][dom]
     flops = per * (nf if unit == "face" else nc)
     ms = float(np.mean(per_kind[dom]))
     achieved = flops / (ms * 1e-3) / 1e12
-    step = value * FP64_FLOPS_PER_CELL_UPDATE / 1e12
+    step = value * FP64_FLOPS[flavour]["cell_update"] / 1e12
     return {"bound": "fp64", "kernel": f"k_{dom}", "achieved": achieved, "peak": peak_tflops, "unit": "TFLOP/s",
             "frac": achieved / peak_tflops, "kernel_ms": ms, "flops_per_launch": flops,
-            "flops_source": f"ncu FP64 thread-instruction counts per {unit} of a 50k-cell channel capture, scaled",
+            "flops_source": FP64_SOURCE[flavour],
             "peak_source": "brx_fma_rate (measured FP64 FMA rate of this GPU)",
-            "step_flops_per_cell_update": FP64_FLOPS_PER_CELL_UPDATE, "step_achieved_tflops": step,
+            "step_flops_per_cell_update": FP64_FLOPS[flavour]["cell_update"], "step_achieved_tflops": step,
             "step_frac": step / peak_tflops}
 
 
@@ -596,7 +602,7 @@ def main():
     total_ms = sum(sum(v) for v in per_kind.values())
     roofline = {"bound": "hbm", "kernel": f"k_{dom}", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak, "traffic": traffic,
-                "traffic_source": ("ncu DRAM bytes per cell of a 900k-cell channel capture, scaled by cells"
+                "traffic_source": ("ncu DRAM bytes per cell of a capture of 24 scenarios with rotors, scaled by cells"
                                    if traffic is not None else None),
                 "peak_source": peak_kind,
                 "kernel_ms": dom_ms, "kernel_share_of_substep": sum(per_kind[dom]) / total_ms,
@@ -765,13 +771,14 @@ def main():
                                  "thread at full occupancy, CUDA events, best of 5")
     fp64_peak = line["compute_peaks"]["fp64_tflops"]
     if precision == "fp64":
-        line["roofline_fp64"] = fp64_roofline(per_kind, nc, nf, value, fp64_peak)
+        line["roofline_fp64"] = fp64_roofline(per_kind, nc, nf, value, fp64_peak, bool(with_rotors))
     if plain is not None:
-        plain["roofline_fp64"] = {"achieved": plain["value"] * FP64_FLOPS_PER_CELL_UPDATE / 1e12, "peak": fp64_peak,
-                                  "unit": "TFLOP/s",
-                                  "frac": plain["value"] * FP64_FLOPS_PER_CELL_UPDATE / 1e12 / fp64_peak,
-                                  "step_flops_per_cell_update": FP64_FLOPS_PER_CELL_UPDATE,
-                                  "flops_source": "ncu FP64 thread-instruction counts per cell-update of a 50k-cell channel"}
+        # the leg's scenarios are taken from those with rotors where there are any
+        flavour = "rotors" if with_rotors else "plain"
+        per = FP64_FLOPS[flavour]["cell_update"]
+        plain["roofline_fp64"] = {"achieved": plain["value"] * per / 1e12, "peak": fp64_peak, "unit": "TFLOP/s",
+                                  "frac": plain["value"] * per / 1e12 / fp64_peak, "step_flops_per_cell_update": per,
+                                  "flops_source": FP64_SOURCE[flavour]}
         line["roofline_fp64"] = dict(plain["roofline_fp64"], leg="plain_fp64")
     if chained is not None:
         line["chained"] = chained

@@ -4,7 +4,8 @@
 // What bounds it: FP64 instructions (brx_num64.cuh). Nearly every face joins
 // two wet states; for those the solve is written out with the terms that
 // vanish or repeat taken out, each remaining operation being the reference's
-// own with the same operands, so the fluxes are the same bits:
+// own with the same operands (a quotient to the bound of quotient()), so the
+// fluxes of all compared faces are the same bits:
 //   * the hydrostatic reconstruction gives both sides one bed, so the bed
 //     jump is zero and with it the steady-state correction of the depth and
 //     momentum jumps (their clamps hold zero in place);

@@ -117,8 +117,9 @@ __device__ __forceinline__ void hllc_riemann(double hl, double ul, double vl, do
 // Bound by FP64 instructions (brx_num64.cuh): velocities come from the opening
 // drag's primitives, the quotients by squared offsets from their stored
 // reciprocals, minima and maxima run on the integer pipe, and a limiter
-// quotient is formed only where it is below the factor held. Same bits as the
-// 44 divisions per cell it replaces. 101k cells: 208 -> 95 us per launch.
+// quotient is formed only where it is below the factor held. 44 divisions per cell
+// gone, their results kept to the bound of quotient(). 101k cells: 208 -> 95 us per
+// launch.
 template <int MAXF>
 __global__ void __launch_bounds__(128) k_hllc_cells(MeshDev m, StateDev s, HllcDev h, HCell *rec, Ctrl *ctrl)
 {

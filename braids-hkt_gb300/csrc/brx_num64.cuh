@@ -33,10 +33,13 @@ __device__ __forceinline__ bool finite_bits(double x)
     return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
 }
 
-// x / y from r = RN(1 / y): a first quotient and one exact remainder
-// (P. Markstein, IBM J. Res. Dev. 34(1):111, 1990). With r correctly rounded
-// the corrected quotient is RN(x / y) unless x / y lies within 2^-104 of a
-// rounding boundary, relative. Three FP64 instructions instead of ten.
+// x / y from r, 1 / y to an ulp (stored and correctly rounded, or reciprocal()): a
+// first quotient and one remainder (P. Markstein, IBM J. Res. Dev. 34(1):111,
+// 1990). The result is the rounding of x / y (1 + d) with |d| < 2^-102, so RN(x / y)
+// unless x / y lies that close to the middle of two numbers. Three FP64
+// instructions instead of ten. Finite x, y and r, x r and the remainder without
+// overflow or underflow; an infinite operand, or a y whose reciprocal overflows or
+// vanishes, gives no number (any_quotient() where such states are accepted).
 __device__ __forceinline__ double quotient(double x, double y, double r)
 {
     const double q = __dmul_rn(x, r);
@@ -45,7 +48,7 @@ __device__ __forceinline__ double quotient(double x, double y, double r)
 
 // 1 / y to about an ulp, for quotient(): the hardware's approximation (PTX
 // rcp.approx.ftz.f64, relative error below 2^-20) and two Newton-Raphson steps;
-// four FP64 instructions instead of a division's ten. y normal and finite.
+// four FP64 instructions instead of a division's ten. 2^-1022 <= |y| <= 2^1022.
 __device__ __forceinline__ double reciprocal(double y)
 {
     double r;

@@ -4,9 +4,9 @@ reciprocal (quotient(x, y, reciprocal(y))) against IEEE division, the integer
 comparisons and tests against the plain ones, the truncation to FP32.
 
 With e the relative error of the reciprocal, the corrected quotient is the
-rounding of x / y (1 + d), |d| <= |e| (|e| + 2^-53) < 2^-103: the correctly rounded
-quotient unless x / y lies that close to the middle of two numbers, which of
-random operands none in 2^49 does."""
+rounding of x / y (1 + d), |d| <= |e| (|e| + 2^-53) plus the remainder's rounding,
+below 2^-102: the correctly rounded quotient unless x / y lies that close to the
+middle of two numbers, which of random operands none in 2^48 does."""
 import ctypes as C
 import subprocess
 
