@@ -812,36 +812,42 @@ extern "C" int brx_forcing_table_set(brx_solver *s, int len, const double *time,
 static int ensure_tables64(brx_solver *s)
 {
     if (s->precision != BRX_FP64 || s->pending) return BRX_OK;     // an interval in flight reads them
-    const bool fwave = s->method == BRX_METHOD_FWAVE;
+    const bool fwave = s->method == BRX_METHOD_FWAVE, cells = fwave && s->small64;
+    const bool weights = !s->work.rarea || (fwave && !s->work.cw), tables = cells && s->tables64_dirty;
+    const size_t nc = s->nc, nadj = s->nadj;
+    Cells64 g = s->c64;
+    double2 *cw = const_cast<double2 *>(s->work.cw);
+    double *rarea = const_cast<double *>(s->work.rarea);
+    // the missing arrays in one allocation
+    std::vector<std::pair<void *, size_t>> missing;                // a pointer's address, bytes
+    const auto need = [&](auto *&p, size_t count) {
+        if (!p) missing.emplace_back(&p, count * sizeof(*p));
+    };
+    need(rarea, nc);
+    if (fwave) need(cw, nadj);
+    if (cells || !fwave) need(g.prim[0], nc);
+    if (cells) {
+        need(g.prim[1], nc); need(g.ls, nc); need(g.lsr, nc); need(g.par, nc); need(g.ccls, nc); need(g.gbed, nc);
+        need(g.cidx, nadj); need(g.ent, nadj); need(g.unit, nadj);
+    }
+    if (!missing.empty()) {
+        const auto padded = [](size_t bytes) { return (bytes + 255) / 256 * 256; };
+        size_t total = 0;
+        for (const auto &m : missing) total += padded(m.second);
+        unsigned char *block;
+        TRY(s->alloc(&block, total));
+        for (const auto &m : missing) { memcpy(m.first, &block, sizeof block); block += padded(m.second); }
+    }
     const int grid = std::max(1, std::min((s->nc + 255) / 256, s->sms * 32));
-    bool formed = false;
-    if (!s->work.rarea || (fwave && !s->work.cw)) {
-        double2 *cw = nullptr;
-        double *rarea = const_cast<double *>(s->work.rarea);
-        if (fwave) TRY(s->alloc(&cw, s->nadj));
-        if (!rarea) TRY(s->alloc(&rarea, s->nc));
-        k64_weights<<<grid, 256>>>(s->mesh, cw, rarea);
-        s->work.cw = cw; s->work.rarea = rarea;
-        formed = true;
+    if (weights) k64_weights<<<grid, 256>>>(s->mesh, cw, rarea);
+    if (tables) k64_tables<<<grid, 256>>>(s->mesh, g);
+    if (weights || tables) {
+        CK(cudaGetLastError());
+        CK(cudaStreamSynchronize(nullptr));
     }
-    Cells64 &g = s->c64;
-    if (!g.prim[0] && (!fwave || s->small64)) {
-        TRY(s->alloc(&g.prim[0], s->nc));
-        s->hllc.prim = g.prim[0];
-    }
-    if (fwave && s->small64 && s->tables64_dirty) {
-        if (!g.prim[1]) {
-            TRY(s->alloc(&g.ls, s->nc)); TRY(s->alloc(&g.lsr, s->nc)); TRY(s->alloc(&g.par, s->nc));
-            TRY(s->alloc(&g.ccls, s->nc)); TRY(s->alloc(&g.cidx, s->nadj)); TRY(s->alloc(&g.ent, s->nadj));
-            TRY(s->alloc(&g.unit, s->nadj)); TRY(s->alloc(&g.gbed, s->nc)); TRY(s->alloc(&g.prim[1], s->nc));
-        }
-        k64_tables<<<grid, 256>>>(s->mesh, g);
-        formed = true;
-    }
-    if (!formed) return BRX_OK;
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(nullptr));
-    if (fwave) s->tables64_dirty = false;
+    s->c64 = g; s->hllc.prim = g.prim[0];
+    s->work.cw = cw; s->work.rarea = rarea;
+    if (tables) s->tables64_dirty = false;
     return BRX_OK;
 }
 
