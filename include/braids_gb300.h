@@ -177,7 +177,9 @@ int brx_forcing_table_set(brx_solver *s, int len, const double *time, const doub
 
 /* Bind caller-owned DEVICE buffers: q (3,nc) accepted state, updated in place;
  * z (nc) bed. The reference keeps q and z in its owner
- * (ShorelineSolver.q / .z, src/braids_core/sediment/shoreline_solver.py:275). */
+ * (ShorelineSolver.q / .z, src/braids_core/sediment/shoreline_solver.py:275).
+ * Best the last call of a set-up: it forms the mesh tables of the method selected
+ * then (a method or boundary modes set later form theirs in the next call). */
 int brx_state_bind(brx_solver *s, double *q_device, double *z_device);
 
 /* Advance every active scenario over [time, time+dt] with the adaptive
